@@ -518,9 +518,9 @@ def tolerance(case):
     if case.get("mixed"):
         return {"rel": 1e-4, "max": 1e-2} if kind == "air_rhs" else {"rel": 6e-4, "max": 5e-2} if kind == "h2_rhs" else {"rel": 4e-6, "max": 4e-5}
     return {"tube": {"rel": 5e-14, "max": 1e-11}, "air_step": {"rel": 2e-15, "max": 1e-13}, "blocks": {"rel": 2e-15, "max": 1e-13},
-            "air_rhs": {"rel": 4e-13, "max": 1e-10}, "h2_step": {"rel": 1e-13, "max": 1e-9}, "h2_rhs": {"rel": 8e-13, "max": 1e-10},
+            "air_rhs": {"rel": 4e-13, "max": 1e-10}, "h2_step": {"rel": 1e-13, "max": 1e-9}, "h2_rhs": {"rel": 2e-12, "max": 1e-10},
             "h2_properties": {"rel": 2e-15, "max": 2e-14}, "cylinder": {"rel": 1e-9, "max": 1e-6},
-            "reactors": {"rel": 3e-9, "max": 1e-6, "differ": 0.005}}[kind]
+            "reactors": {"rel": 1e-8, "max": 1e-5, "differ": 0.005}}[kind]
 
 
 # ---- the same results in plain torch, 64 bits --------------------------------------------------
