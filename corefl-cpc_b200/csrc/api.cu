@@ -95,6 +95,8 @@ struct cb2_ctx {
   Param p{};
   cb2_param_view view{};
   void *d_tables = nullptr;  // mechanism tables (one allocation)
+  TransTabs *trans_tabs = nullptr;  // its transport data for the property kernels (host)
+  ChemTabs *chem_tabs = nullptr;  // the mechanism repacked for the chemistry kernel (host)
   unsigned *d_status = nullptr;
   double *d_dtmin = nullptr;     // running min of the CFL dt
   double *d_partial = nullptr;   // per-CTA partial minima of the reduction
@@ -154,6 +156,28 @@ namespace {
 int fail_cuda(cudaError_t e) {
   set_cuda_error(e);
   return CB2_ERR_CUDA;
+}
+
+// The NASA7 table that travels in the kernels' parameters (ThermoTab).
+void fill_thermo_tab(const cb2_mechanism &m, ThermoTab &t) {
+  t = ThermoTab{};
+  if (m.therm_nasa_7_9 == 9 || m.n_spec > kMaxSpec) return;
+  t.t_low = m.t_low[0];
+  t.t_mid = m.t_mid[0];
+  t.t_high = m.t_high[0];
+  for (int s = 0; s < m.n_spec; ++s) {
+    if (m.t_mid[s] != t.t_mid) return;
+    t.t_low = std::max(t.t_low, m.t_low[s]);
+    t.t_high = std::min(t.t_high, m.t_high[s]);
+    const double r = kRu / m.mw[s];
+    for (int h = 0; h < 2; ++h) {
+      const double *a = (h ? m.high_temp_coeff : m.low_temp_coeff) + 7 * s;
+      for (int n = 0; n < 5; ++n) t.cp[h][s][n] = a[n] * r;
+      t.h[h][s][0] = a[5] * r;
+      for (int n = 1; n < 5; ++n) t.h[h][s][n] = a[n] / (n + 1) * r;
+    }
+  }
+  t.use = 1;
 }
 
 // Copies the mechanism into one device allocation and fills the device pointers of Mech.
@@ -285,6 +309,11 @@ int upload_mechanism(const cb2_mechanism &m, const cb2_two_temperature *tt, cb2_
   for (auto &s : is) *s.dst = reinterpret_cast<const int *>(dev + bd) + s.off;
   d.n_spec = ns;
   d.n_reac = nr;
+  ctx->trans_tabs = make_trans_tabs(m);
+  d.trans_tabs = ctx->trans_tabs;
+  fill_thermo_tab(m, d.tab);
+  ctx->chem_tabs = make_chem_tabs(m);
+  d.chem_tabs = ctx->chem_tabs;
   d.nasa9 = nasa9 ? 1 : 0;
   d.max_range = nasa9 ? m.max_range : 0;
   d.park = park ? 1 : 0;
@@ -556,6 +585,8 @@ void cb2_destroy(cb2_ctx *ctx) {
     cudaFree(b.d_f32);
     cudaFree(b.d_face_sv);
   }
+  free_chem_tabs(ctx->chem_tabs);
+  free_trans_tabs(ctx->trans_tabs);
   cudaFree(ctx->d_tables);
   cudaFree(ctx->d_status);
   cudaFree(ctx->d_partial);

@@ -1,6 +1,11 @@
 // Explicit finite-rate chemistry source over a block (the launch of finite_rate_chemistry,
-// src/FiniteRateChem.cu:1406-1488); the per-node arithmetic is in chem.cuh.
+// src/FiniteRateChem.cu:1406-1488).  One-temperature NASA7 mechanisms of up to kChemTabReac
+// reactions run k_chemistry_tab on a repacked mechanism; the others (NASA9, control temperatures,
+// two temperatures, longer mechanisms) run the generic arithmetic of chem.cuh.
+#include <algorithm>
+#include <cmath>
 #include "chem.cuh"
+#include "chem_tab.cuh"
 #include "launch.h"
 
 namespace cb2 {
@@ -17,10 +22,180 @@ __global__ void __launch_bounds__(kChemThreads, 4) k_chemistry(Zone z, Param p) 
   chemistry_point<NS>(z, p, i, j, k);
 }
 
+// The arrays the table kernel touches: a small argument beside the table.
+struct ChemZone {
+  int mx, plane;  // nodes per line and per k plane
+  Layout L;
+  idx_t sz0;
+  const double *bv, *sv, *jac;
+  double *dq, *rts;
+};
+
+// g/(RT) of every species into column tid of sg, each fit evaluated at the edge of its range
+// outside it.
+template <int NS>
+__device__ __forceinline__ void tab_gibbs(const ChemTab<NS> &m, double t, double lnt, double it,
+                                          double (*sg)[kChemThreads], int tid) {
+  if (m.same_mid && t >= m.t_in_low && t <= m.t_in_high) {
+    const double l1 = 1.0 - lnt;
+    if (t < m.t_mid) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const double *c = m.g[0][s];
+        sg[s][tid] = fma(-t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), fma(c[0], l1, fma(c[5], it, -c[6])));
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const double *c = m.g[1][s];
+        sg[s][tid] = fma(-t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), fma(c[0], l1, fma(c[5], it, -c[6])));
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int s = 0; s < NS; ++s) {
+      const double tt = t < m.tl[s] ? m.tl[s] : (t > m.th[s] ? m.th[s] : t);
+      const double lt = tt == t ? lnt : log(tt);
+      // inside the fit the middle decides the range; outside it the edge's own range is taken
+      const double *c = m.g[(tt == t ? t < m.tm[s] : t < m.tl[s]) ? 0 : 1][s];
+      sg[s][tid] = c[0] * (1.0 - lt) - tt * (c[1] + tt * (c[2] + tt * (c[3] + tt * c[4]))) + c[5] / tt - c[6];
+    }
+  }
+}
+
+// The source of one node per thread, J omega_k added to dq and the reaction time scale.
+//
+// Bound by the FP64 pipe: about 40 exponentials (18 pipe instructions each) and some 400 further
+// FP64 operations per node of the H2/air mechanism.  The table keeps everything else off the
+// critical resources: rate constants are constant-bank operands, zero stoichiometric coefficients
+// cost nothing (the dense loops over integer coefficients took four fifths of the time, most of it
+// in loads and in integer-to-double conversions), and kf / Kc is one exponential without a
+// division.  Concentrations and g/(RT) are indexed by species numbers read from the table, so they
+// live in shared memory, one column per thread (no bank conflicts).  The tile runs along the
+// k plane's nodes, not along one line, so a ragged mx leaves no idle threads.
+template <int NS>
+__global__ void __launch_bounds__(kChemThreads, 5)
+k_chemistry_tab(const __grid_constant__ ChemZone z, const __grid_constant__ ChemTab<NS> m) {
+  __shared__ double sc[NS][kChemThreads], sg[NS][kChemThreads];
+  const int tid = threadIdx.x;
+  const int q = blockIdx.x * kChemThreads + tid;
+  if (q >= z.plane) return;
+  const int j = q / z.mx, i = q - j * z.mx, k = blockIdx.y;
+  const idx_t g = z.L.at(i, j, k), sz = z.L.sz;
+  const double rho = z.bv[g], t = z.bv[g + 5 * sz];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) sc[s][tid] = rho * z.sv[g + s * sz] * m.c_per_rho_y[s];
+  const double lnt = log(t), it = 1.0 / t;
+  if (m.need_gibbs) tab_gibbs<NS>(m, t, lnt, it, sg, tid);
+  double cre[NS], des[NS];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) cre[s] = des[s] = 0;
+#pragma unroll 1
+  for (int r = 0; r < m.n_reac; ++r) {
+    const ChemReac &x = m.r[r];
+    const int ty = x.type;
+    double kf = x.A * exp(fma(x.b, lnt, -x.Ea * it));
+    double cc = 0;
+    if (ty > 3) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) cc = fma(sc[s][tid], x.tb[s], cc);
+    }
+    if (ty == 3) {
+      kf += x.A2 * exp(fma(x.b2, lnt, -x.Ea2 * it));
+    } else if (ty == 4) {
+      kf *= cc;
+    } else if (ty > 4) {
+      const double kl = x.A2 * exp(fma(x.b2, lnt, -x.Ea2 * it));
+      if (kf < 1e-25 && kl < 1e-25) {
+        kf = 0;
+      } else {
+        const double pr = kl * cc / kf;
+        double F = 1.0;
+        if (ty > 5) {
+          double fc = (1 - x.alpha) * exp(-t * x.it3) + x.alpha * exp(-t * x.it1);
+          if (ty == 7) fc += exp(-x.t2 * it);
+          const double lfc = log10(fc);
+          const double cq = -0.4 - 0.67 * lfc, nq = 0.75 - 1.27 * lfc;
+          const double lp = log10(pr) + cq;
+          const double tmp = lp / (nq - 0.14 * lp);
+          F = pow(10.0, lfc / (1.0 + tmp * tmp));
+        }
+        kf = kf * pr / (1.0 + pr) * F;
+      }
+    }
+    double q1 = kf, q2 = 0;
+    unsigned list = x.flist;
+#pragma unroll 1
+    for (int a = 0; a < x.nf; ++a, list >>= 4) q1 *= sc[list & 15u][tid];
+    if (x.back != kBackNone) {
+      if (x.back == kBackEquilibrium) {
+        // kb = kf / Kc, Kc = (p_atm / (R_u T) 1e-3)^order exp(-sum nu g/(RT))
+        double dg = fma(x.order, lnt, -x.order_ln);
+        list = x.flist;
+#pragma unroll 1
+        for (int a = 0; a < x.nf; ++a, list >>= 4) dg -= sg[list & 15u][tid];
+        list = x.blist;
+#pragma unroll 1
+        for (int a = 0; a < x.nb; ++a, list >>= 4) dg += sg[list & 15u][tid];
+        q2 = kf * exp(dg);
+      } else {
+        q2 = x.A2 * exp(fma(x.b2, lnt, -x.Ea2 * it));
+        if (ty == 4) q2 *= cc;
+      }
+      list = x.blist;
+#pragma unroll 1
+      for (int a = 0; a < x.nb; ++a, list >>= 4) q2 *= sc[list & 15u][tid];
+    }
+#pragma unroll 1
+    for (int l = 0; l < x.levels; ++l) {
+      const unsigned mf = x.mf[l], mb = x.mb[l];
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        if (mf >> s & 1u) {
+          des[s] += q1;
+          cre[s] += q2;
+        }
+        if (mb >> s & 1u) {
+          cre[s] += q1;
+          des[s] += q2;
+        }
+      }
+    }
+  }
+  const double jac = z.jac[g];
+  const idx_t g0 = q + (idx_t)k * z.plane;
+  double ts = 1e+6;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double od = des[s] * m.w[s];
+    const double om = cre[s] * m.w[s] - od;
+    z.dq[g0 + (5 + s) * z.sz0] += jac * om;
+    const double y = z.sv[g + s * sz];
+    if (y > 1e-25 && fabs(od) > 1e-25) ts = fmin(ts, fabs(rho * y / od));
+  }
+  if (z.rts) z.rts[g] = ts;
+}
+
+template <int NS>
+static int launch_chemistry_tab(const Zone &z, const ChemTab<NS> &m, cudaStream_t s) {
+  ChemZone c{};
+  c.mx = z.mx;
+  c.plane = z.mx * z.my;
+  c.L = z.L;
+  c.sz0 = z.L0.sz;
+  c.bv = z.bv; c.sv = z.sv; c.jac = z.jac; c.dq = z.dq; c.rts = z.rts;
+  const dim3 grid((unsigned)((c.plane + kChemThreads - 1) / kChemThreads), (unsigned)z.mz);
+  k_chemistry_tab<NS><<<grid, kChemThreads, 0, s>>>(c, m);
+  return check_launch();
+}
+
 int launch_chemistry(const Zone &z, const Param &p, cudaStream_t s, int &n_launch) {
-  dim3 grid((z.mx + kChemThreads - 1) / kChemThreads, z.my, z.mz);
   ProfScope prof("chemistry", s);
   ++n_launch;
+  const ChemTabs *tab = p.i_eve < 0 ? p.mech.chem_tabs : nullptr;
+  if (tab && tab->ns == 9) return launch_chemistry_tab<9>(z, tab->t9, s);
+  if (tab && tab->ns == 5) return launch_chemistry_tab<5>(z, tab->t5, s);
+  dim3 grid((z.mx + kChemThreads - 1) / kChemThreads, z.my, z.mz);
   switch (p.n_spec) {
     case 5: k_chemistry<5><<<grid, kChemThreads, 0, s>>>(z, p); break;
     case 9: k_chemistry<9><<<grid, kChemThreads, 0, s>>>(z, p); break;
@@ -28,5 +203,91 @@ int launch_chemistry(const Zone &z, const Param &p, cudaStream_t s, int &n_launc
   }
   return check_launch();
 }
+
+// ---- repacking (host) --------------------------------------------------------------------------
+namespace {
+
+// Species lists and coefficient masks of one side of a reaction; false if they do not fit.
+bool pack_side(const int *stoi, int ns, unsigned &list, int &n, unsigned short *mask) {
+  list = 0;
+  n = 0;
+  for (int s = 0; s < ns; ++s) {
+    if (stoi[s] < 0 || stoi[s] > kChemTabMult) return false;
+    for (int a = 0; a < stoi[s]; ++a) {
+      if (n == kChemTabList) return false;
+      list |= (unsigned)s << (4 * n++);
+      mask[a] |= (unsigned short)(1u << s);
+    }
+  }
+  return true;
+}
+
+template <int NS>
+bool fill_tab(const cb2_mechanism &m, ChemTab<NS> &t) {
+  const int nr = m.n_reac;
+  t.n_reac = nr;
+  t.same_mid = 1;
+  t.t_mid = m.t_mid[0];
+  t.t_in_low = m.t_low[0];
+  t.t_in_high = m.t_high[0];
+  for (int s = 0; s < NS; ++s) {
+    const double imw = 1.0 / m.mw[s];
+    t.c_per_rho_y[s] = imw * 1e-3;
+    t.w[s] = 1e+3 / imw;
+    t.tl[s] = m.t_low[s]; t.tm[s] = m.t_mid[s]; t.th[s] = m.t_high[s];
+    t.t_in_low = std::max(t.t_in_low, t.tl[s]);
+    t.t_in_high = std::min(t.t_in_high, t.th[s]);
+    if (t.tm[s] != t.t_mid) t.same_mid = 0;
+    for (int h = 0; h < 2; ++h) {
+      const double *a = (h ? m.high_temp_coeff : m.low_temp_coeff) + 7 * s;
+      const double c[7] = {a[0], 0.5 * a[1], a[2] / 6.0, a[3] / 12.0, a[4] / 20.0, a[5], a[6]};
+      for (int n = 0; n < 7; ++n) t.g[h][s][n] = c[n];
+    }
+  }
+  for (int r = 0; r < nr; ++r) {
+    ChemReac &x = t.r[r];
+    x = ChemReac{};
+    const int ty = m.reac_type[r], rev = m.rev_type[r];
+    if (!pack_side(m.stoi_f + r * NS, NS, x.flist, x.nf, x.mf) || !pack_side(m.stoi_b + r * NS, NS, x.blist, x.nb, x.mb))
+      return false;
+    x.type = ty;
+    x.back = ty == 0 ? kBackNone : rev == 1 ? kBackArrhenius : ty != 2 ? kBackEquilibrium : kBackNone;
+    if (x.back == kBackEquilibrium) t.need_gibbs = 1;
+    x.A = m.A[r]; x.b = m.b[r]; x.Ea = m.Ea[r];
+    auto opt = [&](const double *a) { return a ? a[r] : 0.0; };
+    x.A2 = opt(m.A2); x.b2 = opt(m.b2); x.Ea2 = opt(m.Ea2);
+    x.order = m.reac_order ? m.reac_order[r] : 0;
+    x.order_ln = x.order * std::log(kPatm / kRu * 1e-3);
+    if (ty > 5) {
+      if (!m.troe_alpha || !m.troe_t3 || !m.troe_t1 || m.troe_t3[r] == 0 || m.troe_t1[r] == 0) return false;
+      x.alpha = m.troe_alpha[r];
+      x.it3 = 1.0 / m.troe_t3[r];
+      x.it1 = 1.0 / m.troe_t1[r];
+      x.t2 = opt(m.troe_t2);
+    }
+    for (int s = 0; s < NS; ++s) x.tb[s] = m.third_body_coeff ? m.third_body_coeff[r * NS + s] : 0.0;
+    for (int l = 0; l < kChemTabMult; ++l)
+      if (x.mf[l] | x.mb[l]) x.levels = l + 1;
+  }
+  return true;
+}
+
+}  // namespace
+
+ChemTabs *make_chem_tabs(const cb2_mechanism &m) {
+  if (m.therm_nasa_7_9 == 9 || m.two_temperature_reaction_temperature || m.n_reac < 1 || m.n_reac > kChemTabReac ||
+      !m.reac_type || !m.rev_type || !m.stoi_f || !m.stoi_b || !m.A || !m.b || !m.Ea)
+    return nullptr;
+  ChemTabs *t = new ChemTabs{};
+  const bool ok = m.n_spec == 5 ? fill_tab<5>(m, t->t5) : m.n_spec == 9 && fill_tab<9>(m, t->t9);
+  if (ok) {
+    t->ns = m.n_spec;
+    return t;
+  }
+  delete t;
+  return nullptr;
+}
+
+void free_chem_tabs(ChemTabs *t) { delete t; }
 
 }  // namespace cb2

@@ -81,6 +81,19 @@ struct Zone {
   unsigned sweep_mask;  // primitive sweeps to run (bit d: direction d; 0: all)
 };
 
+struct ChemTabs;   // chem_tab.cuh
+struct TransTabs;  // transport_tab.cuh
+
+// NASA7 coefficients of both ranges, by value in the kernels' parameters (thermo.cuh, tab_h_cp):
+// cp = c0 + c1 T + .. and h = a0 + T (c0 + T (a1 + T (a2 + ..))), scaled by the gas constant and the
+// integration factors.  use = 1 where every species has the same middle temperature; valid on
+// [t_low, t_high], the range that every fit covers.
+struct ThermoTab {
+  int use;
+  double t_low, t_mid, t_high;
+  double h[2][kMaxSpec][5], cp[2][kMaxSpec][5];
+};
+
 // Mechanism tables in device memory (copied from cb2_mechanism by cb2_init).
 struct Mech {
   int n_spec, n_reac;
@@ -108,6 +121,9 @@ struct Mech {
   const double *theta_v, *elec_theta, *elec_g, *lt_a, *lt_b, *park_sigma;
   const int *n_level;
   const double *elec_cut;  // [n_spec] truncation constant A of the electronic sums (ve_energy)
+  ThermoTab tab;
+  const TransTabs *trans_tabs;  // HOST memory, the context's: transport data repacked (null: generic)
+  const ChemTabs *chem_tabs;  // HOST memory, the context's: the mechanism repacked (null: it does not fit)
 };
 
 // Scalar settings passed by value to kernels.

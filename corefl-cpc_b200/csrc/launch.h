@@ -79,6 +79,9 @@ int launch_cv_from_bv(const Zone &z, const Param &p, cudaStream_t s, int &n_laun
 // two-temperature VT relaxation over dt_stage of every interior node (a standalone
 // apply_vt_relaxation_rk; launch_stage_update runs it itself for two-temperature contexts)
 int launch_vt_relaxation(const Zone &z, const Param &p, double dt_stage, cudaStream_t s, int &n_launch);
+// The transport data repacked for the property kernels (transport_tab.cuh), or null.
+TransTabs *make_trans_tabs(const cb2_mechanism &m);
+void free_trans_tabs(TransTabs *t);
 int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_boundary(const Zone &z, const Param &p, const FaceBC *faces, int n_faces, cudaStream_t s,
                     int &n_launch);
@@ -106,6 +109,9 @@ int launch_viscous(const Zone &z, const Param &p, const FaceBC *faces, int n_fac
 // the 8th-order node fluxes across one inner face of a multi-block grid (exchange_value task 1)
 int launch_inner_flux_exchange(const Zone &z, const Zone &zt, const Param &p, const cb2_inner_face &f,
                                cudaStream_t s, int &n_launch);
+// The mechanism repacked for the chemistry kernel (chem_tab.cuh), or null where it does not fit.
+ChemTabs *make_chem_tabs(const cb2_mechanism &m);
+void free_chem_tabs(ChemTabs *t);
 int launch_chemistry(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_shock_sensor(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_local_dt(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);

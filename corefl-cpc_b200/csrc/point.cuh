@@ -7,6 +7,7 @@
 #include "thermo.cuh"
 #include "thermo_2t.cuh"
 #include "transport.cuh"
+#include "transport_tab.cuh"
 
 namespace cb2 {
 
@@ -107,10 +108,12 @@ __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p
 // Physical properties of one node (update_physical_properties<mix>,
 // src/FieldOperation.cuh:183-247).  transport = false skips mu, kappa and rho*D of a mixture
 // (used by callers that take no viscous or diffusive term).
-// F32T: the transport coefficients in FP32 (the mixed form).
+// F32T: the transport coefficients in FP32 (the mixed form).  tab (with om, see
+// transport_properties_tab): the FP64 transport on the repacked mechanism.
 template <int NS, bool F32T = false>
 __device__ __forceinline__ void properties_point(const Zone &z, const Param &p, int i, int j, int k,
-                                                 bool transport = true) {
+                                                 bool transport = true, const TransTab<NS ? NS : 1> *tab = nullptr,
+                                                 double *om = nullptr, int om_stride = 0) {
   const idx_t g = z.L.at(i, j, k), sz = z.L.sz;
   const double t = z.bv[g + 5 * sz];
   const double V = norm3d(z.bv[g + sz], z.bv[g + 2 * sz], z.bv[g + 3 * sz]);
@@ -151,6 +154,7 @@ __device__ __forceinline__ void properties_point(const Zone &z, const Param &p, 
     if (!transport) return;
     double mu, kappa, rhoD[NS];
     if constexpr (F32T) transport_properties_f32<NS>(t, mw, y, cp, p.mech, mu, kappa, rhoD);
+    else if (tab) transport_properties_tab<NS>(t, mw, y, cp, *tab, om, om_stride, mu, kappa, rhoD);
     else transport_properties<NS>(t, z.bv[g + 4 * sz], mw, y, cp, p.mech, mu, kappa, rhoD);
     z.mul[g] = mu;
     z.kappa[g] = kappa;

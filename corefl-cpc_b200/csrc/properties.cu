@@ -3,16 +3,18 @@
 // src/TimeAdvanceFunc.cuh:28-127) and its global minimum (min_of_arr + global_time_step,
 // src/TimeAdvanceFunc.cu:114-164).
 #include <algorithm>
+#include <cmath>
 #include "point.cuh"
 #include "launch.h"
 
 namespace cb2 {
 
 constexpr int kPropThreads = 128;
+constexpr int kPropTabCtas = 4;  // CTAs per SM of the FP64 transport kernels: 128 registers
 
-// Bounded to 80 registers (6 CTAs of 128 threads per SM; the FP64 9-species transport otherwise
-// takes 163): the exponential and logarithm chains are latency-bound (192^3 H2/air box: 29.9 -> 20.7
-// ms per step).
+// Mixtures whose mechanism is not repacked, and the mixed form.  Bounded to 80 registers (6 CTAs of
+// 128 threads per SM; the FP64 9-species transport otherwise takes 163): the exponential and
+// logarithm chains are latency-bound (192^3 H2/air box: 29.9 -> 20.7 ms per step).
 template <int NS, bool F32T = false>
 __global__ void __launch_bounds__(kPropThreads, 6) k_properties(Zone z, Param p) {
   const int g_ = z.ngg;
@@ -22,19 +24,30 @@ __global__ void __launch_bounds__(kPropThreads, 6) k_properties(Zone z, Param p)
   properties_point<NS, F32T>(z, p, i, j, k);
 }
 
+// FP64 transport on the repacked mechanism (transport_tab.cuh).  A tile runs along the padded k
+// plane's nodes, so a ragged line leaves no idle threads; shared memory holds the distinct
+// collision integrals of each thread.
+template <int NS>
+__global__ void __launch_bounds__(kPropThreads, kPropTabCtas)
+k_properties_tab(const __grid_constant__ Zone z, const __grid_constant__ Param p, const __grid_constant__ TransTab<NS> m) {
+  extern __shared__ double s_om[];
+  const int g_ = z.ngg, px = z.mx + 2 * g_;
+  const int q = blockIdx.x * kPropThreads + threadIdx.x;
+  if (q >= px * (z.my + 2 * g_)) return;
+  const int j = q / px, i = q - j * px;
+  properties_point<NS>(z, p, i - g_, j - g_, (int)blockIdx.y - g_, true, &m, s_om + threadIdx.x, kPropThreads);
+}
+
 // A 2-D block (mz = 1) carries ngg ghost planes on each side of its one k plane.  The reference
 // evaluates the properties on every one of them (src/RK.cuh:230-235); after eliminate_k_gradient
 // their basic and scalar variables are copies of plane 0, so their properties are copies of
 // plane 0's, which is how they are filled here: the transport evaluation runs once per (i, j)
 // instead of 2 ngg + 1 times.  Only kappa_ve, which also depends on the plane's own T_ve (not
 // copied by eliminate_k_gradient), is re-evaluated where that differs.
-template <int NS, bool F32T = false>
-__global__ void __launch_bounds__(kPropThreads) k_properties_planar(Zone z, Param p) {
+// Copies of plane 0's properties of column (i, j) on the ghost planes.
+template <int NS>
+__device__ __forceinline__ void spread_properties(const Zone &z, const Param &p, int i, int j) {
   const int g_ = z.ngg;
-  const int i = blockIdx.x * kPropThreads + threadIdx.x - g_;
-  const int j = blockIdx.y - g_;
-  if (i >= z.mx + g_) return;
-  properties_point<NS, F32T>(z, p, i, j, 0);
   const idx_t sz = z.L.sz, g0 = z.L.at(i, j, 0);
   for (int kk = -g_; kk <= g_; ++kk) {
     if (kk == 0) continue;
@@ -69,6 +82,40 @@ __global__ void __launch_bounds__(kPropThreads) k_properties_planar(Zone z, Para
   }
 }
 
+template <int NS, bool F32T = false>
+__global__ void __launch_bounds__(kPropThreads) k_properties_planar(Zone z, Param p) {
+  const int g_ = z.ngg;
+  const int i = blockIdx.x * kPropThreads + threadIdx.x - g_;
+  const int j = blockIdx.y - g_;
+  if (i >= z.mx + g_) return;
+  properties_point<NS, F32T>(z, p, i, j, 0);
+  spread_properties<NS>(z, p, i, j);
+}
+
+template <int NS>
+__global__ void __launch_bounds__(kPropThreads, kPropTabCtas)
+k_properties_planar_tab(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                        const __grid_constant__ TransTab<NS> m) {
+  extern __shared__ double s_om[];
+  const int g_ = z.ngg, px = z.mx + 2 * g_;
+  const int q = blockIdx.x * kPropThreads + threadIdx.x;
+  if (q >= px * (z.my + 2 * g_)) return;
+  const int j = q / px, i = q - j * px;
+  properties_point<NS>(z, p, i - g_, j - g_, 0, true, &m, s_om + threadIdx.x, kPropThreads);
+  spread_properties<NS>(z, p, i - g_, j - g_);
+}
+
+template <int NS>
+static int launch_properties_tab(const Zone &z, const Param &p, const TransTab<NS> &m, bool planar, cudaStream_t s) {
+  const int g = z.ngg;
+  const int plane = (z.mx + 2 * g) * (z.my + 2 * g);
+  const dim3 grid((unsigned)((plane + kPropThreads - 1) / kPropThreads), (unsigned)(planar ? 1 : z.mz + 2 * g));
+  const size_t smem = sizeof(double) * m.n_red * kPropThreads;
+  if (planar) k_properties_planar_tab<NS><<<grid, kPropThreads, smem, s>>>(z, p, m);
+  else k_properties_tab<NS><<<grid, kPropThreads, smem, s>>>(z, p, m);
+  return check_launch();
+}
+
 int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_launch) {
   const int g = z.ngg;
   const bool planar = z.mz == 1 && p.dim == 2;
@@ -76,6 +123,9 @@ int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_laun
   dim3 grid((z.mx + 2 * g + kPropThreads - 1) / kPropThreads, z.my + 2 * g, planar ? 1 : z.mz + 2 * g);
   ++n_launch;
   ProfScope prof("properties", s);
+  const TransTabs *tab = mixed ? nullptr : p.mech.trans_tabs;
+  if (tab && p.n_spec == 9) return launch_properties_tab<9>(z, p, tab->t9, planar, s);
+  if (tab && p.n_spec == 5) return launch_properties_tab<5>(z, p, tab->t5, planar, s);
   switch (p.n_spec) {
     case 0:
       if (p.mu_constant > 0 && !z.mach) { --n_launch; return CB2_OK; }  // nothing changes
@@ -106,6 +156,61 @@ int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_laun
   }
   return check_launch();
 }
+
+// ---- repacking (host) ----------------------------------------------------------------------
+template <int NS>
+static bool fill_trans(const cb2_mechanism &m, TransTab<NS> &t) {
+  for (int a = 0; a < NS; ++a) {
+    t.imw[a] = 1.0 / m.mw[a];
+    t.mw[a] = 1.0 / t.imw[a];
+    t.gas[a] = kRu / m.mw[a];
+    t.vis_coeff[a] = m.vis_coeff[a];
+    t.lj_inv[a] = m.LJ_potent_inv[a];
+    if (!(t.lj_inv[a] > 0)) return false;
+    t.vis_a[a] = 1.147 * std::pow(t.lj_inv[a], -0.145);
+    t.geometry[a] = m.geometry[a] == 1 ? 1 : (m.geometry[a] == 2 ? 2 : 0);
+    t.zrot_pi[a] = 3.141592653589793 * m.ZRotF298[a];
+    t.bdc_r[a] = m.binary_diffusivity_coeff[a * NS + a] / t.gas[a];
+    for (int b = 0; b < NS; ++b) {
+      const double sq8 = m.sqrt_WiDivWjPl1Mul8[a * NS + b], bdc = m.binary_diffusivity_coeff[a * NS + b];
+      if (!(sq8 >= 0) || (a < b && !(bdc > 0))) return false;
+      t.sq[a][b] = std::sqrt(sq8);
+      t.w14[a][b] = m.WjDivWi_to_One4th[a * NS + b] * t.sq[a][b];
+      t.ibdc[a][b] = bdc > 0 ? 1.0 / bdc : 0.0;
+    }
+  }
+  t.n_red = 0;
+  for (int a = 0; a < NS; ++a)
+    for (int b = a; b < NS; ++b) {
+      const double k = m.kb_over_eps_jk[a * NS + b];
+      if (!(k > 0)) return false;
+      int u = 0;
+      while (u < t.n_red && t.kbe[u] != k) ++u;
+      if (u == t.n_red) {
+        t.kbe[u] = k;
+        t.om_a[u] = 1.0548 * std::pow(k, -0.15504);
+        ++t.n_red;
+      }
+      t.pair[a][b] = t.pair[b][a] = u;
+      if (a == b) t.kbe_inv[a] = 1.0 / k;
+    }
+  return true;
+}
+
+TransTabs *make_trans_tabs(const cb2_mechanism &m) {
+  if (!m.vis_coeff || !m.LJ_potent_inv || !m.geometry || !m.ZRotF298 || !m.binary_diffusivity_coeff ||
+      !m.kb_over_eps_jk || !m.sqrt_WiDivWjPl1Mul8 || !m.WjDivWi_to_One4th)
+    return nullptr;
+  TransTabs *t = new TransTabs{};
+  if (m.n_spec == 5 ? fill_trans<5>(m, t->t5) : m.n_spec == 9 && fill_trans<9>(m, t->t9)) {
+    t->ns = m.n_spec;
+    return t;
+  }
+  delete t;
+  return nullptr;
+}
+
+void free_trans_tabs(TransTabs *t) { delete t; }
 
 // ---- local time step --------------------------------------------------------------------
 template <int NS>

@@ -121,6 +121,7 @@ struct ReactorShared {
 // Species s as a one-species mechanism (for the per-species thermo of one lane).
 __device__ __forceinline__ Mech mech_species(const Mech &m, int s) {
   Mech o = m;
+  o.tab.use = 0;  // its rows are the whole mechanism's species
   o.t_low += s; o.t_mid += s; o.t_high += s;
   o.lo += 7 * s; o.hi += 7 * s;
   o.gas_const += s; o.imw += s; o.mw += s;
@@ -358,7 +359,7 @@ __device__ __forceinline__ double jacobian_entry(int r, int c, const ReactorShar
 }
 
 template <int NS, bool KRYLOV>
-__global__ void __launch_bounds__(32 * kReactorWarps) k_reactor_advance(cb2_reactor *R, int n, Mech m,
+__global__ void __launch_bounds__(32 * kReactorWarps) k_reactor_advance(cb2_reactor *R, int n, const __grid_constant__ Mech m,
                                                                         int max_attempts, double rtol, double atol) {
   using namespace rok4e;
   using SH = std::conditional_t<KRYLOV, KrylovShared<NS>, ReactorShared<NS>>;
@@ -530,7 +531,7 @@ __global__ void __launch_bounds__(32 * kReactorWarps) k_reactor_advance(cb2_reac
 // explicit three-stage Runge-Kutta, two more source evaluations at the stage temperatures); then
 // T by update_t, p, time += dt (:747-763).  dt is the reactor's h, left unchanged.
 template <int NS>
-__global__ void __launch_bounds__(32 * kReactorWarps) k_reactor_fixed(cb2_reactor *R, int n, Mech m, int max_steps,
+__global__ void __launch_bounds__(32 * kReactorWarps) k_reactor_fixed(cb2_reactor *R, int n, const __grid_constant__ Mech m, int max_steps,
                                                                       int scheme, bool conserve) {
   __shared__ ReactorShared<NS> smem[kReactorWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;

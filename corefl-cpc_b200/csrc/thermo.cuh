@@ -83,10 +83,37 @@ __device__ __forceinline__ void nasa9_gibbs_rt(double t, const Mech &m, double *
   }
 }
 
+// The same polynomials on the table that travels in the kernel's parameters, for t inside every
+// species' fit: the coefficients, scaled by the gas constant and the integration factors at upload,
+// are constant-bank operands of the Horner steps (one instruction each), where reading them from
+// memory costs as many loads as the arithmetic and the generic form divides by 3 per species.
+template <int NS>
+__device__ __forceinline__ void tab_h_cp(double t, const ThermoTab &m, double *h, double *cp) {
+  if (t < m.t_mid) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const double *a = m.h[0][s], *c = m.cp[0][s];
+      if (h) h[s] = fma(t, fma(t, fma(t, fma(t, fma(t, a[4], a[3]), a[2]), a[1]), c[0]), a[0]);
+      if (cp) cp[s] = fma(t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), c[0]);
+    }
+  } else {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const double *a = m.h[1][s], *c = m.cp[1][s];
+      if (h) h[s] = fma(t, fma(t, fma(t, fma(t, fma(t, a[4], a[3]), a[2]), a[1]), c[0]), a[0]);
+      if (cp) cp[s] = fma(t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), c[0]);
+    }
+  }
+}
+
 // h_k [J/kg] and cp_k [J/(kg K)] of every species at temperature t
 // (compute_enthalpy_and_cp, src/Thermo.cu:453-523).
 template <int NS>
 __device__ __forceinline__ void species_h_cp(double t, const Mech &m, double *h, double *cp) {
+  if (m.tab.use && t >= m.tab.t_low && t <= m.tab.t_high) {
+    tab_h_cp<NS>(t, m.tab, h, cp);
+    return;
+  }
   if (m.nasa9) {
     nasa9_h_cp<NS>(t, m, h, cp);
     return;
@@ -119,6 +146,10 @@ __device__ __forceinline__ void species_h_cp(double t, const Mech &m, double *h,
 // h_k only (compute_enthalpy, src/Thermo.cu:386-451).
 template <int NS>
 __device__ __forceinline__ void species_h(double t, const Mech &m, double *h) {
+  if (m.tab.use && t >= m.tab.t_low && t <= m.tab.t_high) {
+    tab_h_cp<NS>(t, m.tab, h, nullptr);
+    return;
+  }
   if (m.nasa9) {
     double cp[NS];
     nasa9_h_cp<NS>(t, m, h, cp);
@@ -149,6 +180,10 @@ __device__ __forceinline__ void species_h(double t, const Mech &m, double *h) {
 // cp_k only (compute_cp, src/Thermo.cu:525-574).
 template <int NS>
 __device__ __forceinline__ void species_cp(double t, const Mech &m, double *cp) {
+  if (m.tab.use && t >= m.tab.t_low && t <= m.tab.t_high) {
+    tab_h_cp<NS>(t, m.tab, nullptr, cp);
+    return;
+  }
   if (m.nasa9) {
     double h[NS];
     nasa9_h_cp<NS>(t, m, h, cp);
