@@ -73,6 +73,11 @@ struct FaceBC {
 int launch_inviscid_char(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_inviscid_comp(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_inviscid_pv(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
+// the FP64 sweeps of 5- and 9-species mixtures, one and two temperatures
+int launch_inviscid_pv_mix5(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
+int launch_inviscid_pv_mix9(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
+int launch_inviscid_pv_2t5(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
+int launch_inviscid_pv_2t9(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_inviscid_pv_f32(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_stage_update(const Zone &z, const Param &p, double dt, int rk, cudaStream_t s, int &n_launch);
 int launch_cv_from_bv(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);

@@ -2,6 +2,7 @@
 // takes by value, so that its constants are constant-bank operands.
 #pragma once
 #include "common.cuh"
+#include "rcp.cuh"
 
 namespace cb2 {
 
@@ -26,16 +27,6 @@ struct TransTabs {
   TransTab<5> t5;
   TransTab<9> t9;
 };
-
-// 1/x for positive normal x: the hardware's approximation (about 20 bits) and one third-order
-// Newton-Householder step, y (1 + e + e^2) with e = 1 - x y, whose error e^3 is below half an ulp.
-// A fifth of the operations of the IEEE division; the result is within one ulp of it.
-__device__ __forceinline__ double recip(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
 
 // om: NS (NS + 1) / 2 values of this thread, `stride` apart (shared memory: pair numbers index it).
 //

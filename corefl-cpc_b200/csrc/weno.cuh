@@ -13,6 +13,7 @@
 // from v[i-r+2 .. i+r] (v[r-2] is node i).  The interface value is plus + minus.
 #pragma once
 #include "common.cuh"
+#include "rcp.cuh"
 
 namespace cb2 {
 
@@ -140,77 +141,76 @@ __device__ __forceinline__ float rcp32(float x) { return __fdividef(1.0f, x); }
 // smoothness indicators: beta of minus sub-stencil r equals beta of plus sub-stencil
 // (last - r).  The pair costs one set of indicators instead of two.
 //   WENO5: v[0..4], v[2] = node n.   WENO7: v[0..6], v[3] = node n.
-template <typename T>
-__device__ __forceinline__ void weno5_node(const T *v, T eps, T &lp, T &rm) {
-  const T k6 = T(1.0 / 6);
-  const T q2 = k6 * (2 * v[2] + 5 * v[3] - v[4]);
-  const T q1 = k6 * (-v[1] + 5 * v[2] + 2 * v[3]);
-  const T q0 = k6 * (2 * v[0] - 7 * v[1] + 11 * v[2]);
-  const T m0 = k6 * (11 * v[2] - 7 * v[3] + 2 * v[4]);  // minus side, sub-stencil {n, n+1, n+2}
-  const T m1 = k6 * (2 * v[1] + 5 * v[2] - v[3]);
-  const T m2 = k6 * (-v[0] + 5 * v[1] + 2 * v[2]);
-  const T k13 = T(13.0 / 12);
-  const T b2 = k13 * sq(v[2] + v[4] - 2 * v[3]) + T(0.25) * sq(3 * v[2] - 4 * v[3] + v[4]);
-  const T b1 = k13 * sq(v[1] + v[3] - 2 * v[2]) + T(0.25) * sq(v[1] - v[3]);
-  const T b0 = k13 * sq(v[0] + v[2] - 2 * v[1]) + T(0.25) * sq(v[0] - 4 * v[1] + 3 * v[2]);
-  T D0 = sq(eps + b0), D1 = sq(eps + b1), D2 = sq(eps + b2);
-  T E0, E1, E2;  // weights of the sub-stencils up to a common factor
-  if constexpr (sizeof(T) == 4) {
-    const T A0 = eps + b0, A1 = eps + b1, A2 = eps + b2;
-    const T Am = fmin(fmin(A0, A1), A2);
-    E0 = sq(Am * rcp32(A0)); E1 = sq(Am * rcp32(A1)); E2 = sq(Am * rcp32(A2));
-  } else {
-    const T sc = binade_inv(fmax(fmax(D0, D1), D2));
-    D0 *= sc; D1 *= sc; D2 *= sc;
-    E2 = D0 * D1; E1 = D0 * D2; E0 = D1 * D2;  // prod of D over the other sub-stencils
-  }
-  const T w2 = T(0.3) * E2, w1 = T(0.6) * E1, w0 = T(0.1) * E0;
-  lp = (w2 * q2 + w1 * q1 + w0 * q0) / (w2 + w1 + w0);
-  const T u0 = T(0.1) * E2, u1 = T(0.6) * E1, u2 = T(0.3) * E0;
-  rm = (u0 * m0 + u1 * m1 + u2 * m2) / (u0 + u1 + u2);
+//
+// Both are written with the undivided differences of the stencil, d (first), s (second), t (third),
+// shared by the smoothness indicators, which are quadratic forms of them, and by the candidate
+// values, taken relative to node n.  That form needs 121 FP64 operations per WENO7 pair where the
+// sums over point values took about 190, and it is the more exact one (no cancellation of the node
+// values).  Sums of products are written as fused operations, so that every kernel that inlines
+// these functions rounds alike.  FP64 only; the FP32 pair is packed (below).
+__device__ __forceinline__ double pow2_inv_max(double a, double b, double c, double d) {
+  // the reciprocal binade of the largest: positive doubles order as their high words do
+  const int h = max(max(__double2hiint(a), __double2hiint(b)), max(__double2hiint(c), __double2hiint(d)));
+  return __hiloint2double(0x7FE00000 - (h & 0x7FF00000), 0);
 }
 
-template <typename T>
-__device__ __forceinline__ void weno7_node(const T *u, T eps, T &lp, T &rm) {
-  const T c0 = T(1.0 / 35), c1 = T(12.0 / 35), c2 = T(18.0 / 35), c3 = T(4.0 / 35);
-  const T q0 = -3 * u[0] + 13 * u[1] - 23 * u[2] + 25 * u[3];
-  const T q1 = u[1] - 5 * u[2] + 13 * u[3] + 3 * u[4];
-  const T q2 = -u[2] + 7 * u[3] + 7 * u[4] - u[5];
-  const T q3 = 3 * u[3] + 13 * u[4] - 5 * u[5] + u[6];
-  // minus side (the plus formulas on the mirrored stencil); m_r lives on plus sub-stencil 3-r
-  const T m0 = -3 * u[6] + 13 * u[5] - 23 * u[4] + 25 * u[3];
-  const T m1 = u[5] - 5 * u[4] + 13 * u[3] + 3 * u[2];
-  const T m2 = -u[4] + 7 * u[3] + 7 * u[2] - u[1];
-  const T m3 = 3 * u[3] + 13 * u[2] - 5 * u[1] + u[0];
-  const T k6 = T(1.0 / 6);
-  const T b0 = beta7(k6 * (-2 * u[0] + 9 * u[1] - 18 * u[2] + 11 * u[3]), -u[0] + 4 * u[1] - 5 * u[2] + 2 * u[3],
-                     -u[0] + 3 * u[1] - 3 * u[2] + u[3]);
-  const T d2m = u[2] - 2 * u[3] + u[4];
-  const T b1 = beta7(k6 * (u[1] - 6 * u[2] + 3 * u[3] + 2 * u[4]), d2m, -u[1] + 3 * u[2] - 3 * u[3] + u[4]);
-  const T b2 = beta7(k6 * (-2 * u[2] - 3 * u[3] + 6 * u[4] - u[5]), d2m, -u[2] + 3 * u[3] - 3 * u[4] + u[5]);
-  const T b3 = beta7(k6 * (-11 * u[3] + 18 * u[4] - 9 * u[5] + 2 * u[6]), 2 * u[3] - 5 * u[4] + 4 * u[5] - u[6],
-                     -u[3] + 3 * u[4] - 3 * u[5] + u[6]);
-  T tau = sq(b0 + 3 * b1 - 3 * b2 - b3);  // unchanged by the mirroring
-  T D0 = sq(eps + b0), D1 = sq(eps + b1), D2 = sq(eps + b2), D3 = sq(eps + b3);
-  T E0, E1, E2, E3;  // Z weights of the sub-stencils up to a common factor
-  if constexpr (sizeof(T) == 4) {
-    const T A0 = eps + b0, A1 = eps + b1, A2 = eps + b2, A3 = eps + b3;
-    const T Am = fmin(fmin(A0, A1), fmin(A2, A3));
-    const T rz = Am * rcp32(fabs(b0 + 3 * b1 - 3 * b2 - b3));
-    const T t = rcp32(1 + rz * rz), u = 1 - t;
-    E0 = u + t * sq(Am * rcp32(A0)); E1 = u + t * sq(Am * rcp32(A1));
-    E2 = u + t * sq(Am * rcp32(A2)); E3 = u + t * sq(Am * rcp32(A3));
-  } else {
-    const T sc = binade_inv(fmax(fmax(D0, D1), fmax(D2, D3)));
-    D0 *= sc; D1 *= sc; D2 *= sc; D3 *= sc; tau *= sc;
-    const T D01 = D0 * D1, D23 = D2 * D3;
-    E0 = (D0 + tau) * (D1 * D23); E1 = (D1 + tau) * (D0 * D23);
-    E2 = (D2 + tau) * (D01 * D3); E3 = (D3 + tau) * (D01 * D2);
-  }
-  const T w0 = c0 * E0, w1 = c1 * E1, w2 = c2 * E2, w3 = c3 * E3;
-  lp = T(1.0 / 12) * (w0 * q0 + w1 * q1 + w2 * q2 + w3 * q3) / (w0 + w1 + w2 + w3);
-  const T v0 = c0 * E3, v1 = c1 * E2, v2 = c2 * E1, v3 = c3 * E0;
-  rm = T(1.0 / 12) * (v0 * m0 + v1 * m1 + v2 * m2 + v3 * m3) / (v0 + v1 + v2 + v3);
+__device__ __forceinline__ void weno5_node(const double *v, double eps, double &lp, double &rm) {
+  const double d0 = v[1] - v[0], d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3];
+  const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
+  const double f0 = fma(0.5, s0, d1), f1 = fma(0.5, s1, d1), f2 = fma(-0.5, s2, d2);
+  const double k13 = 13.0 / 12;
+  double A0 = fma(f0, f0, fma(k13 * s0, s0, eps)), A1 = fma(f1, f1, fma(k13 * s1, s1, eps)),
+         A2 = fma(f2, f2, fma(k13 * s2, s2, eps));
+  const double sc = pow2_inv_max(A0, A1, A2, A2);
+  A0 *= sc; A1 *= sc; A2 *= sc;
+  const double D0 = A0 * A0, D1 = A1 * A1, D2 = A2 * A2;
+  // products of the D of the other sub-stencils, times ten times the linear weights
+  const double E0 = D1 * D2, E1 = 6.0 * (D0 * D2), E2 = D0 * D1;
+  const double k3 = 1.0 / 3, k6 = 1.0 / 6, h1 = 0.5 * d1, h2 = 0.5 * d2;
+  const double W2 = 3.0 * E2, V0 = 3.0 * E0;
+  const double np = fma(W2, fma(-k6, s2, h2), fma(E1, fma(k3, s1, h1), E0 * fma(k3, s0, h1)));
+  const double nm = fma(V0, fma(-k6, s0, -h1), fma(E1, fma(k3, s1, -h2), E2 * fma(k3, s2, -h2)));
+  lp = fma(np, recip(fma(3.0, E2, E0 + E1)), v[2]);
+  rm = fma(nm, recip(fma(3.0, E0, E2 + E1)), v[2]);
+}
+
+__device__ __forceinline__ void weno7_node(const double *u, double eps, double &lp, double &rm) {
+  const double d0 = u[1] - u[0], d1 = u[2] - u[1], d2 = u[3] - u[2], d3 = u[4] - u[3], d4 = u[5] - u[4],
+               d5 = u[6] - u[5];
+  const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2, s3 = d4 - d3, s4 = d5 - d4;
+  const double t0 = s1 - s0, t1 = s2 - s1, t2 = s3 - s2, t3 = s4 - s3;
+  // first and second derivatives of the sub-stencils' cubics at node n (the third are t0 .. t3)
+  const double k3 = 1.0 / 3, k6 = 1.0 / 6, k12 = 1.0 / 12;
+  const double c = fma(0.5, s2, d2);
+  const double f0 = fma(k3, t0, fma(0.5, s1, d2)), f1 = fma(-k6, t1, c), f2 = fma(-k6, t2, c),
+               f3 = fma(k3, t3, fma(-0.5, s3, d3));
+  const double g0 = s1 + t0, g3 = s3 - t3;
+  // A = eps + beta, beta = f^2 + f t / 12 + 13/12 g^2 + 1043/960 t^2
+  const double kg = 13.0 / 12, kt = 1043.0 / 960;
+  const double gm = (kg * s2) * s2;
+  const double b0 = fma(f0, fma(k12, t0, f0), fma(kt * t0, t0, (kg * g0) * g0));
+  const double b1 = fma(f1, fma(k12, t1, f1), fma(kt * t1, t1, gm));
+  const double b2 = fma(f2, fma(k12, t2, f2), fma(kt * t2, t2, gm));
+  const double b3 = fma(f3, fma(k12, t3, f3), fma(kt * t3, t3, (kg * g3) * g3));
+  double tz = fma(3.0, b1 - b2, b0 - b3);
+  double A0 = eps + b0, A1 = eps + b1, A2 = eps + b2, A3 = eps + b3;
+  const double sc = pow2_inv_max(A0, A1, A2, A3);
+  A0 *= sc; A1 *= sc; A2 *= sc; A3 *= sc; tz *= sc;
+  const double D0 = A0 * A0, D1 = A1 * A1, D2 = A2 * A2, D3 = A3 * A3;
+  // Z weights (1 + tau / D_s) times the product of every D
+  const double D01 = D0 * D1, D23 = D2 * D3;
+  const double E0 = fma(tz, tz, D0) * (D1 * D23), E1 = fma(tz, tz, D1) * (D0 * D23);
+  const double E2 = fma(tz, tz, D2) * (D01 * D3), E3 = fma(tz, tz, D3) * (D01 * D2);
+  // candidates relative to u[3]; linear weights times 35: 1, 12, 18, 4
+  const double h2 = 0.5 * d2, h3 = 0.5 * d3, e = fma(k3, s2, h2), em = fma(k3, s2, -h3);
+  const double w1 = 12.0 * E1, w2 = 18.0 * E2, v1 = 12.0 * E2, v2 = 18.0 * E1;
+  const double w3 = 4.0 * E3, v3 = 4.0 * E0;
+  const double np = fma(w3, fma(k12, t3, fma(-k6, s3, h3)),
+                        fma(w2, fma(-k12, t2, e), fma(w1, fma(-k12, t1, e), E0 * fma(0.25, t0, fma(k3, s1, h2)))));
+  const double nm = fma(v3, fma(-k12, t0, fma(-k6, s1, -h2)),
+                        fma(v2, fma(k12, t1, em), fma(v1, fma(k12, t2, em), E3 * fma(-0.25, t3, fma(k3, s3, -h3)))));
+  lp = fma(np, recip(fma(4.0, E3, fma(18.0, E2, fma(12.0, E1, E0)))), u[3]);
+  rm = fma(nm, recip(fma(4.0, E0, fma(18.0, E1, fma(12.0, E2, E3)))), u[3]);
 }
 
 // ---- packed FP32 node-centred pair ------------------------------------------------------
