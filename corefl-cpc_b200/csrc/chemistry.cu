@@ -31,74 +31,74 @@ struct ChemZone {
   double *dq, *rts;
 };
 
-// g/(RT) of every species into column tid of sg, each fit evaluated at the edge of its range
-// outside it.
+// g/(RT) of every species, each fit evaluated at the edge of its range outside it.
 template <int NS>
-__device__ __forceinline__ void tab_gibbs(const ChemTab<NS> &m, double t, double lnt, double it,
-                                          double (*sg)[kChemThreads], int tid) {
+__device__ __forceinline__ void tab_gibbs(const ChemTab<NS> &m, double t, double lnt, double it, double *g) {
   if (m.same_mid && t >= m.t_in_low && t <= m.t_in_high) {
     const double l1 = 1.0 - lnt;
     if (t < m.t_mid) {
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
         const double *c = m.g[0][s];
-        sg[s][tid] = fma(-t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), fma(c[0], l1, fma(c[5], it, -c[6])));
+        g[s] = fma(-t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), fma(c[0], l1, fma(c[5], it, -c[6])));
       }
     } else {
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
         const double *c = m.g[1][s];
-        sg[s][tid] = fma(-t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), fma(c[0], l1, fma(c[5], it, -c[6])));
+        g[s] = fma(-t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), fma(c[0], l1, fma(c[5], it, -c[6])));
       }
     }
   } else {
-#pragma unroll 1
+#pragma unroll
     for (int s = 0; s < NS; ++s) {
       const double tt = t < m.tl[s] ? m.tl[s] : (t > m.th[s] ? m.th[s] : t);
       const double lt = tt == t ? lnt : log(tt);
       // inside the fit the middle decides the range; outside it the edge's own range is taken
       const double *c = m.g[(tt == t ? t < m.tm[s] : t < m.tl[s]) ? 0 : 1][s];
-      sg[s][tid] = c[0] * (1.0 - lt) - tt * (c[1] + tt * (c[2] + tt * (c[3] + tt * c[4]))) + c[5] / tt - c[6];
+      g[s] = c[0] * (1.0 - lt) - tt * (c[1] + tt * (c[2] + tt * (c[3] + tt * c[4]))) + c[5] / tt - c[6];
     }
   }
 }
 
 // The source of one node per thread, J omega_k added to dq and the reaction time scale.
 //
-// Bound by the FP64 pipe: about 40 exponentials (18 pipe instructions each) and some 400 further
-// FP64 operations per node of the H2/air mechanism.  The table keeps everything else off the
-// critical resources: rate constants are constant-bank operands, zero stoichiometric coefficients
-// cost nothing (the dense loops over integer coefficients took four fifths of the time, most of it
-// in loads and in integer-to-double conversions), and kf / Kc is one exponential without a
-// division.  Concentrations and g/(RT) are indexed by species numbers read from the table, so they
-// live in shared memory, one column per thread (no bank conflicts).  The tile runs along the
-// k plane's nodes, not along one line, so a ragged mx leaves no idle threads.
+// Bound by the FP64 pipe and by issue: 40 exponentials and some 36 products with coefficient rows per
+// reaction and node.  Everything about the mechanism is a constant-bank read (the generic kernel spent
+// four fifths of its time on loads and integer-to-double conversions), kf / Kc is one exponential
+// without a division, Troe's powers of ten are exponentials of natural logarithms.  Sums over species
+// run over whole rows: skipping zero coefficients costs more in tests than the operations it saves.
+// Only the products of concentrations pick species by number, from shared memory (one column per
+// thread, no bank conflicts).  The tile runs along the k plane's nodes, not along one line, so a
+// ragged mx leaves no idle threads.
 template <int NS>
-__global__ void __launch_bounds__(kChemThreads, 5)
+__global__ void __launch_bounds__(kChemThreads, 4)
 k_chemistry_tab(const __grid_constant__ ChemZone z, const __grid_constant__ ChemTab<NS> m) {
-  __shared__ double sc[NS][kChemThreads], sg[NS][kChemThreads];
+  __shared__ double sc[NS + 1][kChemThreads];
   const int tid = threadIdx.x;
   const int q = blockIdx.x * kChemThreads + tid;
   if (q >= z.plane) return;
   const int j = q / z.mx, i = q - j * z.mx, k = blockIdx.y;
-  const idx_t g = z.L.at(i, j, k), sz = z.L.sz;
-  const double rho = z.bv[g], t = z.bv[g + 5 * sz];
+  const idx_t gn = z.L.at(i, j, k), sz = z.L.sz;
+  const double rho = z.bv[gn], t = z.bv[gn + 5 * sz];
+  double c[NS];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) sc[s][tid] = rho * z.sv[g + s * sz] * m.c_per_rho_y[s];
+  for (int s = 0; s < NS; ++s) sc[s][tid] = c[s] = rho * z.sv[gn + s * sz] * m.c_per_rho_y[s];
+  sc[NS][tid] = 1.0;
   const double lnt = log(t), it = 1.0 / t;
-  if (m.need_gibbs) tab_gibbs<NS>(m, t, lnt, it, sg, tid);
-  double cre[NS], des[NS];
+  double g[NS], net[NS], des[NS];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) cre[s] = des[s] = 0;
+  for (int s = 0; s < NS; ++s) g[s] = net[s] = des[s] = 0;
+  if (m.need_gibbs) tab_gibbs<NS>(m, t, lnt, it, g);
 #pragma unroll 1
   for (int r = 0; r < m.n_reac; ++r) {
-    const ChemReac &x = m.r[r];
+    const ChemReac<NS> &x = m.r[r];
     const int ty = x.type;
     double kf = x.A * exp(fma(x.b, lnt, -x.Ea * it));
     double cc = 0;
     if (ty > 3) {
 #pragma unroll
-      for (int s = 0; s < NS; ++s) cc = fma(sc[s][tid], x.tb[s], cc);
+      for (int s = 0; s < NS; ++s) cc = fma(c[s], x.tb[s], cc);
     }
     if (ty == 3) {
       kf += x.A2 * exp(fma(x.b2, lnt, -x.Ea2 * it));
@@ -114,66 +114,58 @@ k_chemistry_tab(const __grid_constant__ ChemZone z, const __grid_constant__ Chem
         if (ty > 5) {
           double fc = (1 - x.alpha) * exp(-t * x.it3) + x.alpha * exp(-t * x.it1);
           if (ty == 7) fc += exp(-x.t2 * it);
-          const double lfc = log10(fc);
+          constexpr double log10e = 0.43429448190325182765;
+          const double lnf = log(fc), lfc = lnf * log10e;
           const double cq = -0.4 - 0.67 * lfc, nq = 0.75 - 1.27 * lfc;
-          const double lp = log10(pr) + cq;
+          const double lp = fma(log(pr), log10e, cq);
           const double tmp = lp / (nq - 0.14 * lp);
-          F = pow(10.0, lfc / (1.0 + tmp * tmp));
+          F = exp(lnf / (1.0 + tmp * tmp));
         }
         kf = kf * pr / (1.0 + pr) * F;
       }
     }
-    double q1 = kf, q2 = 0;
     unsigned list = x.flist;
+    double q1 = kf * (sc[list & 15u][tid] * sc[list >> 4 & 15u][tid]), q2 = 0;
+    if (x.nf > 2) {
 #pragma unroll 1
-    for (int a = 0; a < x.nf; ++a, list >>= 4) q1 *= sc[list & 15u][tid];
+      for (int a = 2; a < x.nf; ++a) q1 *= sc[list >> (4 * a) & 15u][tid];
+    }
     if (x.back != kBackNone) {
       if (x.back == kBackEquilibrium) {
         // kb = kf / Kc, Kc = (p_atm / (R_u T) 1e-3)^order exp(-sum nu g/(RT))
         double dg = fma(x.order, lnt, -x.order_ln);
-        list = x.flist;
-#pragma unroll 1
-        for (int a = 0; a < x.nf; ++a, list >>= 4) dg -= sg[list & 15u][tid];
-        list = x.blist;
-#pragma unroll 1
-        for (int a = 0; a < x.nb; ++a, list >>= 4) dg += sg[list & 15u][tid];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) dg = fma(g[s], x.nu[s], dg);
         q2 = kf * exp(dg);
       } else {
         q2 = x.A2 * exp(fma(x.b2, lnt, -x.Ea2 * it));
         if (ty == 4) q2 *= cc;
       }
       list = x.blist;
+      q2 *= sc[list & 15u][tid] * sc[list >> 4 & 15u][tid];
+      if (x.nb > 2) {
 #pragma unroll 1
-      for (int a = 0; a < x.nb; ++a, list >>= 4) q2 *= sc[list & 15u][tid];
-    }
-#pragma unroll 1
-    for (int l = 0; l < x.levels; ++l) {
-      const unsigned mf = x.mf[l], mb = x.mb[l];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        if (mf >> s & 1u) {
-          des[s] += q1;
-          cre[s] += q2;
-        }
-        if (mb >> s & 1u) {
-          cre[s] += q1;
-          des[s] += q2;
-        }
+        for (int a = 2; a < x.nb; ++a) q2 *= sc[list >> (4 * a) & 15u][tid];
       }
     }
+    const double dq12 = q1 - q2;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      net[s] = fma(dq12, x.nu[s], net[s]);
+      des[s] = fma(q1, x.f[s], fma(q2, x.bk[s], des[s]));
+    }
   }
-  const double jac = z.jac[g];
+  const double jac = z.jac[gn];
   const idx_t g0 = q + (idx_t)k * z.plane;
   double ts = 1e+6;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    const double od = des[s] * m.w[s];
-    const double om = cre[s] * m.w[s] - od;
+    const double od = des[s] * m.w[s], om = net[s] * m.w[s];
     z.dq[g0 + (5 + s) * z.sz0] += jac * om;
-    const double y = z.sv[g + s * sz];
+    const double y = z.sv[gn + s * sz];
     if (y > 1e-25 && fabs(od) > 1e-25) ts = fmin(ts, fabs(rho * y / od));
   }
-  if (z.rts) z.rts[g] = ts;
+  if (z.rts) z.rts[gn] = ts;
 }
 
 template <int NS>
@@ -207,18 +199,19 @@ int launch_chemistry(const Zone &z, const Param &p, cudaStream_t s, int &n_launc
 // ---- repacking (host) --------------------------------------------------------------------------
 namespace {
 
-// Species lists and coefficient masks of one side of a reaction; false if they do not fit.
-bool pack_side(const int *stoi, int ns, unsigned &list, int &n, unsigned short *mask) {
+// The species of one side of a reaction, repeated by their coefficients and padded to two; false if
+// they do not fit.
+bool pack_side(const int *stoi, int ns, unsigned &list, int &n) {
   list = 0;
   n = 0;
   for (int s = 0; s < ns; ++s) {
-    if (stoi[s] < 0 || stoi[s] > kChemTabMult) return false;
+    if (stoi[s] < 0) return false;
     for (int a = 0; a < stoi[s]; ++a) {
       if (n == kChemTabList) return false;
       list |= (unsigned)s << (4 * n++);
-      mask[a] |= (unsigned short)(1u << s);
     }
   }
+  while (n < 2) list |= (unsigned)ns << (4 * n++);
   return true;
 }
 
@@ -245,11 +238,16 @@ bool fill_tab(const cb2_mechanism &m, ChemTab<NS> &t) {
     }
   }
   for (int r = 0; r < nr; ++r) {
-    ChemReac &x = t.r[r];
-    x = ChemReac{};
+    ChemReac<NS> &x = t.r[r];
+    x = ChemReac<NS>{};
     const int ty = m.reac_type[r], rev = m.rev_type[r];
-    if (!pack_side(m.stoi_f + r * NS, NS, x.flist, x.nf, x.mf) || !pack_side(m.stoi_b + r * NS, NS, x.blist, x.nb, x.mb))
+    if (!pack_side(m.stoi_f + r * NS, NS, x.flist, x.nf) || !pack_side(m.stoi_b + r * NS, NS, x.blist, x.nb))
       return false;
+    for (int s = 0; s < NS; ++s) {
+      x.f[s] = m.stoi_f[r * NS + s];
+      x.bk[s] = m.stoi_b[r * NS + s];
+      x.nu[s] = x.bk[s] - x.f[s];
+    }
     x.type = ty;
     x.back = ty == 0 ? kBackNone : rev == 1 ? kBackArrhenius : ty != 2 ? kBackEquilibrium : kBackNone;
     if (x.back == kBackEquilibrium) t.need_gibbs = 1;
@@ -266,8 +264,6 @@ bool fill_tab(const cb2_mechanism &m, ChemTab<NS> &t) {
       x.t2 = opt(m.troe_t2);
     }
     for (int s = 0; s < NS; ++s) x.tb[s] = m.third_body_coeff ? m.third_body_coeff[r * NS + s] : 0.0;
-    for (int l = 0; l < kChemTabMult; ++l)
-      if (x.mf[l] | x.mb[l]) x.levels = l + 1;
   }
   return true;
 }

@@ -27,6 +27,17 @@
 
 namespace cb2 {
 
+// One element from global to shared memory without passing through a register (4 or 8 bytes, so any
+// element is aligned).
+template <typename E>
+__device__ __forceinline__ void copy_async(E *dst, const E *src) {
+  static_assert(sizeof(E) == 4 || sizeof(E) == 8, "");
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const size_t g = __cvta_generic_to_global(src);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(g), "n"(sizeof(E)) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // A product rounded on its own (never fused into a following add).  The reciprocal-times
 // products below feed sums; pinning their rounding keeps every kernel that inlines these solvers
 // (the block sweeps, the batched kernels) bitwise identical.
@@ -518,26 +529,33 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
   const idx_t sz = L.sz;
 
   constexpr int NSB = NV + 4 + (SOLVER == CB2_INV_ROE ? 1 : 0);  // first node-flux slot (VF)
-  auto put = [&](int idx, const double *src) { sN[idx] = T(*src); };
+  // Node data goes to shared memory by asynchronous copies where it keeps its type: a thread's copies
+  // for all of its slots are in flight together and hold no registers (staging through registers
+  // waited for the first slot's loads before the halo's were issued; a batch of 96 small blocks
+  // 23.1 -> 15.4 ms, 257^3 sweeps 10.2 -> 10.1).
+  auto put = [&](int idx, const auto *src) {
+    if constexpr (sizeof(*src) == sizeof(T)) copy_async(sN + idx, src);
+    else sN[idx] = T(*src);
+  };
   auto load = [&](idx_t gi, int slot, int i, int j, int k) {
     if constexpr (VF) {
       if constexpr (sizeof(T) == 4) {
         const float *FL = DIR == 0 ? z.fF32 : (DIR == 1 ? z.gF32 : z.hF32);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sN[(NSB + c) * NN + slot] = FL[gi + (c + 1) * sz];
+        for (int c = 0; c < 4; ++c) put((NSB + c) * NN + slot, FL + gi + (c + 1) * sz);
       } else {
         const double *FL = DIR == 0 ? z.fF : (DIR == 1 ? z.gF : z.hF);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sN[(NSB + c) * NN + slot] = FL[gi + (c + 1) * sz];
+        for (int c = 0; c < 4; ++c) put((NSB + c) * NN + slot, FL + gi + (c + 1) * sz);
       }
     }
     if constexpr (sizeof(T) == 4) {
       // mixed form: the FP32 copies of bv, the metric and J
 #pragma unroll
-      for (int l = 0; l < 5; ++l) sN[l * NN + slot] = z.bv32[gi + l * sz];
+      for (int l = 0; l < 5; ++l) put(l * NN + slot, z.bv32 + gi + l * sz);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) sN[(NV + c) * NN + slot] = z.met32[gi + (3 * DIR + c) * sz];
-      sN[(NV + 3) * NN + slot] = z.met32[gi + 9 * sz];
+      for (int c = 0; c < 3; ++c) put((NV + c) * NN + slot, z.met32 + gi + (3 * DIR + c) * sz);
+      put((NV + 3) * NN + slot, z.met32 + gi + 9 * sz);
     } else {
 #pragma unroll
       for (int l = 0; l < 5; ++l) put(l * NN + slot, z.bv + gi + l * sz);
@@ -610,6 +628,7 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
   const bool rec = inside && n >= -1 && n <= ms;
   const bool face = rec && n <= ms - 1 && tpos < (DIR == 0 ? kSweepThreads : NSW) - 1;
   const bool upd = face && n >= 0 && tpos >= 1;
+  copy_async_wait();
   __syncthreads();
 
   T pl[NV + 2];

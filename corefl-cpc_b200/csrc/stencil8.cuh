@@ -28,8 +28,16 @@ __device__ __forceinline__ T d8(F f, int n, int nx, bool bl, bool br) {
          T(-1.0 / 280) * (f(4) - f(-4));
 }
 
+// The central stencil alone, for nodes away from every physical boundary.
+template <typename T, typename F>
+__device__ __forceinline__ T d8_central(F f) {
+  return T(0.8) * (f(1) - f(-1)) + T(-0.2) * (f(2) - f(-2)) + T(4.0 / 105) * (f(3) - f(-3)) +
+         T(-1.0 / 280) * (f(4) - f(-4));
+}
+
 struct BFlags {
   bool il, ir, jl, jr, kl, kr;
+  __device__ __forceinline__ bool any() const { return il | ir | jl | jr | kl | kr; }
 };
 
 __device__ __forceinline__ BFlags bflags(const Zone &z, int i, int j, int k) {

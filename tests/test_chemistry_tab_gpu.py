@@ -1,7 +1,7 @@
 """The block chemistry kernel on a repacked mechanism against the oracle: sizes around the edges of
 its tiles of 128 nodes of a k plane, temperatures in both ranges of the NASA7 fits, at their middle
 and beyond their ends, absent species, and the mechanisms that do not fit a table (more than 24
-reactions, a coefficient above 3), which run the generic kernel."""
+reactions, more than eight reactants), which run the generic kernel."""
 import copy
 import os
 
@@ -25,9 +25,9 @@ def mechanism(kind):
             a = np.asarray(d[name]).reshape(nr, -1)
             d[name] = np.concatenate([a, a[:8]]).reshape(-1).tolist()
         d["n_reac"] = nr + 8
-    elif kind == "steep":  # H + O2 -> O + OH with four H on the left
+    elif kind == "steep":  # H + O2 -> O + OH with ten H on the left
         a = np.asarray(d["stoi_f"]).reshape(nr, ns)
-        a[0, list(h2.species).index("H")] = 4
+        a[0, list(h2.species).index("H")] = 10
         d["stoi_f"] = a.reshape(-1).tolist()
     elif kind == "irreversible":  # no backward rate for some
         d["reac_type"][1] = d["reac_type"][16] = 0
