@@ -116,11 +116,9 @@ struct cb2_ctx {
   } sg;
   RunState *d_run = nullptr;  // time, t_end, dt, step counter of the graph loop
   // batched closed blocks (cb2_block_batch_*)
-  BlockCase *d_batch = nullptr;
-  int n_batch = 0;            // capacity of d_batch
-  int *d_queue = nullptr;     // work counter of the persistent batch grid
+  BatchStore batch;
   int batch_ni = kNI;         // y/z tile width of the batch kernel (cb2_block_batch_autotune)
-  int batch_cs = 8;           // CTAs per thread-block cluster sharing one batched block
+  int batch_cs = 8;           // kept for cb2_block_batch_set_schedule's callers; the batch has no clusters
   // multi-block steps: the per-block work of a stage runs on these streams concurrently, forked
   // from the caller's stream and joined back before anything that reads another block
   std::vector<cudaStream_t> branch;
@@ -578,8 +576,11 @@ void cb2_destroy(cb2_ctx *ctx) {
   if (ctx->sg.graph) cudaGraphDestroy(ctx->sg.graph);
   if (ctx->sg.capture) cudaStreamDestroy(ctx->sg.capture);
   cudaFree(ctx->d_run);
-  cudaFree(ctx->d_batch);
-  cudaFree(ctx->d_queue);
+  cudaFree(ctx->batch.cases);
+  cudaFree(ctx->batch.state);
+  cudaFree(ctx->batch.first);
+  cudaFree(ctx->batch.owner);
+  cudaFree(ctx->batch.n_active);
   for (auto &b : ctx->blocks) {
     cudaFree(b.d_btype);
     cudaFree(b.d_f32);
@@ -818,7 +819,9 @@ int cb2_rhs(cb2_ctx *ctx, int blk, unsigned mask, void *stream) {
                        ? 2
                        : 0;
   // no zeroing of dq when the first term assigns it, or when the caller's dq is added to
-  const bool assign = !accumulate && (pf.visc8_fused || (visc && viscous_assigns_dq(p)));
+  pf.assign_x = !accumulate && !visc && !((mask & CB2_RHS_CHEMISTRY) && p.reaction) && (mask & CB2_RHS_INVISCID) && pv &&
+                !B->z.sweep_mask;
+  const bool assign = !accumulate && (pf.visc8_fused || pf.assign_x || (visc && viscous_assigns_dq(p)));
   if (!assign && !accumulate) {
     ProfScope prof("zero_dq", s);
     CB2_TRY(check_cuda(cudaMemsetAsync(B->z.dq, 0, (size_t)B->z.L0.sz * p.n_var * sizeof(double), s)));
@@ -1360,13 +1363,14 @@ int cb2_reactor_advance_fixed(cb2_ctx *ctx, cb2_reactor *reactors, int n, int ma
 
 }  // extern "C"
 
-// Host records of a batch, largest block first (the persistent grid's work order), in
-// ctx->d_batch; order[pos] is the caller's index of record pos.
-static int build_block_batch(cb2_ctx *ctx, const cb2_block_case *cases, int n, std::vector<BlockCase> &h,
-                             std::vector<int> &order) {
+// Host records of a batch in the caller's order, the CTAs of every phase, and their device copies in
+// ctx->batch.
+static int build_block_batch(cb2_ctx *ctx, const cb2_block_case *cases, int n, int ni, std::vector<BlockState> &st,
+                             std::vector<int> &first, cudaStream_t s) {
   const Param &p = ctx->p;
   const int need_g = p.reconstruction == CB2_REC_WENO7 ? 4 : 3;
-  order.resize(n);
+  std::vector<BlockCase> h((size_t)n, BlockCase{});
+  st.assign(n, BlockState{});
   for (int i = 0; i < n; ++i) {
     const cb2_zone_view &v = cases[i].zone;
     if (v.mx < 1 || v.my < 1 || v.mz < 1 || v.ngg < need_g) return CB2_ERR_INVALID;
@@ -1376,48 +1380,50 @@ static int build_block_batch(cb2_ctx *ctx, const cb2_block_case *cases, int n, s
     const int ms[3] = {v.mx, v.my, v.mz};
     for (int d = 0; d < (v.mz > 1 ? 3 : 2); ++d)
       if (ms[d] < v.ngg + 2) return CB2_ERR_UNSUPPORTED;  // the periodic pair needs m >= g + 2
-    order[i] = i;
-  }
-  auto work = [&](int i) { return (long long)cases[i].zone.mx * cases[i].zone.my * cases[i].zone.mz; };
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work(a) > work(b); });
-  if (n > ctx->n_batch) {
-    cudaFree(ctx->d_batch);
-    ctx->d_batch = nullptr;
-    ctx->n_batch = 0;
-    CB2_TRY(check_cuda(cudaMalloc(&ctx->d_batch, sizeof(BlockCase) * n)));
-    ctx->n_batch = n;
-  }
-  if (!ctx->d_queue) CB2_TRY(check_cuda(cudaMalloc(&ctx->d_queue, sizeof(int))));
-  h.assign(n, BlockCase{});
-  for (int pos = 0; pos < n; ++pos) {
-    const cb2_block_case &c = cases[order[pos]];
-    BlockCase &b = h[pos];
-    b.z = make_zone(c.zone);
-    b.p = p;
-    b.p.dim = c.zone.mz == 1 ? 2 : 3;
-    b.p.status = &ctx->d_batch[pos].flags;
-    const int mx = c.zone.mx, my = c.zone.my, mz = c.zone.mz;
-    b.n_pairs = 0;
-    for (int d = 0; d < (mz > 1 ? 3 : 2); ++d) {
+    h[i].z = make_zone(v);
+    for (int d = 0; d < (v.mz > 1 ? 3 : 2); ++d) {
       // the low periodic face of direction d over the whole block (the register_face ranges)
-      FaceBC f{};
+      FaceBC &f = h[i].pairs[d];
       f.type = CB2_BC_PERIODIC;
       f.face = d;
       f.direction = -1;
-      f.end[0] = d == 0 ? 0 : mx - 1;
-      f.end[1] = d == 1 ? 0 : my - 1;
-      f.end[2] = d == 2 ? 0 : mz - 1;
-      b.pairs[b.n_pairs++] = f;
+      f.end[0] = d == 0 ? 0 : v.mx - 1;
+      f.end[1] = d == 1 ? 0 : v.my - 1;
+      f.end[2] = d == 2 ? 0 : v.mz - 1;
     }
-    b.time = c.time;
-    b.t_end = c.t_end;
-    b.dt_fixed = c.dt;
-    b.last_dt = 0.0;
-    b.steps = 0;
-    b.status = 0;
-    b.flags = 0u;
+    st[i].time = cases[i].time;
+    st[i].t_end = cases[i].t_end;
+    st[i].dt_fixed = cases[i].dt;
   }
-  return CB2_OK;
+  if (!batch_layout(h, ni, first)) return CB2_ERR_UNSUPPORTED;
+  long long owners = 0;
+  for (int ph = 0; ph < kBatchPhases; ++ph) owners += first[(size_t)ph * (n + 1) + n];
+  BatchStore &b = ctx->batch;
+  if (n > b.n_cap) {
+    cudaFree(b.cases);
+    cudaFree(b.state);
+    cudaFree(b.first);
+    b.cases = nullptr; b.state = nullptr; b.first = nullptr;
+    b.n_cap = 0;
+    CB2_TRY(check_cuda(cudaMalloc(&b.cases, sizeof(BlockCase) * n)));
+    CB2_TRY(check_cuda(cudaMalloc(&b.state, sizeof(BlockState) * n)));
+    CB2_TRY(check_cuda(cudaMalloc(&b.first, sizeof(int) * kBatchPhases * (n + 1))));
+    b.n_cap = n;
+  }
+  if (owners > b.owner_cap) {
+    cudaFree(b.owner);
+    b.owner = nullptr;
+    b.owner_cap = 0;
+    CB2_TRY(check_cuda(cudaMalloc(&b.owner, sizeof(int) * owners)));
+    b.owner_cap = owners;
+  }
+  if (!b.n_active) CB2_TRY(check_cuda(cudaMalloc(&b.n_active, sizeof(int))));
+  CB2_TRY(check_cuda(cudaMemcpyAsync(b.cases, h.data(), sizeof(BlockCase) * n, cudaMemcpyHostToDevice, s)));
+  CB2_TRY(check_cuda(cudaMemcpyAsync(b.state, st.data(), sizeof(BlockState) * n, cudaMemcpyHostToDevice, s)));
+  CB2_TRY(check_cuda(cudaMemcpyAsync(b.first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, s)));
+  int nl = 0;
+  CB2_TRY(launch_batch_owners(b, n, first, s, nl));
+  return count(ctx, nl);
 }
 
 extern "C" {
@@ -1426,22 +1432,23 @@ int cb2_block_batch_advance(cb2_ctx *ctx, cb2_block_case *cases, int n, int max_
   if (!ctx || (n > 0 && !cases) || n < 0 || max_steps < 0) return CB2_ERR_INVALID;
   if (!block_batch_supported(ctx->p)) return CB2_ERR_UNSUPPORTED;
   if (n == 0) return CB2_OK;
-  std::vector<BlockCase> h;
-  std::vector<int> order;
-  CB2_TRY(build_block_batch(ctx, cases, n, h, order));
-  ProfGuard pg(ctx);
   cudaStream_t s = (cudaStream_t)stream;
-  CB2_TRY(check_cuda(cudaMemcpyAsync(ctx->d_batch, h.data(), sizeof(BlockCase) * n, cudaMemcpyHostToDevice, s)));
-  CB2_TRY(launch_block_batch(ctx->d_batch, n, ctx->p, max_steps, 0, ctx->batch_ni, ctx->batch_cs, ctx->d_queue, s));
-  ++ctx->n_launch;
-  CB2_TRY(check_cuda(cudaMemcpyAsync(h.data(), ctx->d_batch, sizeof(BlockCase) * n, cudaMemcpyDeviceToHost, s)));
+  std::vector<BlockState> st;
+  std::vector<int> first;
+  CB2_TRY(build_block_batch(ctx, cases, n, ctx->batch_ni, st, first, s));
+  ProfGuard pg(ctx);
+  int nl = 0;
+  CB2_TRY(launch_block_batch(ctx->batch, n, first, ctx->p, max_steps, 0, ctx->batch_ni, s, nl));
+  count(ctx, nl);
+  CB2_TRY(check_cuda(cudaMemcpyAsync(st.data(), ctx->batch.state, sizeof(BlockState) * n, cudaMemcpyDeviceToHost, s)));
   CB2_TRY(check_cuda(cudaStreamSynchronize(s)));
-  for (int pos = 0; pos < n; ++pos) {
-    cb2_block_case &c = cases[order[pos]];
-    c.time = h[pos].time;
-    c.last_dt = h[pos].last_dt;
-    c.steps = h[pos].steps;
-    c.status = h[pos].status;
+  for (int i = 0; i < n; ++i) {
+    cb2_block_case &c = cases[i];
+    c.time = st[i].time;
+    c.last_dt = st[i].last_dt;
+    c.steps = st[i].steps;
+    c.status = (st[i].time >= st[i].t_end ? CB2_BLOCK_DONE : 0) |
+               ((st[i].status & CB2_BLOCK_FAILED) || st[i].flags ? CB2_BLOCK_FAILED : 0);
   }
   return CB2_OK;
 }
@@ -1450,39 +1457,33 @@ int cb2_block_batch_autotune(cb2_ctx *ctx, cb2_block_case *cases, int n, int *ti
   if (!ctx || (n > 0 && !cases) || n < 0) return CB2_ERR_INVALID;
   if (!block_batch_supported(ctx->p)) return CB2_ERR_UNSUPPORTED;
   if (n > 0) {
-    std::vector<BlockCase> h;
-    std::vector<int> order;
-    CB2_TRY(build_block_batch(ctx, cases, n, h, order));
+    std::vector<BlockState> st;
+    std::vector<int> first;
     cudaStream_t s = (cudaStream_t)stream;
-    CB2_TRY(check_cuda(cudaMemcpyAsync(ctx->d_batch, h.data(), sizeof(BlockCase) * n, cudaMemcpyHostToDevice, s)));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int rc = check_cuda(cudaEventCreate(&e0));
     if (rc == CB2_OK) rc = check_cuda(cudaEventCreate(&e1));
     float best_ms = 1e30f;
-    int best = kNI, best_cs = 8;
-    const int cluster[4] = {1, 2, 4, 8};
-    for (int c = 0; c < 3 && rc == CB2_OK; ++c)
-      for (int q = 0; q < 4 && rc == CB2_OK; ++q) {
-        const int ni = kTileNI[c], cs = cluster[q];
-        rc = launch_block_batch(ctx->d_batch, n, ctx->p, 0, 1, ni, cs, ctx->d_queue, s);  // warm-up
-        if (rc == CB2_OK) rc = check_cuda(cudaEventRecord(e0, s));
-        for (int r = 0; r < 2 && rc == CB2_OK; ++r)
-          rc = launch_block_batch(ctx->d_batch, n, ctx->p, 0, 1, ni, cs, ctx->d_queue, s);
-        if (rc == CB2_OK) rc = check_cuda(cudaEventRecord(e1, s));
-        if (rc == CB2_OK) rc = check_cuda(cudaEventSynchronize(e1));
-        float ms = 0;
-        if (rc == CB2_OK) rc = check_cuda(cudaEventElapsedTime(&ms, e0, e1));
-        if (rc == CB2_OK && ms < best_ms) {
-          best_ms = ms;
-          best = ni;
-          best_cs = cs;
-        }
+    int best = kNI, nl = 0;
+    for (int c = 0; c < 3 && rc == CB2_OK; ++c) {
+      const int ni = kTileNI[c];
+      rc = build_block_batch(ctx, cases, n, ni, st, first, s);
+      if (rc == CB2_OK) rc = launch_block_batch(ctx->batch, n, first, ctx->p, 0, 1, ni, s, nl);  // warm-up
+      if (rc == CB2_OK) rc = check_cuda(cudaEventRecord(e0, s));
+      for (int r = 0; r < 2 && rc == CB2_OK; ++r) rc = launch_block_batch(ctx->batch, n, first, ctx->p, 0, 1, ni, s, nl);
+      if (rc == CB2_OK) rc = check_cuda(cudaEventRecord(e1, s));
+      if (rc == CB2_OK) rc = check_cuda(cudaEventSynchronize(e1));
+      float ms = 0;
+      if (rc == CB2_OK) rc = check_cuda(cudaEventElapsedTime(&ms, e0, e1));
+      if (rc == CB2_OK && ms < best_ms) {
+        best_ms = ms;
+        best = ni;
       }
+    }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (rc != CB2_OK) return rc;
     ctx->batch_ni = best;
-    ctx->batch_cs = best_cs;
   }
   if (tile_ni_out) {
     tile_ni_out[0] = ctx->batch_ni;

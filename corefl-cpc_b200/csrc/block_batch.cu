@@ -1,14 +1,16 @@
-// Batched closed blocks: many 2-D / 3-D blocks of uneven size advanced by whole SSP-RK3 steps in
-// one persistent launch.  Each CTA takes the next block from a work queue ordered by decreasing
-// size, runs its steps with the block path's per-node functions (the sweep tiles of
-// inviscid_pv.cuh, stage_update_point, the periodic pair items of boundary.cuh,
-// properties_point), CTA barriers standing in for the kernel boundaries of cb2_rk3_step, and then
-// takes the next block.  The order of every phase is the block path's (RK3<mix>, src/RK.cuh:
-// 107-237 for an inviscid air case with periodic faces), so a block's results are bitwise those
-// of cb2_rk3_step on it.
+// Batched closed blocks: many 2-D / 3-D blocks of uneven size advanced by whole SSP-RK3 steps.  Every
+// phase of a step runs over the tiles or nodes of all blocks in one launch, with the block path's
+// per-node functions (the sweep tiles of inviscid_pv.cuh, stage_update_point, the periodic pair items
+// of boundary.cuh, properties_point), and the phases follow one another in the block path's order
+// (RK3<mix>, src/RK.cuh:107-237 for an inviscid air case with periodic faces), so a block's results
+// are bitwise those of cb2_rk3_step on it.
+//
+// The blocks differ in size (a factor of 37 between 12^3 and 40^3 nodes), so one thread-block cluster
+// per block left most of the GPU waiting for the largest: 96 such blocks, 1.7 M nodes, took 15.4 ms for
+// two steps.  With the tiles of all blocks in one grid the work is even whatever the sizes; the price
+// is a launch per phase (26 per step).
 #include <algorithm>
 #include <vector>
-#include <cooperative_groups.h>
 #include "point.cuh"
 #include "inviscid_pv.cuh"
 #include "boundary.cuh"
@@ -17,189 +19,290 @@
 
 namespace cb2 {
 
-__device__ __forceinline__ double cta_min(double v, double *red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_down_sync(0xffffffffu, v, o));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  double m = 1e+6;
-  for (int w = 0; w < kSweepThreads / 32; ++w) m = fmin(m, red[w]);
-  return m;
+namespace {
+
+constexpr int kBatchThreads = 256;
+
+// Work item of a CTA: its block and its number among the block's CTAs of this phase.
+struct BatchItem {
+  int c, t;
+};
+__device__ __forceinline__ BatchItem batch_item(const int *owner, const int *first) {
+  const int c = owner[blockIdx.x];
+  return {c, (int)blockIdx.x - first[c]};
 }
 
-// One phase: the y/z tiles of direction DIR over the whole block, tile t on cluster rank t % cs.
-template <int DIR, int REC, int SOLVER, int NI>
-__device__ __forceinline__ void sweep_yz(const Zone &z, const Param &p, unsigned char *smem, int rank, int cs) {
-  constexpr int NSW = kSweepThreads / NI;
-  const int nit = (z.mx + NI - 1) / NI;
-  const int ms = DIR == 1 ? z.my : z.mz;
-  const int nst = (ms + NSW - 3) / (NSW - 2);
-  const int other = DIR == 1 ? z.mz : z.my;
-  for (int t = rank; t < nit * nst * other; t += cs) {
-    const int bx = t % nit, r = t / nit;
-    pv_tile<double, 0, DIR, REC, SOLVER, NI>(z, p, 0, bx, r % nst, r / nst, smem);
+// The context's settings as one block of the batch sees them.
+__device__ __forceinline__ Param block_param(const Param &p0, const Zone &z, BlockState *st) {
+  Param p = p0;
+  p.dim = z.mz == 1 ? 2 : 3;
+  p.status = &st->flags;
+  return p;
+}
+
+__global__ void k_batch_owner(const int *first, int n, int total, int *owner) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  int lo = 0, hi = n - 1;  // the last block whose first tile is <= t
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (first[mid] <= t) lo = mid; else hi = mid - 1;
   }
+  owner[t] = lo;
 }
 
-// A thread-block cluster advances one block at a time: cluster rank 0 takes the next block from
-// the work queue, every phase spreads its tiles and nodes over the cluster's CTAs, and cluster
-// barriers (release/acquire at cluster scope, which orders the global-memory writes) separate
-// the phases.  All CTAs of a cluster follow the same control flow, so every barrier is reached
-// by all of them.  mode 0: whole steps; mode 1: only the residual of one stage, for timing.
-template <int REC, int SOLVER, int NI>
-__global__ void __launch_bounds__(kSweepThreads) k_block_batch(BlockCase *cases, int n_cases, int max_steps,
-                                                                int mode, int *queue) {
-  namespace cg = cooperative_groups;
+// Closes the step just taken (if any) and opens the next one.
+__global__ void k_batch_step(BlockState *state, int n, int close, int *n_active) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  BlockState &s = state[c];
+  if (close && s.active) {
+    if (s.bad) {
+      s.status |= CB2_BLOCK_FAILED;
+    } else {
+      const double dt = __longlong_as_double((long long)s.dt_bits);
+      s.time += dt;
+      s.last_dt = dt;
+      ++s.steps;
+    }
+  }
+  s.active = !(s.status & CB2_BLOCK_FAILED) && s.time < s.t_end;
+  s.bad = 0;
+  s.dt_bits = (unsigned long long)__double_as_longlong(s.dt_fixed > 0 ? s.dt_fixed : 1e+6);
+  if (s.active) atomicAdd(n_active, 1);
+}
+
+// qn <- cv of the padded block, and the CFL step's minimum over its interior nodes.
+__global__ void __launch_bounds__(kBatchThreads) k_batch_head(const BlockCase *cases, BlockState *state, const int *owner,
+                                                              const int *first, const __grid_constant__ Param p0) {
+  const BatchItem it = batch_item(owner, first);
+  BlockState &st = state[it.c];
+  if (!st.active) return;
+  const Zone &z = cases[it.c].z;
+  const long long e = (long long)it.t * kBatchThreads + threadIdx.x;
+  const int g = z.ngg, px = z.mx + 2 * g, py = z.my + 2 * g;
+  const idx_t sz = z.L.sz;
+  double m = 1e+6;
+  bool bad = false;
+  if (e < sz) {
+#pragma unroll
+    for (int l = 0; l < 5; ++l) z.qn[e + l * sz] = z.cv[e + l * sz];
+    const int i = (int)(e % px) - g;
+    const long long r = e / px;
+    const int j = (int)(r % py) - g, k = (int)(r / py) - g;
+    if (!(st.dt_fixed > 0) && i >= 0 && i < z.mx && j >= 0 && j < z.my && k >= 0 && k < z.mz) {
+      m = local_dt_point<0>(z, block_param(p0, z, &st), i, j, k);
+      bad = !(m > 0) || !isfinite(m);
+      if (bad) m = 1e+6;
+    }
+  }
+  if (st.dt_fixed > 0) return;
+  if (bad) st.bad = 1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && m < 1e+6) atomicMin(&st.dt_bits, (unsigned long long)__double_as_longlong(m));
+}
+
+// One sweep tile; the x sweep, the residual's first term, assigns dq (Param::assign_x).
+template <int DIR, int REC, int SOLVER, int NI>
+__global__ void __launch_bounds__(kSweepThreads, 4) k_batch_sweep(const BlockCase *cases, BlockState *state, const int *owner,
+                                                               const int *first, const __grid_constant__ Param p0) {
   extern __shared__ __align__(16) unsigned char bb_smem[];
-  __shared__ double red[kSweepThreads / 32];
-  __shared__ double s_part;
-  __shared__ int s_case;
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank(), cs = (int)cl.num_blocks();
-  const int tid = threadIdx.x, nt = kSweepThreads;
-  const long long g0 = (long long)rank * nt + tid, gs = (long long)cs * nt;  // cluster-wide thread index
-  for (;;) {
-    if (rank == 0 && tid == 0) s_case = atomicAdd(queue, 1);
-    cl.sync();
-    const int c = *cl.map_shared_rank(&s_case, 0);
-    cl.sync();  // every CTA has read the case before rank 0 takes the next one
-    if (c >= n_cases) return;
-    BlockCase &bc = cases[c];
-    if (bc.status) continue;
-    const Zone &z = bc.z;
-    const Param &p = bc.p;
-    constexpr int NV = 5;
-    const idx_t sz = z.L.sz, sz0 = z.L0.sz;
+  const BatchItem it = batch_item(owner, first);
+  BlockState &st = state[it.c];
+  if (!st.active || st.bad) return;
+  const Zone z = cases[it.c].z;
+  const Param p = block_param(p0, z, &st);
+  if constexpr (DIR == 0) {
     const idx_t run = (idx_t)z.L.my * z.L.disp2;
     const int ntx = (int)((run + (kSweepThreads - 2) - 1) / (kSweepThreads - 2));
-    const int g = z.ngg;
-    const int px = z.mx + 2 * g, py = z.my + 2 * g, pz = z.mz + 2 * g;
-    const long long npad = (long long)px * py * pz;
-    const long long nint = (long long)z.mx * z.my * z.mz;
-    auto residual = [&]() {
-      for (long long e = g0; e < sz0 * NV; e += gs) z.dq[e] = 0.0;
-      cl.sync();
-      for (int t = rank; t < ntx * z.mz; t += cs) pv_tile<double, 0, 0, REC, SOLVER>(z, p, run, t % ntx, 0, t / ntx, bb_smem);
-      cl.sync();
-      sweep_yz<1, REC, SOLVER, NI>(z, p, bb_smem, rank, cs);
-      cl.sync();
-      if (z.mz > 1) {
-        sweep_yz<2, REC, SOLVER, NI>(z, p, bb_smem, rank, cs);
-        cl.sync();
-      }
-    };
-    if (mode == 1) {
-      residual();
-      continue;
-    }
-    double time = bc.time;
-    int step = 0;
-    bool failed = false;
-    double last = bc.last_dt;
-    for (int s = 0; s < max_steps && time < bc.t_end; ++s) {
-      for (long long e = g0; e < sz * NV; e += gs) z.qn[e] = z.cv[e];
-      double dt = bc.dt_fixed;
-      if (!(dt > 0)) {
-        double m = 1e+6;
-        bool bad = false;
-        for (long long e = g0; e < nint; e += gs) {
-          const int i = (int)(e % z.mx), r = (int)(e / z.mx);
-          const double d = local_dt_point<0>(z, p, i, r % z.my, r / z.my);
-          bad |= !(d > 0) || !isfinite(d);
-          m = fmin(m, d);
-        }
-        m = cta_min(bad ? -1.0 : m, red);  // a bad step shows as a negative minimum
-        if (tid == 0) s_part = m;
-        cl.sync();
-        dt = 1e+6;
-        for (int r = 0; r < cs; ++r) dt = fmin(dt, *cl.map_shared_rank(&s_part, r));
-        cl.sync();  // the partial minima are read before they are written again
-        if (!(dt > 0)) {
-          failed = true;
-          break;
-        }
-      } else {
-        cl.sync();  // qn is copied before any stage update overwrites cv
-      }
-      for (int rk = 0; rk < 3; ++rk) {
-        residual();
-        for (long long e = g0; e < nint; e += gs) {
-          const int i = (int)(e % z.mx), r = (int)(e / z.mx);
-          stage_update_point<0>(z, p, dt, rk, i, r % z.my, r / z.my);
-        }
-        cl.sync();
-        for (int f = 0; f < bc.n_pairs; ++f) {
-          const FaceBC &fb = bc.pairs[f];
-          const long long items = (long long)(2 * g + 1) * (fb.end[0] - fb.start[0] + 1) *
-                                  (fb.end[1] - fb.start[1] + 1) * (fb.end[2] - fb.start[2] + 1);
-          for (long long t = g0; t < items; t += gs) bc_periodic_pair_item<0>(z, p, fb, t);
-          cl.sync();
-        }
-        if (p.dim == 2 && z.mz == 1) {
-          for (long long e = g0; e < (long long)px * py; e += gs)
-            eliminate_k_gradient_point(z, p, (int)(e % px) - g, (int)(e / px) - g);
-          cl.sync();
-        }
-        if (!(p.mu_constant > 0 && !z.mach)) {
-          for (long long e = g0; e < npad; e += gs) {
-            const int i = (int)(e % px) - g;
-            const long long r = e / px;
-            properties_point<0>(z, p, i, (int)(r % py) - g, (int)(r / py) - g);
-          }
-          cl.sync();
-        }
-      }
-      time += dt;
-      ++step;
-      last = dt;
-    }
-    cl.sync();
-    if (rank == 0 && tid == 0) {
-      bc.time = time;
-      bc.steps = step;
-      bc.last_dt = last;
-      int st = 0;
-      if (time >= bc.t_end) st |= CB2_BLOCK_DONE;
-      if (failed || bc.flags) st |= CB2_BLOCK_FAILED;
-      bc.status = st;
-    }
+    pv_tile<double, 0, 0, REC, SOLVER>(z, p, run, it.t % ntx, 0, it.t / ntx, bb_smem);
+  } else {
+    constexpr int NSW = kSweepThreads / NI;
+    const int nit = (z.mx + NI - 1) / NI, ms = DIR == 1 ? z.my : z.mz, nst = (ms + NSW - 3) / (NSW - 2);
+    const int bx = it.t % nit, r = it.t / nit;
+    pv_tile<double, 0, DIR, REC, SOLVER, NI>(z, p, 0, bx, r % nst, r / nst, bb_smem);
   }
 }
 
-template <int REC, int SOLVER, int NI>
-static int batch_launch(BlockCase *cases, int n, int max_steps, int mode, int cs, int *queue, cudaStream_t s) {
-  const size_t smem = std::max(pv_tile_smem<double, 0, REC, SOLVER>(0), pv_tile_smem<double, 0, REC, SOLVER>(1, NI));
-  auto kern = k_block_batch<REC, SOLVER, NI>;
+__global__ void __launch_bounds__(kBatchThreads) k_batch_update(const BlockCase *cases, BlockState *state, const int *owner,
+                                                                const int *first, const __grid_constant__ Param p0, int rk) {
+  const BatchItem it = batch_item(owner, first);
+  BlockState &st = state[it.c];
+  if (!st.active || st.bad) return;
+  const Zone &z = cases[it.c].z;
+  const long long e = (long long)it.t * kBatchThreads + threadIdx.x;
+  if (e >= z.L0.sz) return;
+  const int i = (int)(e % z.mx), r = (int)(e / z.mx);
+  stage_update_point<0>(z, block_param(p0, z, &st), __longlong_as_double((long long)st.dt_bits), rk, i, r % z.my,
+                        r / z.my);
+}
+
+__global__ void __launch_bounds__(kBatchThreads) k_batch_faces(const BlockCase *cases, BlockState *state, const int *owner,
+                                                               const int *first, const __grid_constant__ Param p0, int d) {
+  const BatchItem it = batch_item(owner, first);
+  BlockState &st = state[it.c];
+  if (!st.active || st.bad) return;
+  const Zone &z = cases[it.c].z;
+  bc_periodic_pair_item<0>(z, block_param(p0, z, &st), cases[it.c].pairs[d],
+                           (long long)it.t * kBatchThreads + threadIdx.x);
+}
+
+__global__ void __launch_bounds__(kBatchThreads) k_batch_columns(const BlockCase *cases, BlockState *state, const int *owner,
+                                                                 const int *first, const __grid_constant__ Param p0) {
+  const BatchItem it = batch_item(owner, first);
+  BlockState &st = state[it.c];
+  if (!st.active || st.bad) return;
+  const Zone &z = cases[it.c].z;
+  const int g = z.ngg, px = z.mx + 2 * g, py = z.my + 2 * g;
+  const long long e = (long long)it.t * kBatchThreads + threadIdx.x;
+  if (e >= (long long)px * py) return;
+  eliminate_k_gradient_point(z, block_param(p0, z, &st), (int)(e % px) - g, (int)(e / px) - g);
+}
+
+__global__ void __launch_bounds__(kBatchThreads) k_batch_properties(const BlockCase *cases, BlockState *state,
+                                                                    const int *owner, const int *first,
+                                                                    const __grid_constant__ Param p0) {
+  const BatchItem it = batch_item(owner, first);
+  BlockState &st = state[it.c];
+  if (!st.active || st.bad) return;
+  const Zone &z = cases[it.c].z;
+  if (p0.mu_constant > 0 && !z.mach) return;  // nothing changes
+  const int g = z.ngg, px = z.mx + 2 * g, py = z.my + 2 * g;
+  const long long e = (long long)it.t * kBatchThreads + threadIdx.x;
+  if (e >= z.L.sz) return;
+  const long long r = e / px;
+  properties_point<0>(z, block_param(p0, z, &st), (int)(e % px) - g, (int)(r % py) - g, (int)(r / py) - g);
+}
+
+// first: prefix sums on the host; off(ph): where phase ph's owners start.
+struct Batch {
+  const BatchStore &b;
+  int n;
+  const std::vector<int> &first;
+  cudaStream_t s;
+  int &nl;
+  int count(int ph) const { return first[(size_t)ph * (n + 1) + n]; }
+  const int *dfirst(int ph) const { return b.first + (size_t)ph * (n + 1); }
+  const int *owner(int ph) const {
+    long long o = 0;
+    for (int q = 0; q < ph; ++q) o += count(q);
+    return b.owner + o;
+  }
+};
+
+template <int DIR, int REC, int SOLVER, int NI>
+int sweep(const Batch &t, const Param &p) {
+  const int ph = DIR == 0 ? kTilesX : (DIR == 1 ? kTilesY : kTilesZ);
+  if (!t.count(ph)) return CB2_OK;
+  const size_t smem = pv_tile_smem<double, 0, REC, SOLVER>(DIR, NI);
+  auto kern = k_batch_sweep<DIR, REC, SOLVER, NI>;
   CB2_TRY(prepare_smem(kern, smem));
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(kSweepThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.gridDim = dim3((unsigned)cs);
-  int clusters = 0;
-  CB2_TRY(check_cuda(cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg)));
-  clusters = std::max(1, std::min(n, clusters));
-  cfg.gridDim = dim3((unsigned)(clusters * cs));
-  CB2_TRY(check_cuda(cudaMemsetAsync(queue, 0, sizeof(int), s)));
-  CB2_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kern, cases, n, max_steps, mode, queue)));
+  kern<<<t.count(ph), kSweepThreads, smem, t.s>>>(t.b.cases, t.b.state, t.owner(ph), t.dfirst(ph), p);
+  ++t.nl;
   return check_launch();
 }
 
+template <int REC, int SOLVER, int NI>
+int residual(const Batch &t, const Param &p) {
+  CB2_TRY((sweep<0, REC, SOLVER, kNI>(t, p)));
+  CB2_TRY((sweep<1, REC, SOLVER, NI>(t, p)));
+  return sweep<2, REC, SOLVER, NI>(t, p);
+}
+
+constexpr int kCheckSteps = 16;  // steps between looks at whether any block still runs
+
+template <int REC, int SOLVER, int NI>
+int run(const Batch &t, const Param &p0, int max_steps, int mode) {
+  const BatchStore &b = t.b;
+  Param p = p0;
+  p.assign_x = 1;
+  const int T = kBatchThreads, nb = (t.n + T - 1) / T;
+  auto open = [&](int close) {
+    CB2_TRY(check_cuda(cudaMemsetAsync(b.n_active, 0, sizeof(int), t.s)));
+    k_batch_step<<<nb, T, 0, t.s>>>(b.state, t.n, close, b.n_active);
+    ++t.nl;
+    return check_launch();
+  };
+  CB2_TRY(open(0));
+  if (mode == 1) return residual<REC, SOLVER, NI>(t, p);
+  for (int step = 0; step < max_steps; ++step) {
+    if (step > 0 && step % kCheckSteps == 0) {
+      int active = 0;
+      CB2_TRY(check_cuda(cudaMemcpyAsync(&active, b.n_active, sizeof(int), cudaMemcpyDeviceToHost, t.s)));
+      CB2_TRY(check_cuda(cudaStreamSynchronize(t.s)));
+      if (!active) break;
+    }
+    k_batch_head<<<t.count(kPadded), T, 0, t.s>>>(b.cases, b.state, t.owner(kPadded), t.dfirst(kPadded), p);
+    ++t.nl;
+    CB2_TRY(check_launch());
+    for (int rk = 0; rk < 3; ++rk) {
+      CB2_TRY((residual<REC, SOLVER, NI>(t, p)));
+      k_batch_update<<<t.count(kNodes), T, 0, t.s>>>(b.cases, b.state, t.owner(kNodes), t.dfirst(kNodes), p, rk);
+      ++t.nl;
+      for (int d = 0; d < 3; ++d) {
+        const int ph = kFacesX + d;
+        if (!t.count(ph)) continue;
+        k_batch_faces<<<t.count(ph), T, 0, t.s>>>(b.cases, b.state, t.owner(ph), t.dfirst(ph), p, d);
+        ++t.nl;
+      }
+      if (t.count(kColumns)) {
+        k_batch_columns<<<t.count(kColumns), T, 0, t.s>>>(b.cases, b.state, t.owner(kColumns), t.dfirst(kColumns), p);
+        ++t.nl;
+      }
+      k_batch_properties<<<t.count(kPadded), T, 0, t.s>>>(b.cases, b.state, t.owner(kPadded), t.dfirst(kPadded), p);
+      ++t.nl;
+      CB2_TRY(check_launch());
+    }
+    CB2_TRY(open(1));
+  }
+  return CB2_OK;
+}
+
 template <int REC, int SOLVER>
-static int batch_launch_ni(BlockCase *cases, int n, int max_steps, int mode, int ni, int cs, int *queue,
-                           cudaStream_t s) {
-  if (ni == 4) return batch_launch<REC, SOLVER, 4>(cases, n, max_steps, mode, cs, queue, s);
-  if (ni == 16) return batch_launch<REC, SOLVER, 16>(cases, n, max_steps, mode, cs, queue, s);
-  return batch_launch<REC, SOLVER, 8>(cases, n, max_steps, mode, cs, queue, s);
+int run_ni(const Batch &t, const Param &p, int max_steps, int mode, int ni) {
+  if (ni == 4) return run<REC, SOLVER, 4>(t, p, max_steps, mode);
+  if (ni == 16) return run<REC, SOLVER, 16>(t, p, max_steps, mode);
+  return run<REC, SOLVER, 8>(t, p, max_steps, mode);
+}
+
+}  // namespace
+
+bool batch_layout(const std::vector<BlockCase> &cases, int ni, std::vector<int> &first) {
+  const int n = (int)cases.size();
+  first.assign((size_t)kBatchPhases * (n + 1), 0);
+  long long total[kBatchPhases] = {};
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  for (int c = 0; c < n; ++c) {
+    const Zone &z = cases[c].z;
+    const int g = z.ngg, nsw = kSweepThreads / ni;
+    const long long px = z.mx + 2 * g, py = z.my + 2 * g;
+    const long long pairs[3] = {(long long)z.my * z.mz, (long long)z.mx * z.mz, (long long)z.mx * z.my};
+    long long k[kBatchPhases];
+    k[kTilesX] = up((long long)z.my * z.L.disp2, kSweepThreads - 2) * z.mz;
+    k[kTilesY] = up(z.mx, ni) * up(z.my, nsw - 2) * z.mz;
+    k[kTilesZ] = z.mz > 1 ? up(z.mx, ni) * up(z.mz, nsw - 2) * z.my : 0;
+    k[kNodes] = up(z.L0.sz, kBatchThreads);
+    k[kPadded] = up(z.L.sz, kBatchThreads);
+    for (int d = 0; d < 3; ++d) k[kFacesX + d] = d < 2 || z.mz > 1 ? up((2 * g + 1) * pairs[d], kBatchThreads) : 0;
+    k[kColumns] = z.mz == 1 ? up(px * py, kBatchThreads) : 0;
+    for (int ph = 0; ph < kBatchPhases; ++ph) {
+      total[ph] += k[ph];
+      if (total[ph] > 0x7fffffffLL) return false;
+      first[(size_t)ph * (n + 1) + c + 1] = (int)total[ph];
+    }
+  }
+  return true;
+}
+
+int launch_batch_owners(const BatchStore &b, int n, const std::vector<int> &first, cudaStream_t s, int &n_launch) {
+  const Batch t{b, n, first, s, n_launch};
+  for (int ph = 0; ph < kBatchPhases; ++ph) {
+    if (!t.count(ph)) continue;
+    k_batch_owner<<<(t.count(ph) + 255) / 256, 256, 0, s>>>(t.dfirst(ph), n, t.count(ph), const_cast<int *>(t.owner(ph)));
+    ++n_launch;
+  }
+  return check_launch();
 }
 
 bool block_batch_supported(const Param &p) {
@@ -208,17 +311,17 @@ bool block_batch_supported(const Param &p) {
          (p.inviscid_scheme == CB2_INV_AUSMP || p.inviscid_scheme == CB2_INV_HLLC);
 }
 
-int launch_block_batch(BlockCase *cases, int n, const Param &p, int max_steps, int mode, int ni, int cs,
-                       int *queue, cudaStream_t s) {
-  if (cs < 1 || cs > 8) return CB2_ERR_INVALID;
+int launch_block_batch(const BatchStore &b, int n, const std::vector<int> &first, const Param &p, int max_steps,
+                       int mode, int ni, cudaStream_t s, int &n_launch) {
   if (n <= 0) return CB2_OK;
   if (!block_batch_supported(p)) return CB2_ERR_UNSUPPORTED;
   ProfScope prof(mode == 1 ? "block_batch_residual" : "block_batch", s);
+  const Batch t{b, n, first, s, n_launch};
   const bool w7 = p.reconstruction == CB2_REC_WENO7, ausm = p.inviscid_scheme == CB2_INV_AUSMP;
-  if (w7 && ausm) return batch_launch_ni<7, CB2_INV_AUSMP>(cases, n, max_steps, mode, ni, cs, queue, s);
-  if (w7) return batch_launch_ni<7, CB2_INV_HLLC>(cases, n, max_steps, mode, ni, cs, queue, s);
-  if (ausm) return batch_launch_ni<5, CB2_INV_AUSMP>(cases, n, max_steps, mode, ni, cs, queue, s);
-  return batch_launch_ni<5, CB2_INV_HLLC>(cases, n, max_steps, mode, ni, cs, queue, s);
+  if (w7 && ausm) return run_ni<7, CB2_INV_AUSMP>(t, p, max_steps, mode, ni);
+  if (w7) return run_ni<7, CB2_INV_HLLC>(t, p, max_steps, mode, ni);
+  if (ausm) return run_ni<5, CB2_INV_AUSMP>(t, p, max_steps, mode, ni);
+  return run_ni<5, CB2_INV_HLLC>(t, p, max_steps, mode, ni);
 }
 
 }  // namespace cb2

@@ -139,6 +139,7 @@ struct Param {
   // J d(node flux)/d(its direction) (the viscous divergence), and the x sweep, the first writer
   // of the residual, assigns dq instead of adding to it
   int visc8_fused;
+  int assign_x;  // primitive sweeps: the x sweep is the residual's first term and assigns dq
   int limit_flow;
   double lf_ll[5], lf_ul[5];  // limit_flow bounds of rho, u, v, w, p
   double dt;                  // the current step's time step (positivity limiter)

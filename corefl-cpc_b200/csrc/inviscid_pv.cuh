@@ -692,6 +692,9 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
         if (first) z.dq[gd + v * sz0] = vis - inv;
         else z.dq[gd + v * sz0] = (z.dq[gd + v * sz0] + vis) - inv;
       }
+    } else if (DIR == 0 && p.assign_x) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) z.dq[gd + v * sz0] = -double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v)
