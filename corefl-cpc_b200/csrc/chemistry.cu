@@ -211,7 +211,8 @@ bool pack_side(const int *stoi, int ns, unsigned &list, int &n) {
       list |= (unsigned)s << (4 * n++);
     }
   }
-  while (n < 2) list |= (unsigned)ns << (4 * n++);
+  for (int a = n; a < kChemTabList; ++a) list |= (unsigned)ns << (4 * a);
+  n = std::max(n, 2);
   return true;
 }
 
@@ -243,6 +244,7 @@ bool fill_tab(const cb2_mechanism &m, ChemTab<NS> &t) {
     const int ty = m.reac_type[r], rev = m.rev_type[r];
     if (!pack_side(m.stoi_f + r * NS, NS, x.flist, x.nf) || !pack_side(m.stoi_b + r * NS, NS, x.blist, x.nb))
       return false;
+    t.list_len = std::max(t.list_len, std::max(x.nf, x.nb));
     for (int s = 0; s < NS; ++s) {
       x.f[s] = m.stoi_f[r * NS + s];
       x.bk[s] = m.stoi_b[r * NS + s];
@@ -270,20 +272,33 @@ bool fill_tab(const cb2_mechanism &m, ChemTab<NS> &t) {
 
 }  // namespace
 
+template <int NS>
+static bool upload_rows(const ChemTab<NS> &t, void *&rows) {
+  const size_t bytes = sizeof(ChemReac<NS>) * t.n_reac;
+  return cudaMalloc(&rows, bytes) == cudaSuccess &&
+         cudaMemcpy(rows, t.r, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+}
+
 ChemTabs *make_chem_tabs(const cb2_mechanism &m) {
   if (m.therm_nasa_7_9 == 9 || m.two_temperature_reaction_temperature || m.n_reac < 1 || m.n_reac > kChemTabReac ||
       !m.reac_type || !m.rev_type || !m.stoi_f || !m.stoi_b || !m.A || !m.b || !m.Ea)
     return nullptr;
   ChemTabs *t = new ChemTabs{};
-  const bool ok = m.n_spec == 5 ? fill_tab<5>(m, t->t5) : m.n_spec == 9 && fill_tab<9>(m, t->t9);
+  const bool ok = m.n_spec == 5 ? fill_tab<5>(m, t->t5) && upload_rows(t->t5, t->rows)
+                                : m.n_spec == 9 && fill_tab<9>(m, t->t9) && upload_rows(t->t9, t->rows);
   if (ok) {
     t->ns = m.n_spec;
     return t;
   }
-  delete t;
+  cudaGetLastError();  // without a table the generic kernels run
+  free_chem_tabs(t);
   return nullptr;
 }
 
-void free_chem_tabs(ChemTabs *t) { delete t; }
+void free_chem_tabs(ChemTabs *t) {
+  if (!t) return;
+  cudaFree(t->rows);
+  delete t;
+}
 
 }  // namespace cb2

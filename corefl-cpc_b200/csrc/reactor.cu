@@ -621,6 +621,12 @@ __global__ void __launch_bounds__(32 * kReactorWarps) k_reactor_fixed(cb2_reacto
   }
 }
 
+}  // namespace cb2
+
+#include "reactor_rok4e.cuh"
+
+namespace cb2 {
+
 int launch_reactor_fixed(const Param &p, cb2_reactor *r, int n, int max_steps, int scheme, cudaStream_t s) {
   const int form = scheme & 0xf;
   const bool conserve = (scheme & CB2_REACTOR_CONSERVE_MASS) != 0;
@@ -654,6 +660,17 @@ int launch_reactor_advance(const Param &p, cb2_reactor *r, int n, int max_attemp
   const unsigned blocks = (unsigned)((n + kReactorWarps - 1) / kReactorWarps);
   ProfScope prof(krylov ? "reactor_advance_krylov" : "reactor_advance", s);
   const unsigned th = 32 * kReactorWarps;
+  const ChemTabs *tab = !krylov && p.mech.tab.use ? p.mech.chem_tabs : nullptr;
+  if (tab && tab->ns == 9) {
+    k_reactor_rok4e<9><<<blocks, th, 0, s>>>(r, n, p.mech, tab->t9, static_cast<const ChemReac<9> *>(tab->rows),
+                                             max_attempts, rtol, atol);
+    return check_launch();
+  }
+  if (tab && tab->ns == 5) {
+    k_reactor_rok4e<5><<<blocks, th, 0, s>>>(r, n, p.mech, tab->t5, static_cast<const ChemReac<5> *>(tab->rows),
+                                             max_attempts, rtol, atol);
+    return check_launch();
+  }
   switch (p.n_spec * 2 + (krylov ? 1 : 0)) {
     case 10: k_reactor_advance<5, false><<<blocks, th, 0, s>>>(r, n, p.mech, max_attempts, rtol, atol); break;
     case 11: k_reactor_advance<5, true><<<blocks, th, 0, s>>>(r, n, p.mech, max_attempts, rtol, atol); break;
