@@ -99,8 +99,6 @@ struct cb2_ctx {
   ChemTabs *chem_tabs = nullptr;  // the mechanism repacked for the chemistry kernel (host)
   unsigned *d_status = nullptr;
   double *d_dtmin = nullptr;     // running min of the CFL dt
-  double *d_partial = nullptr;   // per-CTA partial minima of the reduction
-  int n_partial = 0;
   std::vector<Block> blocks;
   unsigned long long n_launch = 0;
   Profiler *prof = nullptr;  // non-null while profiling is enabled
@@ -590,7 +588,6 @@ void cb2_destroy(cb2_ctx *ctx) {
   free_trans_tabs(ctx->trans_tabs);
   cudaFree(ctx->d_tables);
   cudaFree(ctx->d_status);
-  cudaFree(ctx->d_partial);
   delete ctx->prof;
   delete ctx;
 }
@@ -744,15 +741,6 @@ int cb2_bind_block(cb2_ctx *ctx, int blk, const cb2_zone_view *v, const cb2_face
   B.z.bt.jr = base + off; off += jr.size();
   B.z.bt.kl = base + off; off += kl.size();
   B.z.bt.kr = base + off;
-  // reduction scratch sized for the largest bound block
-  const int np = min_reduce_partials((long long)mx * my * mz);
-  if (np > ctx->n_partial) {
-    cudaFree(ctx->d_partial);
-    ctx->d_partial = nullptr;
-    e = cudaMalloc(&ctx->d_partial, np * sizeof(double));
-    if (e != cudaSuccess) { ctx->n_partial = 0; return fail_cuda(e); }
-    ctx->n_partial = np;
-  }
   if (p.precision == CB2_PREC_MIXED) {
     // FP32 copies: bv (refreshed per residual) and metric + J (snapshot of the bound block)
     const size_t sz = (size_t)B.z.L.sz;
@@ -899,13 +887,17 @@ int cb2_shock_sensor(cb2_ctx *ctx, int blk, void *stream) {
   return count(ctx, nl);
 }
 
-int cb2_stage_update(cb2_ctx *ctx, int blk, double dt, int rk, void *stream) {
+static int stage_update(cb2_ctx *ctx, int blk, double dt, int rk, bool first, void *stream) {
   Block *B = get_block(ctx, blk);
   if (!B || rk < 0 || rk > 2) return CB2_ERR_INVALID;
   ProfGuard pg(ctx);
   int nl = 0;
-  CB2_TRY(launch_stage_update(B->z, ctx->p, dt, rk, (cudaStream_t)stream, nl));
+  CB2_TRY(launch_stage_update(B->z, ctx->p, dt, rk, (cudaStream_t)stream, nl, first));
   return count(ctx, nl);
+}
+
+int cb2_stage_update(cb2_ctx *ctx, int blk, double dt, int rk, void *stream) {
+  return stage_update(ctx, blk, dt, rk, false, stream);
 }
 
 int cb2_autotune(cb2_ctx *ctx, int blk, int *tile_ni_out, void *stream) {
@@ -1086,9 +1078,7 @@ static int enqueue_cfl_dt(cb2_ctx *ctx, cudaStream_t s) {
   for (auto &B : ctx->blocks) {
     if (!B.bound) continue;
     if (!B.z.dtl) return CB2_ERR_INVALID;
-    CB2_TRY(launch_local_dt(B.z, ctx->p, s, nl));
-    const long long n = (long long)B.z.mx * B.z.my * B.z.mz;
-    CB2_TRY(launch_min_reduce(B.z.dtl, n, ctx->d_partial, min_reduce_partials(n), ctx->d_dtmin, s, nl));
+    CB2_TRY(launch_local_dt(B.z, ctx->p, ctx->d_dtmin, s, nl));
   }
   return count(ctx, nl);
 }
@@ -1108,11 +1098,10 @@ int cb2_cfl_dt(cb2_ctx *ctx, double *dt_out, void *stream) {
 
 }  // extern "C"
 
-// qn <- cv and the shock sensor of every bound block: the part of a step before its dt.
+// The shock sensor of every bound block: the part of a step before its dt.  (qn <- cv rides on stage
+// 0's update.)
 static int enqueue_step_head(cb2_ctx *ctx, void *stream) {
   const int nb = (int)ctx->blocks.size();
-  for (int b = 0; b < nb; ++b)
-    if (ctx->blocks[b].bound) CB2_TRY(cb2_store_qn(ctx, b, stream));
   if (ctx->p.sensor_threshold > 1e-10)  // hybrid linear/WENO weights (src/RK.cuh:139-143)
     for (int b = 0; b < nb; ++b)
       if (ctx->blocks[b].bound) CB2_TRY(cb2_shock_sensor(ctx, b, stream));
@@ -1178,7 +1167,7 @@ static int enqueue_stages(cb2_ctx *ctx, double dt, void *stream) {
       if (!ctx->blocks[b].bound) continue;
       void *sb = on(slot++);
       CB2_TRY(cb2_rhs(ctx, b, mask, sb));
-      CB2_TRY(cb2_stage_update(ctx, b, dt, rk, sb));
+      CB2_TRY(stage_update(ctx, b, dt, rk, rk == 0, sb));
       CB2_TRY(cb2_boundary(ctx, b, sb));
     }
     if (nbr) CB2_TRY(join_branches(ctx, s, nbr));

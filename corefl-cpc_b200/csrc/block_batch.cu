@@ -53,6 +53,7 @@ __global__ void k_batch_owner(const int *first, int n, int total, int *owner) {
 
 // Closes the step just taken (if any) and opens the next one.
 __global__ void k_batch_step(BlockState *state, int n, int close, int *n_active) {
+  chain_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   BlockState &s = state[c];
@@ -75,6 +76,7 @@ __global__ void k_batch_step(BlockState *state, int n, int close, int *n_active)
 // qn <- cv of the padded block, and the CFL step's minimum over its interior nodes.
 __global__ void __launch_bounds__(kBatchThreads) k_batch_head(const BlockCase *cases, BlockState *state, const int *owner,
                                                               const int *first, const __grid_constant__ Param p0) {
+  chain_begin();
   const BatchItem it = batch_item(owner, first);
   BlockState &st = state[it.c];
   if (!st.active) return;
@@ -108,6 +110,7 @@ template <int DIR, int REC, int SOLVER, int NI>
 __global__ void __launch_bounds__(kSweepThreads, 4) k_batch_sweep(const BlockCase *cases, BlockState *state, const int *owner,
                                                                const int *first, const __grid_constant__ Param p0) {
   extern __shared__ __align__(16) unsigned char bb_smem[];
+  chain_begin();
   const BatchItem it = batch_item(owner, first);
   BlockState &st = state[it.c];
   if (!st.active || st.bad) return;
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_batch_sweep(const BlockCas
 
 __global__ void __launch_bounds__(kBatchThreads) k_batch_update(const BlockCase *cases, BlockState *state, const int *owner,
                                                                 const int *first, const __grid_constant__ Param p0, int rk) {
+  chain_begin();
   const BatchItem it = batch_item(owner, first);
   BlockState &st = state[it.c];
   if (!st.active || st.bad) return;
@@ -140,6 +144,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_update(const BlockCase 
 
 __global__ void __launch_bounds__(kBatchThreads) k_batch_faces(const BlockCase *cases, BlockState *state, const int *owner,
                                                                const int *first, const __grid_constant__ Param p0, int d) {
+  chain_begin();
   const BatchItem it = batch_item(owner, first);
   BlockState &st = state[it.c];
   if (!st.active || st.bad) return;
@@ -150,6 +155,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_faces(const BlockCase *
 
 __global__ void __launch_bounds__(kBatchThreads) k_batch_columns(const BlockCase *cases, BlockState *state, const int *owner,
                                                                  const int *first, const __grid_constant__ Param p0) {
+  chain_begin();
   const BatchItem it = batch_item(owner, first);
   BlockState &st = state[it.c];
   if (!st.active || st.bad) return;
@@ -163,6 +169,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_columns(const BlockCase
 __global__ void __launch_bounds__(kBatchThreads) k_batch_properties(const BlockCase *cases, BlockState *state,
                                                                     const int *owner, const int *first,
                                                                     const __grid_constant__ Param p0) {
+  chain_begin();
   const BatchItem it = batch_item(owner, first);
   BlockState &st = state[it.c];
   if (!st.active || st.bad) return;
@@ -198,9 +205,9 @@ int sweep(const Batch &t, const Param &p) {
   const size_t smem = pv_tile_smem<double, 0, REC, SOLVER>(DIR, NI);
   auto kern = k_batch_sweep<DIR, REC, SOLVER, NI>;
   CB2_TRY(prepare_smem(kern, smem));
-  kern<<<t.count(ph), kSweepThreads, smem, t.s>>>(t.b.cases, t.b.state, t.owner(ph), t.dfirst(ph), p);
   ++t.nl;
-  return check_launch();
+  return launch_chain(kern, t.count(ph), kSweepThreads, smem, t.s, (const BlockCase *)t.b.cases, t.b.state, t.owner(ph),
+                      t.dfirst(ph), p);
 }
 
 template <int REC, int SOLVER, int NI>
@@ -220,7 +227,7 @@ int run(const Batch &t, const Param &p0, int max_steps, int mode) {
   const int T = kBatchThreads, nb = (t.n + T - 1) / T;
   auto open = [&](int close) {
     CB2_TRY(check_cuda(cudaMemsetAsync(b.n_active, 0, sizeof(int), t.s)));
-    k_batch_step<<<nb, T, 0, t.s>>>(b.state, t.n, close, b.n_active);
+    CB2_TRY(launch_chain(k_batch_step, nb, T, 0, t.s, b.state, t.n, close, b.n_active));
     ++t.nl;
     return check_launch();
   };
@@ -233,24 +240,24 @@ int run(const Batch &t, const Param &p0, int max_steps, int mode) {
       CB2_TRY(check_cuda(cudaStreamSynchronize(t.s)));
       if (!active) break;
     }
-    k_batch_head<<<t.count(kPadded), T, 0, t.s>>>(b.cases, b.state, t.owner(kPadded), t.dfirst(kPadded), p);
+    CB2_TRY(launch_chain(k_batch_head, t.count(kPadded), T, 0, t.s, (const BlockCase *)b.cases, b.state, t.owner(kPadded), t.dfirst(kPadded), p));
     ++t.nl;
     CB2_TRY(check_launch());
     for (int rk = 0; rk < 3; ++rk) {
       CB2_TRY((residual<REC, SOLVER, NI>(t, p)));
-      k_batch_update<<<t.count(kNodes), T, 0, t.s>>>(b.cases, b.state, t.owner(kNodes), t.dfirst(kNodes), p, rk);
+      CB2_TRY(launch_chain(k_batch_update, t.count(kNodes), T, 0, t.s, (const BlockCase *)b.cases, b.state, t.owner(kNodes), t.dfirst(kNodes), p, rk));
       ++t.nl;
       for (int d = 0; d < 3; ++d) {
         const int ph = kFacesX + d;
         if (!t.count(ph)) continue;
-        k_batch_faces<<<t.count(ph), T, 0, t.s>>>(b.cases, b.state, t.owner(ph), t.dfirst(ph), p, d);
+        CB2_TRY(launch_chain(k_batch_faces, t.count(ph), T, 0, t.s, (const BlockCase *)b.cases, b.state, t.owner(ph), t.dfirst(ph), p, d));
         ++t.nl;
       }
       if (t.count(kColumns)) {
-        k_batch_columns<<<t.count(kColumns), T, 0, t.s>>>(b.cases, b.state, t.owner(kColumns), t.dfirst(kColumns), p);
+        CB2_TRY(launch_chain(k_batch_columns, t.count(kColumns), T, 0, t.s, (const BlockCase *)b.cases, b.state, t.owner(kColumns), t.dfirst(kColumns), p));
         ++t.nl;
       }
-      k_batch_properties<<<t.count(kPadded), T, 0, t.s>>>(b.cases, b.state, t.owner(kPadded), t.dfirst(kPadded), p);
+      CB2_TRY(launch_chain(k_batch_properties, t.count(kPadded), T, 0, t.s, (const BlockCase *)b.cases, b.state, t.owner(kPadded), t.dfirst(kPadded), p));
       ++t.nl;
       CB2_TRY(check_launch());
     }

@@ -14,6 +14,7 @@
 //   wall     : no-slip, non-catalytic, adiabatic or isothermal (apply_wall,
 //              src/BoundCond.cu:3055-3389)
 // Every filled node gets its cv recomputed (compute_cv_from_bv_1_point, FieldOperation.cuh:163).
+#include <algorithm>
 #include "point.cuh"
 #include "launch.h"
 #include "boundary.cuh"
@@ -64,8 +65,16 @@ __device__ __forceinline__ double node_gamma(const Zone &z, const Param &p, idx_
   }
 }
 
+// The outflow faces of a block that one launch fills: blockIdx.y picks the face.
+struct FaceSet {
+  FaceBC f[6];
+};
+
 template <int NS>
-__global__ void k_bc_outflow(Zone z, Param p, FaceBC f) {
+__global__ void k_bc_outflow(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                             const __grid_constant__ FaceSet set) {
+  chain_begin();
+  const FaceBC &f = set.f[blockIdx.y];
   int i, j, k, gl;
   if (!face_layer_point(f, z.ngg, i, j, k, gl)) return;
   ++gl;  // ghost layers 1..ngg
@@ -620,7 +629,8 @@ int launch_inner_flux_exchange(const Zone &z, const Zone &zt, const Param &p, co
 }
 
 // 2-D blocks: copy the k = 0 plane into every k ghost plane (eliminate_k_gradient_point).
-__global__ void k_eliminate_k_gradient(Zone z, Param p) {
+__global__ void k_eliminate_k_gradient(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x - z.ngg;
   const int j = blockIdx.y - z.ngg;
   if (i >= z.mx + z.ngg) return;
@@ -672,14 +682,18 @@ static inline long long face_points(const FaceBC &f) {
 }
 
 template <int NS>
-__global__ void k_bc_periodic_pair(Zone z, Param p, FaceBC f) {
+__global__ void k_bc_periodic_pair(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                                   const __grid_constant__ FaceBC f) {
+  chain_begin();
   bc_periodic_pair_item<NS>(z, p, f, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The same pairing for the 8th-order viscous node fluxes (components 1..n_var-1 of the three
 // flux arrays; component 0 carries no viscous flux and is never read).
 template <typename F>
-__global__ void k_periodic_flux_pair(Zone z, Param p, FaceBC f) {
+__global__ void k_periodic_flux_pair(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                                     const __grid_constant__ FaceBC f) {
+  chain_begin();
   PairItem it;
   const int g = z.ngg;
   if (!pair_item(f, g, (long long)blockIdx.x * blockDim.x + threadIdx.x, it)) return;
@@ -727,6 +741,20 @@ static int periodic_pair(const Zone &z, const FaceBC *faces, int n, int f, int *
   return a.direction < 0 ? f : q;
 }
 
+// Whether two outflow faces neither write a common ghost node nor read what the other writes: faces of
+// the block's own extent (not extended into the tangential ghosts), on different sides or with
+// tangential ranges apart.
+static bool outflow_apart(const Zone &z, const FaceBC &a, const FaceBC &b) {
+  const int ext[3] = {z.mx, z.my, z.mz};
+  for (const FaceBC *f : {&a, &b})
+    for (int d = 0; d < 3; ++d)
+      if (std::min(f->start[d], f->end[d]) < 0 || std::max(f->start[d], f->end[d]) > ext[d] - 1) return false;
+  if (a.face != b.face || a.direction != b.direction) return true;
+  for (int d = 0; d < 3; ++d)
+    if (d != a.face && (a.end[d] < b.start[d] || b.end[d] < a.start[d])) return true;
+  return false;
+}
+
 // Small CTAs: a face has few nodes, and spreading them over more SMs shortens the launch.
 constexpr int kFaceThreads = 64;
 
@@ -748,23 +776,43 @@ static int launch_bc_ns(const Zone &z, const Param &p, const FaceBC *faces, int 
         if (lf >= 0) {
           const long long np = face_points(faces[lf]) * (2 * z.ngg + 1);
           ProfScope prof("boundary_face", s);
-          k_bc_periodic_pair<NS><<<(unsigned)((np + 127) / 128), 128, 0, s>>>(z, p, faces[lf]);
+          CB2_TRY(launch_chain(k_bc_periodic_pair<NS>, (unsigned)((np + 127) / 128), 128, 0, s, z, p, faces[lf]));
           ++nl;
-          CB2_TRY(check_launch());
           f = q;  // the partner is done
           continue;
         }
       }
+      if (t == CB2_BC_OUTFLOW) {
+        // an outflow face reads the block's nodes and writes ghosts beyond it, so faces whose ghosts
+        // do not overlap fill in one launch
+        FaceSet set;
+        int ns = 0;
+        long long most = 0;
+        for (; f < n && ns < 6; ++f) {
+          if (faces[f].type != t || face_points(faces[f]) == 0) continue;
+          bool apart = true;
+          for (int a = 0; a < ns; ++a) apart = apart && outflow_apart(z, set.f[a], faces[f]);
+          if (!apart) break;
+          set.f[ns++] = faces[f];
+          most = std::max(most, face_points(faces[f]) * z.ngg);
+        }
+        --f;  // the loop moves on to the first face not taken
+        if (ns == 0) continue;
+        ProfScope prof("boundary_face", s);
+        const dim3 grid((unsigned)((most + kFaceThreads - 1) / kFaceThreads), (unsigned)ns);
+        CB2_TRY(launch_chain(k_bc_outflow<NS>, grid, kFaceThreads, 0, s, z, p, set));
+        ++nl;
+        continue;
+      }
       const long long np = face_points(faces[f]);
       if (np == 0) continue;
-      // threads per face node: one per ghost layer (outflow), one per layer including the face
-      // node (inflow, symmetry, wall), one per line (periodic)
-      const int layers = t == CB2_BC_OUTFLOW ? z.ngg : (t == CB2_BC_PERIODIC ? 1 : z.ngg + 1);
+      // threads per face node: one per layer including the face node (farfield, inflow, symmetry,
+      // wall), one per line (periodic)
+      const int layers = t == CB2_BC_PERIODIC ? 1 : z.ngg + 1;
       const unsigned blocks = (unsigned)((np * layers + kFaceThreads - 1) / kFaceThreads);
       ProfScope prof("boundary_face", s);
       switch (t) {
         case CB2_BC_FARFIELD: k_bc_farfield<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
-        case CB2_BC_OUTFLOW: k_bc_outflow<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
         case CB2_BC_INFLOW: k_bc_inflow<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
         case CB2_BC_SYMMETRY: k_bc_symmetry<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
         case CB2_BC_WALL: k_bc_wall<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
@@ -933,9 +981,8 @@ int launch_eliminate_k_gradient(const Zone &z, const Param &p, cudaStream_t s, i
   const int g = z.ngg;
   dim3 grid((z.mx + 2 * g + 127) / 128, z.my + 2 * g, 1);
   ProfScope prof("eliminate_k_gradient", s);
-  k_eliminate_k_gradient<<<grid, 128, 0, s>>>(z, p);
   ++nl;
-  return check_launch();
+  return launch_chain(k_eliminate_k_gradient, grid, 128, 0, s, z, p);
 }
 
 int launch_boundary(const Zone &z, const Param &p, const FaceBC *faces, int n_faces, cudaStream_t s,
@@ -957,12 +1004,9 @@ int launch_periodic_flux_exchange(const Zone &z, const Param &p, const FaceBC *f
     if (lf >= 0) {
       const long long np = face_points(faces[lf]) * (2 * z.ngg + 1);
       ProfScope prof("periodic_flux_exchange", s);
-      if (visc8_f32(p))
-        k_periodic_flux_pair<float><<<(unsigned)((np + 127) / 128), 128, 0, s>>>(z, p, faces[lf]);
-      else
-        k_periodic_flux_pair<double><<<(unsigned)((np + 127) / 128), 128, 0, s>>>(z, p, faces[lf]);
+      CB2_TRY(launch_chain(visc8_f32(p) ? k_periodic_flux_pair<float> : k_periodic_flux_pair<double>,
+                           (unsigned)((np + 127) / 128), 128, 0, s, z, p, faces[lf]));
       ++n_launch;
-      CB2_TRY(check_launch());
       f = q;
       continue;
     }

@@ -75,6 +75,7 @@ template <int NS>
 __global__ void __launch_bounds__(kChemThreads, 4)
 k_chemistry_tab(const __grid_constant__ ChemZone z, const __grid_constant__ ChemTab<NS> m) {
   __shared__ double sc[NS + 1][kChemThreads];
+  chain_begin();
   const int tid = threadIdx.x;
   const int q = blockIdx.x * kChemThreads + tid;
   if (q >= z.plane) return;
@@ -177,8 +178,7 @@ static int launch_chemistry_tab(const Zone &z, const ChemTab<NS> &m, cudaStream_
   c.sz0 = z.L0.sz;
   c.bv = z.bv; c.sv = z.sv; c.jac = z.jac; c.dq = z.dq; c.rts = z.rts;
   const dim3 grid((unsigned)((c.plane + kChemThreads - 1) / kChemThreads), (unsigned)z.mz);
-  k_chemistry_tab<NS><<<grid, kChemThreads, 0, s>>>(c, m);
-  return check_launch();
+  return launch_chain(k_chemistry_tab<NS>, grid, kChemThreads, 0, s, c, m);
 }
 
 int launch_chemistry(const Zone &z, const Param &p, cudaStream_t s, int &n_launch) {

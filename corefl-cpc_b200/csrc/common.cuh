@@ -139,7 +139,7 @@ struct Param {
   // J d(node flux)/d(its direction) (the viscous divergence), and the x sweep, the first writer
   // of the residual, assigns dq instead of adding to it
   int visc8_fused;
-  int assign_x;  // primitive sweeps: the x sweep is the residual's first term and assigns dq
+  int assign_x;  // primitive and characteristic sweeps: the x sweep is the residual's first term and assigns dq
   int limit_flow;
   double lf_ll[5], lf_ul[5];  // limit_flow bounds of rho, u, v, w, p
   double dt;                  // the current step's time step (positivity limiter)
@@ -148,6 +148,13 @@ struct Param {
   unsigned *status;  // device status word
   Mech mech;
 };
+
+// First statement of a kernel that launch_chain starts: waits until the kernel before it in the stream
+// has finished and its writes are visible, then lets the next one start its own launch.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ void flag_status(const Param &p, unsigned bits) {
   if (p.status) atomicOr(p.status, bits);

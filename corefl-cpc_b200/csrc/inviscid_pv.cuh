@@ -719,7 +719,8 @@ __device__ __forceinline__ void pv_tile(const Zone &z, const Param &p, idx_t run
 }
 
 template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false, bool TT = false>
-__global__ void __launch_bounds__(kSweepThreads) k_inviscid_pv(Zone z, Param p, idx_t run) {
+__global__ void __launch_bounds__(kSweepThreads) k_inviscid_pv(const __grid_constant__ Zone z, const __grid_constant__ Param p, idx_t run) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char pv_smem[];
   pv_tile<T, NS, DIR, REC, SOLVER, NI, VF, TT>(z, p, run, blockIdx.x, blockIdx.y, blockIdx.z, pv_smem);
 }
@@ -727,7 +728,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_inviscid_pv(Zone z, Param p, 
 // The mixture sweeps, held to 128 registers (two CTAs per SM): they would otherwise take up to 170
 // and run one CTA per SM (192^3 H2/air box, WENO5 + HLLC, FP64: 21.6 -> 18.1 ms per step).
 template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false>
-__global__ void __launch_bounds__(kSweepThreads, 2) k_inviscid_pv_mb2(Zone z, Param p, idx_t run) {
+__global__ void __launch_bounds__(kSweepThreads, 2) k_inviscid_pv_mb2(const __grid_constant__ Zone z, const __grid_constant__ Param p, idx_t run) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char pv_smem[];
   pv_tile<T, NS, DIR, REC, SOLVER, NI, VF>(z, p, run, blockIdx.x, blockIdx.y, blockIdx.z, pv_smem);
 }
@@ -768,8 +770,7 @@ static int launch_pv_yz(const Zone &z, const Param &p, cudaStream_t s) {
   const size_t smem = pv_tile_smem<T, NS, REC, SOLVER, VF>(DIR, NI);
   auto kern = pv_kernel<T, NS, DIR, REC, SOLVER, NI, VF, TT>();
   CB2_TRY(prepare_smem(kern, smem));
-  kern<<<grid, kSweepThreads, smem, s>>>(z, p, 0);
-  return check_launch();
+  return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, (idx_t)0);
 }
 
 // y/z sweep with the block's tile width: the autotuned widths exist for the WENO5/7 air sweeps
@@ -792,8 +793,7 @@ static int launch_pv_dir(int d, const Zone &z, const Param &p, cudaStream_t s) {
     const size_t smem = pv_tile_smem<T, NS, REC, SOLVER, VF>(0);
     auto kern = pv_kernel<T, NS, 0, REC, SOLVER, kNI, VF, TT>();
     CB2_TRY(prepare_smem(kern, smem));
-    kern<<<grid, kSweepThreads, smem, s>>>(z, p, geo.run);
-    return check_launch();
+    return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, geo.run);
   }
   if (d == 1) return launch_pv_yz_ni<T, NS, 1, REC, SOLVER, VF, TT>(z, p, s);
   return launch_pv_yz_ni<T, NS, 2, REC, SOLVER, VF, TT>(z, p, s);

@@ -58,6 +58,24 @@ inline int prepare_smem(K kern, size_t bytes) {
   return CB2_OK;
 }
 
+// Launches a kernel whose first statement is chain_begin() so that its launch overlaps the tail of the
+// kernel before it (programmatic dependent launch): a step is a chain of dependent kernels, and on
+// small blocks the gaps between them take longer than the kernels.
+template <typename... P, typename... A>
+inline int launch_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A &...a) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, a...));
+}
+
 // Face boundary condition in device-usable form (after the reference's register_boundary).
 struct FaceBC {
   int type, face, direction;
@@ -79,7 +97,9 @@ int launch_inviscid_pv_mix9(const Zone &z, const Param &p, cudaStream_t s, int &
 int launch_inviscid_pv_2t5(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_inviscid_pv_2t9(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_inviscid_pv_f32(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
-int launch_stage_update(const Zone &z, const Param &p, double dt, int rk, cudaStream_t s, int &n_launch);
+// first: stage 0 of a step whose qn has not been stored: the update reads cv in its place and stores it
+int launch_stage_update(const Zone &z, const Param &p, double dt, int rk, cudaStream_t s, int &n_launch,
+                        bool first = false);
 int launch_cv_from_bv(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 // two-temperature VT relaxation over dt_stage of every interior node (a standalone
 // apply_vt_relaxation_rk; launch_stage_update runs it itself for two-temperature contexts)
@@ -119,10 +139,8 @@ ChemTabs *make_chem_tabs(const cb2_mechanism &m);
 void free_chem_tabs(ChemTabs *t);
 int launch_chemistry(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
 int launch_shock_sensor(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
-int launch_local_dt(const Zone &z, const Param &p, cudaStream_t s, int &n_launch);
-int launch_min_reduce(const double *src, long long n, double *partial, int n_partial, double *out,
-                      cudaStream_t s, int &n_launch);
-int min_reduce_partials(long long n);
+// dt_local of every interior node, and *dt_min lowered to their minimum
+int launch_local_dt(const Zone &z, const Param &p, double *dt_min, cudaStream_t s, int &n_launch);
 int launch_set_value(double *dst, double v, cudaStream_t s, int &n_launch);
 // dst[i] = float(src[i]) for i < n (the mixed form's FP32 copies)
 int launch_to_f32(const double *src, float *dst, size_t n, cudaStream_t s, int &n_launch);

@@ -39,9 +39,10 @@ __device__ __forceinline__ double newton_temperature(double e, const double *y, 
 // SSP-RK3 stage update of one interior node (update_cv_and_bv_rk<mix>, src/RK.cuh:277-367).
 // TT: two-temperature model, rho*e_ve at cv comp 5 + NS (clipped at zero), e_ve at sv comp NS,
 // T_ve and T from the two-temperature inversion.
+// first: qn is not stored yet: it takes cv's value, which stands for it here (stage 0).
 template <int NS, bool TT = false>
 __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p, double dt, int rk, int i, int j,
-                                                   int k) {
+                                                   int k, bool first = false) {
   static_assert(!TT || NS > 0, "the two-temperature model needs species");
   constexpr int NV = 5 + NS + (TT ? 1 : 0);
   double a, b, c;
@@ -50,8 +51,17 @@ __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p
   const idx_t g0 = z.L0.at(i, j, k), sz0 = z.L0.sz;
   const double dtj = dt / z.jac[g];
   double q[NV];
+  if (first) {
 #pragma unroll
-  for (int l = 0; l < NV; ++l) q[l] = a * z.qn[g + l * sz] + b * z.cv[g + l * sz] + c * dtj * z.dq[g0 + l * sz0];
+    for (int l = 0; l < NV; ++l) {
+      const double v = z.cv[g + l * sz];
+      z.qn[g + l * sz] = v;
+      q[l] = a * v + b * v + c * dtj * z.dq[g0 + l * sz0];
+    }
+  } else {
+#pragma unroll
+    for (int l = 0; l < NV; ++l) q[l] = a * z.qn[g + l * sz] + b * z.cv[g + l * sz] + c * dtj * z.dq[g0 + l * sz0];
+  }
   if (z.mz == 1) q[3] = 0;
   if (!(q[0] > 0) || !isfinite(q[4])) flag_status(p, 1u);
 

@@ -16,7 +16,8 @@ constexpr int kPropTabCtas = 4;  // CTAs per SM of the FP64 transport kernels: 1
 // 128 threads per SM; the FP64 9-species transport otherwise takes 163): the exponential and
 // logarithm chains are latency-bound (192^3 H2/air box: 29.9 -> 20.7 ms per step).
 template <int NS, bool F32T = false>
-__global__ void __launch_bounds__(kPropThreads, 6) k_properties(Zone z, Param p) {
+__global__ void __launch_bounds__(kPropThreads, 6) k_properties(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
+  chain_begin();
   const int g_ = z.ngg;
   const int i = blockIdx.x * kPropThreads + threadIdx.x - g_;
   const int j = blockIdx.y - g_, k = blockIdx.z - g_;
@@ -31,6 +32,7 @@ template <int NS>
 __global__ void __launch_bounds__(kPropThreads, kPropTabCtas)
 k_properties_tab(const __grid_constant__ Zone z, const __grid_constant__ Param p, const __grid_constant__ TransTab<NS> m) {
   extern __shared__ double s_om[];
+  chain_begin();
   const int g_ = z.ngg, px = z.mx + 2 * g_;
   const int q = blockIdx.x * kPropThreads + threadIdx.x;
   if (q >= px * (z.my + 2 * g_)) return;
@@ -83,7 +85,8 @@ __device__ __forceinline__ void spread_properties(const Zone &z, const Param &p,
 }
 
 template <int NS, bool F32T = false>
-__global__ void __launch_bounds__(kPropThreads) k_properties_planar(Zone z, Param p) {
+__global__ void __launch_bounds__(kPropThreads) k_properties_planar(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
+  chain_begin();
   const int g_ = z.ngg;
   const int i = blockIdx.x * kPropThreads + threadIdx.x - g_;
   const int j = blockIdx.y - g_;
@@ -97,6 +100,7 @@ __global__ void __launch_bounds__(kPropThreads, kPropTabCtas)
 k_properties_planar_tab(const __grid_constant__ Zone z, const __grid_constant__ Param p,
                         const __grid_constant__ TransTab<NS> m) {
   extern __shared__ double s_om[];
+  chain_begin();
   const int g_ = z.ngg, px = z.mx + 2 * g_;
   const int q = blockIdx.x * kPropThreads + threadIdx.x;
   if (q >= px * (z.my + 2 * g_)) return;
@@ -111,9 +115,7 @@ static int launch_properties_tab(const Zone &z, const Param &p, const TransTab<N
   const int plane = (z.mx + 2 * g) * (z.my + 2 * g);
   const dim3 grid((unsigned)((plane + kPropThreads - 1) / kPropThreads), (unsigned)(planar ? 1 : z.mz + 2 * g));
   const size_t smem = sizeof(double) * m.n_red * kPropThreads;
-  if (planar) k_properties_planar_tab<NS><<<grid, kPropThreads, smem, s>>>(z, p, m);
-  else k_properties_tab<NS><<<grid, kPropThreads, smem, s>>>(z, p, m);
-  return check_launch();
+  return launch_chain(planar ? k_properties_planar_tab<NS> : k_properties_tab<NS>, grid, kPropThreads, smem, s, z, p, m);
 }
 
 int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_launch) {
@@ -126,35 +128,19 @@ int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_laun
   const TransTabs *tab = mixed ? nullptr : p.mech.trans_tabs;
   if (tab && p.n_spec == 9) return launch_properties_tab<9>(z, p, tab->t9, planar, s);
   if (tab && p.n_spec == 5) return launch_properties_tab<5>(z, p, tab->t5, planar, s);
+  // nothing changes for air of constant viscosity without a Mach array
+  if (p.n_spec == 0 && p.mu_constant > 0 && !z.mach) { --n_launch; return CB2_OK; }
+  auto go = [&](auto kern) { return launch_chain(kern, grid, kPropThreads, 0, s, z, p); };
   switch (p.n_spec) {
-    case 0:
-      if (p.mu_constant > 0 && !z.mach) { --n_launch; return CB2_OK; }  // nothing changes
-      if (planar) k_properties_planar<0><<<grid, kPropThreads, 0, s>>>(z, p);
-      else k_properties<0><<<grid, kPropThreads, 0, s>>>(z, p);
-      break;
+    case 0: return go(planar ? k_properties_planar<0> : k_properties<0>);
     case 5:
-      if (mixed) {
-        if (planar) k_properties_planar<5, true><<<grid, kPropThreads, 0, s>>>(z, p);
-        else k_properties<5, true><<<grid, kPropThreads, 0, s>>>(z, p);
-      } else if (planar) {
-        k_properties_planar<5><<<grid, kPropThreads, 0, s>>>(z, p);
-      } else {
-        k_properties<5><<<grid, kPropThreads, 0, s>>>(z, p);
-      }
-      break;
+      if (mixed) return go(planar ? k_properties_planar<5, true> : k_properties<5, true>);
+      return go(planar ? k_properties_planar<5> : k_properties<5>);
     case 9:
-      if (mixed) {
-        if (planar) k_properties_planar<9, true><<<grid, kPropThreads, 0, s>>>(z, p);
-        else k_properties<9, true><<<grid, kPropThreads, 0, s>>>(z, p);
-      } else if (planar) {
-        k_properties_planar<9><<<grid, kPropThreads, 0, s>>>(z, p);
-      } else {
-        k_properties<9><<<grid, kPropThreads, 0, s>>>(z, p);
-      }
-      break;
+      if (mixed) return go(planar ? k_properties_planar<9, true> : k_properties<9, true>);
+      return go(planar ? k_properties_planar<9> : k_properties<9>);
     default: return CB2_ERR_UNSUPPORTED;
   }
-  return check_launch();
 }
 
 // ---- repacking (host) ----------------------------------------------------------------------
@@ -212,73 +198,54 @@ TransTabs *make_trans_tabs(const cb2_mechanism &m) {
 
 void free_trans_tabs(TransTabs *t) { delete t; }
 
-// ---- local time step --------------------------------------------------------------------
-template <int NS>
-__global__ void __launch_bounds__(kPropThreads) k_local_dt(Zone z, Param p) {
-  const int i = blockIdx.x * kPropThreads + threadIdx.x;
-  const int j = blockIdx.y, k = blockIdx.z;
-  if (i >= z.mx) return;
-  z.dtl[z.L0.at(i, j, k)] = local_dt_point<NS>(z, p, i, j, k);
+// ---- local time step and its minimum ------------------------------------------------------
+// The smaller of *out and v, exactly and for any sign: bits of non-negative doubles order as signed
+// integers, bits of negative ones in reverse as unsigned.
+__device__ __forceinline__ void atomic_min_double(double *out, double v) {
+  if (v >= 0) atomicMin(reinterpret_cast<long long *>(out), __double_as_longlong(v));
+  else atomicMax(reinterpret_cast<unsigned long long *>(out), (unsigned long long)__double_as_longlong(v));
 }
 
-int launch_local_dt(const Zone &z, const Param &p, cudaStream_t s, int &n_launch) {
+// dt of every interior node; the minimum goes to *dt_min (seeded by the caller), one atomic per warp.
+// The reference seeds its minimum with 1e+6 (src/TimeAdvanceFunc.cu:152), so a block whose every dt
+// exceeds 1e6 reports 1e6; NaN does not count.
+template <int NS>
+__global__ void __launch_bounds__(kPropThreads) k_local_dt(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                                                           double *dt_min) {
+  chain_begin();
+  const int i = blockIdx.x * kPropThreads + threadIdx.x;
+  const int j = blockIdx.y, k = blockIdx.z;
+  double v = 1e+6;
+  if (i < z.mx) {
+    const double dt = local_dt_point<NS>(z, p, i, j, k);
+    z.dtl[z.L0.at(i, j, k)] = dt;
+    v = fmin(v, dt);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0 && v < 1e+6) atomic_min_double(dt_min, v);
+}
+
+int launch_local_dt(const Zone &z, const Param &p, double *dt_min, cudaStream_t s, int &n_launch) {
   dim3 grid((z.mx + kPropThreads - 1) / kPropThreads, z.my, z.mz);
   ++n_launch;
   ProfScope prof("local_dt", s);
   switch (p.n_spec) {
-    case 0: k_local_dt<0><<<grid, kPropThreads, 0, s>>>(z, p); break;
-    case 5: k_local_dt<5><<<grid, kPropThreads, 0, s>>>(z, p); break;
-    case 9: k_local_dt<9><<<grid, kPropThreads, 0, s>>>(z, p); break;
+    case 0: return launch_chain(k_local_dt<0>, grid, kPropThreads, 0, s, z, p, dt_min);
+    case 5: return launch_chain(k_local_dt<5>, grid, kPropThreads, 0, s, z, p, dt_min);
+    case 9: return launch_chain(k_local_dt<9>, grid, kPropThreads, 0, s, z, p, dt_min);
     default: return CB2_ERR_UNSUPPORTED;
   }
-  return check_launch();
 }
 
-// ---- min reduction: grid-stride partial minima, then one CTA over the partials ----------
-constexpr int kRedThreads = 256;
-
-__device__ __forceinline__ double warp_min(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_down_sync(0xffffffffu, v, o));
-  return v;
+__global__ void k_set_value(double *dst, double v) {
+  chain_begin();
+  *dst = v;
 }
-
-__device__ __forceinline__ double block_min(double v) {
-  __shared__ double sw[kRedThreads / 32];
-  v = warp_min(v);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sw[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    v = lane < kRedThreads / 32 ? sw[lane] : 1e+6;
-    v = warp_min(v);
-  }
-  return v;
-}
-
-// The reference seeds every thread with 1e+6 (src/TimeAdvanceFunc.cu:152), so a block
-// whose every dt exceeds 1e6 reports 1e6; the same seed is kept here.
-__global__ void __launch_bounds__(kRedThreads) k_min_partial(const double *src, long long n, double *partial) {
-  double v = 1e+6;
-  for (long long t = (long long)blockIdx.x * kRedThreads + threadIdx.x; t < n; t += (long long)gridDim.x * kRedThreads)
-    v = fmin(v, src[t]);
-  v = block_min(v);
-  if (threadIdx.x == 0) partial[blockIdx.x] = v;
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_min_final(const double *partial, int n, double *out) {
-  double v = 1e+6;
-  for (int t = threadIdx.x; t < n; t += kRedThreads) v = fmin(v, partial[t]);
-  v = block_min(v);
-  if (threadIdx.x == 0) *out = fmin(*out, v);
-}
-
-__global__ void k_set_value(double *dst, double v) { *dst = v; }
 
 int launch_set_value(double *dst, double v, cudaStream_t s, int &n_launch) {
-  k_set_value<<<1, 1, 0, s>>>(dst, v);
   ++n_launch;
-  return check_launch();
+  return launch_chain(k_set_value, 1, 1, 0, s, dst, v);
 }
 
 // Grid-stride FP64 -> FP32 conversion (coalesced 8-byte loads and 4-byte stores).
@@ -292,24 +259,6 @@ int launch_to_f32(const double *src, float *dst, size_t n, cudaStream_t s, int &
   const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 32);
   k_to_f32<<<blocks, 256, 0, s>>>(src, dst, n);
   ++n_launch;
-  return check_launch();
-}
-
-int min_reduce_partials(long long n) {
-  long long b = (n + kRedThreads - 1) / kRedThreads;
-  if (b > 148 * 8) b = 148 * 8;
-  if (b < 1) b = 1;
-  return (int)b;
-}
-
-// out must hold the running minimum on entry (the caller seeds it, e.g. with 1e6).
-int launch_min_reduce(const double *src, long long n, double *partial, int n_partial, double *out, cudaStream_t s,
-                      int &n_launch) {
-  ProfScope prof("min_reduce", s);
-  k_min_partial<<<n_partial, kRedThreads, 0, s>>>(src, n, partial);
-  CB2_TRY(check_launch());
-  k_min_final<<<1, kRedThreads, 0, s>>>(partial, n_partial, out);
-  n_launch += 2;
   return check_launch();
 }
 

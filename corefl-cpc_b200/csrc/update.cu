@@ -11,11 +11,13 @@ namespace cb2 {
 constexpr int kPtThreads = 128;
 
 template <int NS, bool TT>
-__global__ void __launch_bounds__(kPtThreads) k_stage_update(Zone z, Param p, double dt, int rk) {
+__global__ void __launch_bounds__(kPtThreads) k_stage_update(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                                                             double dt, int rk, int first) {
+  chain_begin();
   const int i = blockIdx.x * kPtThreads + threadIdx.x;
   const int j = blockIdx.y, k = blockIdx.z;
   if (i >= z.mx) return;
-  stage_update_point<NS, TT>(z, p, step_dt(p, dt), rk, i, j, k);
+  stage_update_point<NS, TT>(z, p, step_dt(p, dt), rk, i, j, k, first != 0);
 }
 
 // VT relaxation of every interior node over dt_scale x the step's dt (apply_vt_relaxation_rk,
@@ -124,19 +126,18 @@ static int launch_vt_ns(const Zone &z, const Param &p, double dt, double dt_scal
 }
 
 template <int NS>
-static int launch_update_ns(const Zone &z, const Param &p, double dt, int rk, cudaStream_t s, int &nl) {
+static int launch_update_ns(const Zone &z, const Param &p, double dt, int rk, bool first, cudaStream_t s, int &nl) {
   dim3 grid((z.mx + kPtThreads - 1) / kPtThreads, z.my, z.mz);
   const bool tt = p.i_eve >= 0;
   {
     ProfScope prof("stage_update", s);
     if constexpr (NS > 0) {
-      if (tt) k_stage_update<NS, true><<<grid, kPtThreads, 0, s>>>(z, p, dt, rk);
-      else k_stage_update<NS, false><<<grid, kPtThreads, 0, s>>>(z, p, dt, rk);
+      CB2_TRY(launch_chain(tt ? k_stage_update<NS, true> : k_stage_update<NS, false>, grid, kPtThreads, 0, s, z, p, dt,
+                           rk, (int)first));
     } else {
-      k_stage_update<NS, false><<<grid, kPtThreads, 0, s>>>(z, p, dt, rk);
+      CB2_TRY(launch_chain(k_stage_update<NS, false>, grid, kPtThreads, 0, s, z, p, dt, rk, (int)first));
     }
   }
-  CB2_TRY(check_launch());
   if constexpr (NS > 0) {
     // the stage's VT relaxation follows its update and precedes limit_flow (src/RK.cuh:198-207)
     if (tt) {
@@ -155,12 +156,12 @@ static int launch_update_ns(const Zone &z, const Param &p, double dt, int rk, cu
   return CB2_OK;
 }
 
-int launch_stage_update(const Zone &z, const Param &p, double dt, int rk, cudaStream_t s, int &n_launch) {
+int launch_stage_update(const Zone &z, const Param &p, double dt, int rk, cudaStream_t s, int &n_launch, bool first) {
   ++n_launch;
   switch (p.n_spec) {
-    case 0: return launch_update_ns<0>(z, p, dt, rk, s, n_launch);
-    case 5: return launch_update_ns<5>(z, p, dt, rk, s, n_launch);
-    case 9: return launch_update_ns<9>(z, p, dt, rk, s, n_launch);
+    case 0: return launch_update_ns<0>(z, p, dt, rk, first, s, n_launch);
+    case 5: return launch_update_ns<5>(z, p, dt, rk, first, s, n_launch);
+    case 9: return launch_update_ns<9>(z, p, dt, rk, first, s, n_launch);
     default: return CB2_ERR_UNSUPPORTED;
   }
 }

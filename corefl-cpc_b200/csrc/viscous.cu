@@ -118,11 +118,15 @@ __device__ __forceinline__ void visc8_node_flux_air(const Zone &z, const Param &
   else visc8_node_flux_air_at<T, true>(z, p, i, j, k, b);
 }
 
-__global__ void __launch_bounds__(kVisThreads) k_visc8_node_flux_air_f64(Zone z, Param p) {
+__global__ void __launch_bounds__(kVisThreads) k_visc8_node_flux_air_f64(const __grid_constant__ Zone z,
+                                                                         const __grid_constant__ Param p) {
+  chain_begin();
   visc8_node_flux_air<double>(z, p);
 }
 // bounded to 64 registers: four CTAs of 256 threads per SM
-__global__ void __launch_bounds__(kVisThreads, 4) k_visc8_node_flux_air_f32(Zone z, Param p) {
+__global__ void __launch_bounds__(kVisThreads, 4) k_visc8_node_flux_air_f32(const __grid_constant__ Zone z,
+                                                                            const __grid_constant__ Param p) {
+  chain_begin();
   visc8_node_flux_air<float>(z, p);
 }
 
@@ -336,7 +340,9 @@ __device__ __forceinline__ void visc8_divergence_row(const Zone &z, const Param 
 // warps in flight hide the loads: with one test per node in place of the three per variable the loads
 // batch better but take 64 registers, and the kernel takes 4.1 ms in place of 2.2 at 257^3.
 template <bool ASSIGN>
-__global__ void __launch_bounds__(kVisRow) k_visc8_divergence_f64(Zone z, Param p) {
+__global__ void __launch_bounds__(kVisRow) k_visc8_divergence_f64(const __grid_constant__ Zone z,
+                                                                  const __grid_constant__ Param p) {
+  chain_begin();
   visc8_divergence_row<double, ASSIGN>(z, p);
 }
 template <bool ASSIGN>
@@ -516,7 +522,8 @@ __device__ __forceinline__ void visc2_tile(const Zone &z, const Param &p) {
 }
 
 template <int NS, int DIR>
-__global__ void __launch_bounds__(kV2TI *kV2TS) k_visc2(Zone z, Param p) {
+__global__ void __launch_bounds__(kV2TI *kV2TS) k_visc2(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
+  chain_begin();
   visc2_tile<NS, DIR, false>(z, p);
 }
 
@@ -541,9 +548,8 @@ static int launch_visc2_ns(const Zone &z, const Param &p, cudaStream_t s, int &n
       else if (d == 1) k_visc2_2t<NS, 1><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
       else k_visc2_2t<NS, 2><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
     } else {
-      if (d == 0) k_visc2<NS, 0><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
-      else if (d == 1) k_visc2<NS, 1><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
-      else k_visc2<NS, 2><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
+      CB2_TRY(launch_chain(d == 0 ? k_visc2<NS, 0> : (d == 1 ? k_visc2<NS, 1> : k_visc2<NS, 2>), grid, kV2TI * kV2TS, 0,
+                           s, z, p));
     }
     ++nl;
     CB2_TRY(check_launch());
@@ -561,8 +567,8 @@ int launch_viscous(const Zone &z, const Param &p, const FaceBC *faces, int n_fac
     {
       ProfScope prof("visc8_node_flux", s);
       if (p.n_spec == 0) {
-        if (p.precision == CB2_PREC_MIXED) k_visc8_node_flux_air_f32<<<grid, block, 0, s>>>(z, p);
-        else k_visc8_node_flux_air_f64<<<grid, block, 0, s>>>(z, p);
+        CB2_TRY(launch_chain(p.precision == CB2_PREC_MIXED ? k_visc8_node_flux_air_f32 : k_visc8_node_flux_air_f64, grid,
+                             block, 0, s, z, p));
       } else {
         // mixtures: FP64 in both forms (their mixed form keeps the viscous terms in FP64)
         if (!z.kappa || !z.rhoD || (p.i_eve >= 0 && (!z.tve || !z.kappa_ve))) return CB2_ERR_INVALID;
@@ -593,10 +599,9 @@ int launch_viscous(const Zone &z, const Param &p, const FaceBC *faces, int n_fac
       if (visc8_f32(p)) {
         if (assign) k_visc8_divergence_f32<true><<<grow, kVisRow, 0, s>>>(z, p);
         else k_visc8_divergence_f32<false><<<grow, kVisRow, 0, s>>>(z, p);
-      } else if (assign) {
-        k_visc8_divergence_f64<true><<<grow, kVisRow, 0, s>>>(z, p);
       } else {
-        k_visc8_divergence_f64<false><<<grow, kVisRow, 0, s>>>(z, p);
+        CB2_TRY(launch_chain(assign ? k_visc8_divergence_f64<true> : k_visc8_divergence_f64<false>, grow, kVisRow, 0, s,
+                             z, p));
       }
     }
     ++nl;

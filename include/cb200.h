@@ -406,8 +406,9 @@ int cb2_cfl_dt(cb2_ctx *ctx, double *dt_out, void *stream);
 #define CB2_NOALLOC_MAX_NODES (16384LL * 2048LL)
 int cb2_min_dt_noalloc(const double *dt_local, long long n, double *dt_min, void *stream);
 
-/* One whole SSP-RK3 step over all bound blocks (src/RK.cuh:107-237): qn<-cv, [CFL dt],
- * 3 x (rhs, stage update, boundary, properties).  With fixed_dt != 0 the step uses
+/* One whole SSP-RK3 step over all bound blocks (src/RK.cuh:107-237): [CFL dt], 3 x (rhs, stage
+ * update, boundary, properties).  qn <- cv rides on stage 0's update, which stores the interior
+ * nodes (the stages read no others; cb2_store_qn copies the ghosts too).  With fixed_dt != 0 the step uses
  * *dt_inout and performs no host synchronisation; otherwise the CFL dt is computed first
  * and written to *dt_inout. */
 int cb2_rk3_step(cb2_ctx *ctx, double *dt_inout, int fixed_dt, void *stream);
