@@ -807,8 +807,8 @@ int cb2_rhs(cb2_ctx *ctx, int blk, unsigned mask, void *stream) {
                        ? 2
                        : 0;
   // no zeroing of dq when the first term assigns it, or when the caller's dq is added to
-  pf.assign_x = !accumulate && !visc && !((mask & CB2_RHS_CHEMISTRY) && p.reaction) && (mask & CB2_RHS_INVISCID) && pv &&
-                !B->z.sweep_mask;
+  pf.assign_x = !accumulate && !visc && !((mask & CB2_RHS_CHEMISTRY) && p.reaction) && (mask & CB2_RHS_INVISCID) &&
+                (pv ? !B->z.sweep_mask : p.inviscid_scheme == CB2_INV_WENO5_CH || p.inviscid_scheme == CB2_INV_WENO7_CH);
   const bool assign = !accumulate && (pf.visc8_fused || pf.assign_x || (visc && viscous_assigns_dq(p)));
   if (!assign && !accumulate) {
     ProfScope prof("zero_dq", s);
@@ -818,7 +818,7 @@ int cb2_rhs(cb2_ctx *ctx, int blk, unsigned mask, void *stream) {
   if ((mask & CB2_RHS_CHEMISTRY) && p.reaction) CB2_TRY(launch_chemistry(B->z, p, s, nl));
   if (mask & CB2_RHS_INVISCID) {
     if (p.inviscid_scheme == CB2_INV_WENO5_CH || p.inviscid_scheme == CB2_INV_WENO7_CH)
-      CB2_TRY(launch_inviscid_char(B->z, p, s, nl));
+      CB2_TRY(launch_inviscid_char(B->z, pf, s, nl));
     else if (p.inviscid_scheme == CB2_INV_WENO5_CP || p.inviscid_scheme == CB2_INV_WENO7_CP)
       CB2_TRY(launch_inviscid_comp(B->z, p, s, nl));
     else

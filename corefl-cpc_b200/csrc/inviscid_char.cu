@@ -33,7 +33,6 @@ __device__ __forceinline__ void char_flux(const double *__restrict__ sQ, const d
                                           int c, int st, double kx, double ky, double kz, double eps,
                                           bool shock, const Mech &mech, double *out, int os) {
   constexpr int NSC = NS + (TT ? 1 : 0);  // transported scalars: species (+ e_ve)
-  constexpr int NV = 5 + NSC;
   constexpr int R = ORDER / 2 + 1;  // nodes on each side of the interface
   constexpr int NW = 2 * R - 1;     // values per WENO side
 #define Qv(v, m) sQ[(v) * NN + c + (m) * st]
@@ -46,19 +45,18 @@ __device__ __forceinline__ void char_flux(const double *__restrict__ sQ, const d
   // Roe average at the interface between node c (m = 0) and c + st (m = 1)
   const double rho_l = Qv(0, 0), rho_r = Qv(0, 1);
   double t1 = sqrt(rho_l * rho_r);
-  const double rlc = 1 / (rho_l + t1), rrc = 1 / (t1 + rho_r);
+  const double rlc = recip(rho_l + t1), rrc = recip(t1 + rho_r);
   const double um = rlc * Qv(1, 0) + rrc * Qv(1, 1);
   const double vm = rlc * Qv(2, 0) + rrc * Qv(2, 1);
   const double wm = rlc * Qv(3, 0) + rrc * Qv(3, 1);
   double cm, gm1;
-  // scalar-coupling sums sum_s alpha_s Q_s and sum_s alpha_s Q_s U_k at each stencil node
-  double sbq[NS > 0 ? 2 * R : 1], sbf[NS > 0 ? 2 * R : 1];
+  double alpha[NS > 0 ? NSC : 1];  // scalar coupling of the pressure form
   if constexpr (NS == 0) {
     const double t_roe = (rlc * Fv(4, 0) + rrc * Fv(4, 1)) / kRAir;
     cm = sqrt(kGammaAir * kRAir * t_roe);
     gm1 = kGammaAir - 1;
   } else {
-    double svm[NSC], alpha[NSC], ecoef[NSC];
+    double svm[NSC], ecoef[NSC];
     double rmix = 0;
 #pragma unroll
     for (int s = 0; s < NSC; ++s) svm[s] = rlc * Qv(5 + s, 0) + rrc * Qv(5 + s, 1);
@@ -71,17 +69,6 @@ __device__ __forceinline__ void char_flux(const double *__restrict__ sQ, const d
     gm1 = gamma - 1;
 #pragma unroll
     for (int s = 0; s < NSC; ++s) out[(5 + s) * os] = ecoef[s];
-#pragma unroll
-    for (int m = 0; m < 2 * R; ++m) {
-      double sp = 0, sm = 0;
-#pragma unroll
-      for (int s = 0; s < NSC; ++s) {
-        sp = fma(alpha[s], Qv(5 + s, m - R + 1), sp);
-        sm = fma(alpha[s], Qv(5 + s, m - R + 1) * Fv(0, m - R + 1), sm);
-      }
-      sbq[m] = sp;
-      sbf[m] = sm;
-    }
   }
   // orthonormal basis (k, n, q)
   t1 = rnorm3d(kx, ky, kz);
@@ -107,44 +94,81 @@ __device__ __forceinline__ void char_flux(const double *__restrict__ sQ, const d
     const double l = fabs(Fv(0, m)) + Fv(5, m);
     if (l > lam) lam = l;
   }
+  // The acoustic fields 0 and 4 and the entropy field 3 project onto three linear forms of a node's
+  // (Q, F): P, the pressure form (with the scalars' coupling), S, the acoustic form, and the density:
+  //   L0 = P + S,  L4 = P - S,  L3 = Q0 - 2 P.
+  // Their split values at the stencil nodes are formed once; a field at a time would read the whole
+  // stencil from shared memory five times, which bound the kernel (520 reads per interface against
+  // 264).
   double fch[5];
-  // one characteristic field at a time: keeps the stencil projections of a single field live
-#pragma unroll 1
-  for (int l = 0; l < 5; ++l) {
-    double L0, L1, L2, L3, L4, tc;
-    if (l == 0 || l == 4) {
-      const double sg = l == 0 ? 1.0 : -1.0;
-      L0 = (alf + sg * Uk_bar * cm) * ic2 * 0.5;
-      L1 = -(gm1 * um + sg * kx * cm) * ic2 * 0.5;
-      L2 = -(gm1 * vm + sg * ky * cm) * ic2 * 0.5;
-      L3 = -(gm1 * wm + sg * kz * cm) * ic2 * 0.5;
-      L4 = gm1 * ic2 * 0.5;
-      tc = 0.5;
-    } else if (l == 1) {
-      L0 = -Un; L1 = nx; L2 = ny; L3 = nz; L4 = 0; tc = 0;
-    } else if (l == 2) {
-      L0 = -Uq; L1 = qx; L2 = qy; L3 = qz; L4 = 0; tc = 0;
-    } else {
-      L0 = 1 - alf * ic2; L1 = gm1 * um * ic2; L2 = gm1 * vm * ic2; L3 = gm1 * wm * ic2; L4 = -gm1 * ic2;
-      tc = -1;
+  {
+    const double h2 = 0.5 * ic2, pa = h2 * alf, pg = h2 * gm1, pu = -pg * um, pv = -pg * vm, pw = -pg * wm;
+    const double hc = h2 * cm, s0 = hc * Uk_bar, sx = -hc * kx, sy = -hc * ky, sz = -hc * kz;
+    double pp[NW], pm[NW], sp[NW], sm[NW];
+#pragma unroll
+    for (int m = 0; m < 2 * R; ++m) {
+      const int o = m - R + 1;
+      const double uk = FvL(0, o), q0 = QvL(0, o), q1 = QvL(1, o), q2 = QvL(2, o), q3 = QvL(3, o), q4 = QvL(4, o);
+      const double f0 = q0 * uk, f1 = FvL(1, o), f2 = FvL(2, o), f3 = FvL(3, o), f4 = (q4 + FvL(4, o)) * uk;
+      double PQ = fma(pa, q0, fma(pu, q1, fma(pv, q2, fma(pw, q3, pg * q4))));
+      double PF = fma(pa, f0, fma(pu, f1, fma(pv, f2, fma(pw, f3, pg * f4))));
+      if constexpr (NS > 0) {
+        double sc = 0;
+#pragma unroll
+        for (int s = 0; s < NSC; ++s) sc = fma(alpha[s], QvL(5 + s, o), sc);
+        PQ = fma(0.5, sc, PQ);
+        PF = fma(0.5 * sc, uk, PF);
+      }
+      const double SQ = fma(s0, q0, fma(sx, q1, fma(sy, q2, sz * q3)));
+      const double SF = fma(s0, f0, fma(sx, f1, fma(sy, f2, sz * f3)));
+      const double hj = 0.5 * FvL(6, o);
+      if (m < NW) {
+        pp[m] = hj * fma(lam, PQ, PF);
+        sp[m] = hj * fma(lam, SQ, SF);
+      }
+      if (m > 0) {
+        pm[m - 1] = hj * fma(-lam, PQ, PF);
+        sm[m - 1] = hj * fma(-lam, SQ, SF);
+      }
     }
+#pragma unroll 1
+    for (int e = 0; e < 2; ++e) {
+      const double sg = e == 0 ? 1.0 : -1.0;
+      double vp[NW], vmn[NW];
+#pragma unroll
+      for (int m = 0; m < NW; ++m) {
+        vp[m] = fma(sg, sp[m], pp[m]);
+        vmn[m] = fma(sg, sm[m], pm[m]);
+      }
+      const double f = weno_pm<ORDER>(vp, vmn, eps, shock);
+      if (e == 0) fch[0] = f; else fch[4] = f;
+    }
+#pragma unroll
+    for (int m = 0; m < 2 * R; ++m) {
+      const int o = m - R + 1;
+      const double uk = FvL(0, o), qj = QvL(0, o) * (0.5 * FvL(6, o));
+      if (m < NW) pp[m] = fma(-2.0, pp[m], qj * (uk + lam));
+      if (m > 0) pm[m - 1] = fma(-2.0, pm[m - 1], qj * (uk - lam));
+    }
+    fch[3] = weno_pm<ORDER>(pp, pm, eps, shock);
+  }
+  // the two shear fields
+#pragma unroll 1
+  for (int l = 0; l < 2; ++l) {
+    const double lx = l == 0 ? nx : qx, ly = l == 0 ? ny : qy, lz = l == 0 ? nz : qz, l0 = l == 0 ? -Un : -Uq;
     double vp[NW], vmn[NW];
 #pragma unroll
     for (int m = 0; m < 2 * R; ++m) {
       const int o = m - R + 1;
-      const double uk = FvL(0, o);
-      const double q0 = QvL(0, o), q4 = QvL(4, o);
-      double LF = L0 * (q0 * uk) + L1 * FvL(1, o) + L2 * FvL(2, o) + L3 * FvL(3, o) + L4 * ((q4 + FvL(4, o)) * uk);
-      double LQ = L0 * q0 + L1 * QvL(1, o) + L2 * QvL(2, o) + L3 * QvL(3, o) + L4 * q4;
-      if constexpr (NS > 0) {
-        LF += tc * sbf[m];
-        LQ += tc * sbq[m];
-      }
+      const double q0 = QvL(0, o);
+      const double LF = fma(l0, q0 * FvL(0, o), fma(lx, FvL(1, o), fma(ly, FvL(2, o), lz * FvL(3, o))));
+      const double LQ = fma(l0, q0, fma(lx, QvL(1, o), fma(ly, QvL(2, o), lz * QvL(3, o))));
       const double hj = 0.5 * FvL(6, o);
-      if (m < NW) vp[m] = hj * (LF + lam * LQ);
-      if (m > 0) vmn[m - 1] = hj * (LF - lam * LQ);
+      if (m < NW) vp[m] = hj * fma(lam, LQ, LF);
+      if (m > 0) vmn[m - 1] = hj * fma(-lam, LQ, LF);
     }
-    fch[l] = weno_pm<ORDER>(vp, vmn, eps, shock);
+    const double f = weno_pm<ORDER>(vp, vmn, eps, shock);
+    if (l == 0) fch[1] = f; else fch[2] = f;
   }
   // back-projection with the right eigenvectors
   const double f034 = fch[0] + fch[3] + fch[4];
@@ -190,7 +214,7 @@ __device__ __forceinline__ void load_node(const Zone &z, idx_t g, double *sQ, do
   const double m0 = z.metric[g + (3 * DIR) * sz], m1 = z.metric[g + (3 * DIR + 1) * sz],
                m2 = z.metric[g + (3 * DIR + 2) * sz];
   const double pk = z.bv[g + 4 * sz];
-  const double Uk = (q1 * m0 + q2 * m1 + q3 * m2) / q0;
+  const double Uk = (q1 * m0 + q2 * m1 + q3 * m2) * recip(q0);
   sQ[0 * NN + slot] = q0;
   sQ[1 * NN + slot] = q1;
   sQ[2 * NN + slot] = q2;
@@ -203,9 +227,10 @@ __device__ __forceinline__ void load_node(const Zone &z, idx_t g, double *sQ, do
   sF[2 * NN + slot] = fma(q2, Uk, pk * m1);
   sF[3 * NN + slot] = fma(q3, Uk, pk * m2);
   sF[4 * NN + slot] = pk;
-  double cg = norm3d(m0, m1, m2);
-  if constexpr (NS == 0) cg *= sqrt(kGammaAir * kRAir * z.bv[g + 5 * sz]);
-  else cg *= z.acoustic[g];
+  const double k2 = fma(m0, m0, fma(m1, m1, m2 * m2));
+  double cg;
+  if constexpr (NS == 0) cg = sqrt(k2 * (kGammaAir * kRAir * z.bv[g + 5 * sz]));
+  else cg = sqrt(k2) * z.acoustic[g];
   sF[5 * NN + slot] = cg;
   sF[6 * NN + slot] = z.jac[g];
 }
@@ -268,7 +293,9 @@ __device__ __forceinline__ void positive_limit(const double *sQ, const double *s
 }
 
 template <int NS, int DIR, int ORDER, bool TT = false>
-__global__ void __launch_bounds__(kSweepThreads, 2) k_weno_char(Zone z, Param p, idx_t run) {
+__global__ void __launch_bounds__(kSweepThreads, 2) k_weno_char(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                                                                   idx_t run) {
+  chain_begin();
   constexpr int NV = 5 + NS + (TT ? 1 : 0);
   constexpr int R = ORDER / 2 + 1;
   constexpr int NN = DIR == 0 ? (kSweepThreads + 2 * R - 1) : kTI * (kTS + 2 * R - 1);
@@ -362,9 +389,15 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_weno_char(Zone z, Param p,
     const int tprev = DIR == 0 ? tid - 1 : tid - kTI;
     const idx_t gd = z.L0.at(ni, nj, nk);
     const idx_t sz0 = z.L0.sz;
+    if (DIR == 0 && p.assign_x) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v)
-      z.dq[gd + v * sz0] -= sFl[v * kSweepThreads + tid] - sFl[v * kSweepThreads + tprev];
+      for (int v = 0; v < NV; ++v)
+        z.dq[gd + v * sz0] = -(sFl[v * kSweepThreads + tid] - sFl[v * kSweepThreads + tprev]);
+    } else {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        z.dq[gd + v * sz0] -= sFl[v * kSweepThreads + tid] - sFl[v * kSweepThreads + tprev];
+    }
   }
 }
 
@@ -556,17 +589,16 @@ static int launch_dir(int dir, const Zone &z, const Param &p, cudaStream_t s) {
   if (dir == 0) {
     auto kern = k_weno_char<NS, 0, ORDER, TT>;
     CB2_TRY(prepare_smem(kern, smem));
-    kern<<<grid, kSweepThreads, smem, s>>>(z, p, geo.run);
+    return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, geo.run);
   } else if (dir == 1) {
     auto kern = k_weno_char<NS, 1, ORDER, TT>;
     CB2_TRY(prepare_smem(kern, smem));
-    kern<<<grid, kSweepThreads, smem, s>>>(z, p, 0);
+    return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, (idx_t)0);
   } else {
     auto kern = k_weno_char<NS, 2, ORDER, TT>;
     CB2_TRY(prepare_smem(kern, smem));
-    kern<<<grid, kSweepThreads, smem, s>>>(z, p, 0);
+    return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, (idx_t)0);
   }
-  return check_launch();
 }
 
 template <int NS, bool TT = false>

@@ -4,7 +4,7 @@
 // weno7: Z-type weights a_r = d_r (1 + tau7/(eps+beta_r)^2), tau7 = (b0+3b1-3b2-b3)^2
 //        (src/WENO.cu:3090-3196).
 // Both fall back to the linear (optimal) weights when `shock` is false.
-// The normalised weights are evaluated with one division per side: every a_r is multiplied
+// The normalised weights are evaluated with one reciprocal per side: every a_r is multiplied
 // by the product of all (eps+beta)^2 terms, which leaves sum(a_r q_r)/sum(a_r) unchanged
 // (the reference divides once per sub-stencil, src/WENO.cu:3051-3053, 3127-3130).
 //
@@ -31,94 +31,64 @@ __device__ __forceinline__ float binade_inv(float x) {
   return __int_as_float(0x7F000000 - (__float_as_int(x) & 0x7F800000));
 }
 
-// ---- WENO5 -------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T weno5_plus(const T *v, T eps, bool shock) {
-  const T k6 = T(1.0 / 6);
-  // candidate stencils S2={i,i+1,i+2}, S1={i-1,i,i+1}, S0={i-2,i-1,i}
-  const T q2 = k6 * (2 * v[2] + 5 * v[3] - v[4]);
-  const T q1 = k6 * (-v[1] + 5 * v[2] + 2 * v[3]);
-  const T q0 = k6 * (2 * v[0] - 7 * v[1] + 11 * v[2]);
-  if (!shock) return T(0.3) * q2 + T(0.6) * q1 + T(0.1) * q0;
-  const T k13 = T(13.0 / 12);
-  const T b2 = k13 * sq(v[2] + v[4] - 2 * v[3]) + T(0.25) * sq(3 * v[2] - 4 * v[3] + v[4]);
-  const T b1 = k13 * sq(v[1] + v[3] - 2 * v[2]) + T(0.25) * sq(v[1] - v[3]);
-  const T b0 = k13 * sq(v[0] + v[2] - 2 * v[1]) + T(0.25) * sq(v[0] - 4 * v[1] + 3 * v[2]);
-  // a_r = d_r / D_r with D_r = (eps + beta_r)^2; multiplying every a_r by D0 D1 D2 leaves
-  // the normalised weights unchanged and needs one division instead of four
-  T D0 = sq(eps + b0), D1 = sq(eps + b1), D2 = sq(eps + b2);
-  const T sc = binade_inv(fmax(fmax(D0, D1), D2));
-  D0 *= sc; D1 *= sc; D2 *= sc;
-  const T w2 = T(0.3) * (D0 * D1), w1 = T(0.6) * (D0 * D2), w0 = T(0.1) * (D1 * D2);
-  return (w2 * q2 + w1 * q1 + w0 * q0) / (w2 + w1 + w0);
+// ---- one side of an interface ------------------------------------------------------------
+// FP64, from the undivided differences of the stencil (see the node-centred pair below): the
+// smoothness indicators and the candidate values, relative to the middle node, share them.
+__device__ __forceinline__ double pow2_inv_max(double a, double b, double c, double d) {
+  // the reciprocal binade of the largest: positive doubles order as their high words do
+  const int h = max(max(__double2hiint(a), __double2hiint(b)), max(__double2hiint(c), __double2hiint(d)));
+  return __hiloint2double(0x7FE00000 - (h & 0x7FF00000), 0);
 }
 
-template <typename T>
-__device__ __forceinline__ T weno5_minus(const T *v, T eps, bool shock) {
-  const T k6 = T(1.0 / 6);
-  const T q0 = k6 * (11 * v[2] - 7 * v[3] + 2 * v[4]);
-  const T q1 = k6 * (2 * v[1] + 5 * v[2] - v[3]);
-  const T q2 = k6 * (-v[0] + 5 * v[1] + 2 * v[2]);
-  if (!shock) return T(0.1) * q0 + T(0.6) * q1 + T(0.3) * q2;
-  const T k13 = T(13.0 / 12);
-  const T b0 = k13 * sq(v[2] + v[4] - 2 * v[3]) + T(0.25) * sq(3 * v[2] - 4 * v[3] + v[4]);
-  const T b1 = k13 * sq(v[1] + v[3] - 2 * v[2]) + T(0.25) * sq(v[1] - v[3]);
-  const T b2 = k13 * sq(v[0] + v[2] - 2 * v[1]) + T(0.25) * sq(v[0] - 4 * v[1] + 3 * v[2]);
-  T D0 = sq(eps + b0), D1 = sq(eps + b1), D2 = sq(eps + b2);
-  const T sc = binade_inv(fmax(fmax(D0, D1), D2));
-  D0 *= sc; D1 *= sc; D2 *= sc;
-  const T w0 = T(0.1) * (D1 * D2), w1 = T(0.6) * (D0 * D2), w2 = T(0.3) * (D0 * D1);
-  return (w0 * q0 + w1 * q1 + w2 * q2) / (w0 + w1 + w2);
+__device__ __forceinline__ double weno5_side(double u0, double u1, double u2, double u3, double u4, double eps,
+                                             bool shock) {
+  const double d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3;
+  const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
+  const double k3 = 1.0 / 3, k6 = 1.0 / 6, h1 = 0.5 * d1;
+  // candidates relative to u2; linear weights times ten: 1, 6, 3
+  const double c0 = fma(k3, s0, h1), c1 = fma(k3, s1, h1), c2 = fma(-k6, s2, 0.5 * d2);
+  if (!shock) return fma(0.3, c2, fma(0.6, c1, fma(0.1, c0, u2)));
+  const double f0 = fma(0.5, s0, d1), f1 = fma(0.5, s1, d1), f2 = fma(-0.5, s2, d2);
+  const double k13 = 13.0 / 12;
+  double A0 = fma(f0, f0, fma(k13 * s0, s0, eps)), A1 = fma(f1, f1, fma(k13 * s1, s1, eps)),
+         A2 = fma(f2, f2, fma(k13 * s2, s2, eps));
+  const double sc = pow2_inv_max(A0, A1, A2, A2);
+  A0 *= sc; A1 *= sc; A2 *= sc;
+  const double D0 = A0 * A0, D1 = A1 * A1, D2 = A2 * A2;
+  const double w0 = D1 * D2, w1 = 6.0 * (D0 * D2), E2 = D0 * D1, w2 = 3.0 * E2;
+  return fma(fma(w2, c2, fma(w1, c1, w0 * c0)), recip(fma(3.0, E2, w0 + w1)), u2);
 }
 
-// ---- WENO7 -------------------------------------------------------------------------
-// Smoothness indicator of one 4-point sub-stencil written with its first, second and
-// third undivided differences d1, d2, d3: beta = d1^2 + 13/12 d2^2 + 1043/960 d3^2 + d1 d3/12.
-template <typename T>
-__device__ __forceinline__ T beta7(T d1, T d2, T d3) {
-  return d1 * d1 + T(13.0 / 12.0) * d2 * d2 + T(1043.0 / 960) * d3 * d3 + T(1.0 / 12) * d1 * d3;
-}
-
-// Plus side on u[0..6] (u[3] = node i).  The minus side is the same function applied to
-// the mirrored stencil (u[k] = v[6-k]) of the right-biased values.
-template <typename T>
-__device__ __forceinline__ T weno7_side(T u0, T u1, T u2, T u3, T u4, T u5, T u6, T eps, bool shock) {
-  const T c0 = T(1.0 / 35), c1 = T(12.0 / 35), c2 = T(18.0 / 35), c3 = T(4.0 / 35);
-  const T q0 = -3 * u0 + 13 * u1 - 23 * u2 + 25 * u3;
-  const T q1 = u1 - 5 * u2 + 13 * u3 + 3 * u4;
-  const T q2 = -u2 + 7 * u3 + 7 * u4 - u5;
-  const T q3 = 3 * u3 + 13 * u4 - 5 * u5 + u6;
-  if (!shock) return T(1.0 / 12) * (c0 * q0 + c1 * q1 + c2 * q2 + c3 * q3);
-  const T k6 = T(1.0 / 6);
-  const T b0 = beta7(k6 * (-2 * u0 + 9 * u1 - 18 * u2 + 11 * u3), -u0 + 4 * u1 - 5 * u2 + 2 * u3,
-                     -u0 + 3 * u1 - 3 * u2 + u3);
-  const T d2m = u2 - 2 * u3 + u4;  // shared second difference of sub-stencils 1 and 2
-  const T b1 = beta7(k6 * (u1 - 6 * u2 + 3 * u3 + 2 * u4), d2m, -u1 + 3 * u2 - 3 * u3 + u4);
-  const T b2 = beta7(k6 * (-2 * u2 - 3 * u3 + 6 * u4 - u5), d2m, -u2 + 3 * u3 - 3 * u4 + u5);
-  const T b3 = beta7(k6 * (-11 * u3 + 18 * u4 - 9 * u5 + 2 * u6), 2 * u3 - 5 * u4 + 4 * u5 - u6,
-                     -u3 + 3 * u4 - 3 * u5 + u6);
-  T tau = sq(b0 + 3 * b1 - 3 * b2 - b3);
-  // a_r = c_r (1 + tau/D_r) = c_r (D_r + tau)/D_r, D_r = (eps + beta_r)^2; scaled by
-  // D0 D1 D2 D3 the normalised weights need a single division.  D_r and tau are first
-  // brought to the binade of the largest D_r, so the triple products cannot underflow.
-  T D0 = sq(eps + b0), D1 = sq(eps + b1), D2 = sq(eps + b2), D3 = sq(eps + b3);
-  const T sc = binade_inv(fmax(fmax(D0, D1), fmax(D2, D3)));
-  D0 *= sc; D1 *= sc; D2 *= sc; D3 *= sc; tau *= sc;
-  const T D01 = D0 * D1, D23 = D2 * D3;
-  const T w0 = c0 * (D0 + tau) * (D1 * D23);
-  const T w1 = c1 * (D1 + tau) * (D0 * D23);
-  const T w2 = c2 * (D2 + tau) * (D01 * D3);
-  const T w3 = c3 * (D3 + tau) * (D01 * D2);
-  return T(1.0 / 12) * (w0 * q0 + w1 * q1 + w2 * q2 + w3 * q3) / (w0 + w1 + w2 + w3);
-}
-
-template <typename T>
-__device__ __forceinline__ T weno7_plus(const T *v, T eps, bool shock) {
-  return weno7_side(v[0], v[1], v[2], v[3], v[4], v[5], v[6], eps, shock);
-}
-template <typename T>
-__device__ __forceinline__ T weno7_minus(const T *v, T eps, bool shock) {
-  return weno7_side(v[6], v[5], v[4], v[3], v[2], v[1], v[0], eps, shock);
+__device__ __forceinline__ double weno7_side(double u0, double u1, double u2, double u3, double u4, double u5,
+                                             double u6, double eps, bool shock) {
+  const double d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4, d5 = u6 - u5;
+  const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2, s3 = d4 - d3, s4 = d5 - d4;
+  const double t0 = s1 - s0, t1 = s2 - s1, t2 = s3 - s2, t3 = s4 - s3;
+  const double k3 = 1.0 / 3, k6 = 1.0 / 6, k12 = 1.0 / 12;
+  const double h2 = 0.5 * d2, e = fma(k3, s2, h2);
+  const double c0 = fma(0.25, t0, fma(k3, s1, h2)), c1 = fma(-k12, t1, e), c2 = fma(-k12, t2, e),
+               c3 = fma(k12, t3, fma(-k6, s3, 0.5 * d3));
+  if (!shock)
+    return fma(4.0 / 35, c3, fma(18.0 / 35, c2, fma(12.0 / 35, c1, fma(1.0 / 35, c0, u3))));
+  const double c = fma(0.5, s2, d2);
+  const double f0 = fma(k3, t0, fma(0.5, s1, d2)), f1 = fma(-k6, t1, c), f2 = fma(-k6, t2, c),
+               f3 = fma(k3, t3, fma(-0.5, s3, d3));
+  const double g0 = s1 + t0, g3 = s3 - t3;
+  const double kg = 13.0 / 12, kt = 1043.0 / 960;
+  const double gm = (kg * s2) * s2;
+  const double b0 = fma(f0, fma(k12, t0, f0), fma(kt * t0, t0, (kg * g0) * g0));
+  const double b1 = fma(f1, fma(k12, t1, f1), fma(kt * t1, t1, gm));
+  const double b2 = fma(f2, fma(k12, t2, f2), fma(kt * t2, t2, gm));
+  const double b3 = fma(f3, fma(k12, t3, f3), fma(kt * t3, t3, (kg * g3) * g3));
+  double tz = fma(3.0, b1 - b2, b0 - b3);
+  double A0 = eps + b0, A1 = eps + b1, A2 = eps + b2, A3 = eps + b3;
+  const double sc = pow2_inv_max(A0, A1, A2, A3);
+  A0 *= sc; A1 *= sc; A2 *= sc; A3 *= sc; tz *= sc;
+  const double D0 = A0 * A0, D1 = A1 * A1, D2 = A2 * A2, D3 = A3 * A3;
+  const double D01 = D0 * D1, D23 = D2 * D3;
+  const double w0 = fma(tz, tz, D0) * (D1 * D23), w1 = 12.0 * (fma(tz, tz, D1) * (D0 * D23));
+  const double w2 = 18.0 * (fma(tz, tz, D2) * (D01 * D3)), E3 = fma(tz, tz, D3) * (D01 * D2), w3 = 4.0 * E3;
+  return fma(fma(w3, c3, fma(w2, c2, fma(w1, c1, w0 * c0))), recip(fma(4.0, E3, (w0 + w1) + w2)), u3);
 }
 
 // FP32 weights.  The single-division product form needs the product of three or four
@@ -148,12 +118,6 @@ __device__ __forceinline__ float rcp32(float x) { return __fdividef(1.0f, x); }
 // sums over point values took about 190, and it is the more exact one (no cancellation of the node
 // values).  Sums of products are written as fused operations, so that every kernel that inlines
 // these functions rounds alike.  FP64 only; the FP32 pair is packed (below).
-__device__ __forceinline__ double pow2_inv_max(double a, double b, double c, double d) {
-  // the reciprocal binade of the largest: positive doubles order as their high words do
-  const int h = max(max(__double2hiint(a), __double2hiint(b)), max(__double2hiint(c), __double2hiint(d)));
-  return __hiloint2double(0x7FE00000 - (h & 0x7FF00000), 0);
-}
-
 __device__ __forceinline__ void weno5_node(const double *v, double eps, double &lp, double &rm) {
   const double d0 = v[1] - v[0], d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3];
   const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
@@ -297,10 +261,15 @@ __device__ __forceinline__ void weno7_node_x2(const float *u, float eps, float &
   rm = r.y;
 }
 
-template <int ORDER, typename T>
-__device__ __forceinline__ T weno_pm(const T *vp, const T *vm, T eps, bool shock) {
-  if constexpr (ORDER == 5) return weno5_plus(vp, eps, shock) + weno5_minus(vm, eps, shock);
-  else return weno7_plus(vp, eps, shock) + weno7_minus(vm, eps, shock);
+// plus + minus value of an interface; vp / vm: the NW values of each side's stencil
+template <int ORDER>
+__device__ __forceinline__ double weno_pm(const double *vp, const double *vm, double eps, bool shock) {
+  if constexpr (ORDER == 5)
+    return weno5_side(vp[0], vp[1], vp[2], vp[3], vp[4], eps, shock) +
+           weno5_side(vm[4], vm[3], vm[2], vm[1], vm[0], eps, shock);
+  else
+    return weno7_side(vp[0], vp[1], vp[2], vp[3], vp[4], vp[5], vp[6], eps, shock) +
+           weno7_side(vm[6], vm[5], vm[4], vm[3], vm[2], vm[1], vm[0], eps, shock);
 }
 
 }  // namespace cb2
