@@ -154,15 +154,39 @@ int fail_cuda(cudaError_t e) {
   return CB2_ERR_CUDA;
 }
 
-// The NASA7 table that travels in the kernels' parameters (ThermoTab).
+// The thermodynamic table that travels in the kernels' parameters (ThermoTab); use = 0 where the
+// mechanism does not fit one.
 void fill_thermo_tab(const cb2_mechanism &m, ThermoTab &t) {
   t = ThermoTab{};
-  if (m.therm_nasa_7_9 == 9 || m.n_spec > kMaxSpec) return;
+  if (m.therm_nasa_7_9 == 9) {
+    if (m.n_spec > kTab9Spec) return;
+    const int nr = m.n_temperature_range[0], row = m.max_range + 1;
+    if (nr > kTab9Range) return;
+    for (int s = 0; s < m.n_spec; ++s) {
+      if (m.n_temperature_range[s] != nr) return;
+      for (int r = 0; r <= nr; ++r)
+        if (m.temperature_range[s * row + r] != m.temperature_range[r]) return;
+      const double g = kRu / m.mw[s];
+      for (int r = 0; r < nr; ++r) {
+        const double *a = m.therm_poly_coeff + ((size_t)s * m.max_range + r) * 9;
+        for (int n = 0; n < 7; ++n) t.cp9[r][s][n] = a[n] * g;
+        for (int n = 0; n < 4; ++n) t.h9[r][s][n] = a[3 + n] / (n + 2) * g;
+        t.h9[r][s][4] = a[7] * g;
+      }
+    }
+    t.t_low = m.temperature_range[0];
+    t.t_high = m.temperature_range[nr];
+    t.cut[0] = nr > 1 ? m.temperature_range[1] : t.t_high;
+    t.cut[1] = nr > 2 ? m.temperature_range[2] : t.t_high;
+    t.use = 2;
+    return;
+  }
+  if (m.n_spec > kMaxSpec) return;
   t.t_low = m.t_low[0];
-  t.t_mid = m.t_mid[0];
+  t.cut[0] = m.t_mid[0];
   t.t_high = m.t_high[0];
   for (int s = 0; s < m.n_spec; ++s) {
-    if (m.t_mid[s] != t.t_mid) return;
+    if (m.t_mid[s] != t.cut[0]) return;
     t.t_low = std::max(t.t_low, m.t_low[s]);
     t.t_high = std::min(t.t_high, m.t_high[s]);
     const double r = kRu / m.mw[s];
@@ -171,6 +195,10 @@ void fill_thermo_tab(const cb2_mechanism &m, ThermoTab &t) {
       for (int n = 0; n < 5; ++n) t.cp[h][s][n] = a[n] * r;
       t.h[h][s][0] = a[5] * r;
       for (int n = 1; n < 5; ++n) t.h[h][s][n] = a[n] / (n + 1) * r;
+      for (int n = 0; n < 5; ++n) {
+        t.cpf[h][s][n] = (float)t.cp[h][s][n];
+        t.hf[h][s][n] = (float)t.h[h][s][n];
+      }
     }
   }
   t.use = 1;
@@ -200,6 +228,8 @@ int upload_mechanism(const cb2_mechanism &m, const cb2_two_temperature *tt, cb2_
     imw[s] = 1.0 / m.mw[s];
     rg[s] = kRu / m.mw[s];
     mw2[s] = 1.0 / imw[s];
+    d.iw[s] = imw[s];
+    d.rg[s] = rg[s];
   }
   addd(&d.imw, imw.data(), ns);
   addd(&d.gas_const, rg.data(), ns);
@@ -268,8 +298,23 @@ int upload_mechanism(const cb2_mechanism &m, const cb2_two_temperature *tt, cb2_
     addd(&d.theta_v, tt->theta_v, ns);
     addd(&d.elec_theta, tt->elec_theta, ns * ml);
     addd(&d.elec_g, tt->elec_g, ns * ml);
-    addd(&d.lt_a, tt->lt_a, (size_t)ns * ns);
-    addd(&d.lt_b, tt->lt_b, (size_t)ns * ns);
+    // Millikan-White constants of every pair: the given ones, or the defaults
+    // (src/Thermo.cu:806-812)
+    std::vector<double> la((size_t)ns * ns), lb((size_t)ns * ns);
+    for (int v = 0; v < ns; ++v)
+      for (int q = 0; q < ns; ++q) {
+        double a = tt->lt_a[v * ns + q], b = tt->lt_b[v * ns + q];
+        if (a <= 0.0 || b <= 0.0) {
+          const double mv = 1.0 / std::max(imw[v], 1e-20), mp = 1.0 / std::max(imw[q], 1e-20);
+          const double mu = mv * mp / std::max(mv + mp, 1e-20);
+          a = 1.16e-3 * std::sqrt(std::max(mu, 1e-20)) * std::pow(std::max(tt->theta_v[v], 0.0), 4.0 / 3.0);
+          b = 0.015 * std::pow(std::max(mu, 1e-20), 0.25);
+        }
+        la[(size_t)v * ns + q] = a;
+        lb[(size_t)v * ns + q] = b;
+      }
+    addd(&d.lt_a, la.data(), (size_t)ns * ns);
+    addd(&d.lt_b, lb.data(), (size_t)ns * ns);
     addd(&d.park_sigma, tt->park_sigma, ns);
     addi(&d.n_level, tt->n_level, ns);
     // Electronic levels past which the partition sums stop changing (see ve_energy): for

@@ -84,20 +84,32 @@ struct Zone {
 struct ChemTabs;   // chem_tab.cuh
 struct TransTabs;  // transport_tab.cuh
 
-// NASA7 coefficients of both ranges, by value in the kernels' parameters (thermo.cuh, tab_h_cp):
-// cp = c0 + c1 T + .. and h = a0 + T (c0 + T (a1 + T (a2 + ..))), scaled by the gas constant and the
-// integration factors.  use = 1 where every species has the same middle temperature; valid on
-// [t_low, t_high], the range that every fit covers.
+// Thermodynamic polynomials by value in the kernels' parameters (thermo.cuh, tab_h_cp), scaled by the
+// gas constant and the integration factors; valid on [t_low, t_high], the range that every fit covers.
+//   use = 1, NASA7, every species with the same middle temperature cut[0]:
+//     cp = c0 + c1 T + .., h = a0 + T (c0 + T (a1 + T (a2 + ..)))
+//   use = 2, NASA9 of up to five species with the same (up to three) ranges, cut at cut[0], cut[1]:
+//     cp = (c0 / T + c1) / T + c2 + c3 T + .., h = -c0 / T + c1 ln T + T (c2 + T (a0 + T (a1 + ..))) + b
+constexpr int kTab9Spec = 5, kTab9Range = 3;
 struct ThermoTab {
   int use;
-  double t_low, t_mid, t_high;
-  double h[2][kMaxSpec][5], cp[2][kMaxSpec][5];
+  double t_low, t_high, cut[2];
+  union {
+    struct {
+      double h[2][kMaxSpec][5], cp[2][kMaxSpec][5];
+      float hf[2][kMaxSpec][5], cpf[2][kMaxSpec][5];  // the same in FP32 (the mixed form's sweeps)
+    };
+    struct {
+      double h9[kTab9Range][kTab9Spec][5], cp9[kTab9Range][kTab9Spec][7];  // h9: a0 .. a3, b
+    };
+  };
 };
 
 // Mechanism tables in device memory (copied from cb2_mechanism by cb2_init).
 struct Mech {
   int n_spec, n_reac;
   const double *imw, *gas_const, *mw;
+  double iw[kMaxSpec], rg[kMaxSpec];  // imw and gas_const by value, for loops over whole mechanisms
   const double *lo, *hi;         // [n_spec*7]
   const double *t_low, *t_mid, *t_high;
   const double *geometry, *lj_inv, *vis_coeff;

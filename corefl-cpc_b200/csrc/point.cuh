@@ -11,21 +11,55 @@
 
 namespace cb2 {
 
+// The mixture's NASA7 coefficients in range R: h = h0 + T (c0 + T (a1 + ..)), cp = c0 + T (c1 + ..).
+struct MixturePoly {
+  double h0, c0, a[4], c[4];
+};
+template <int NS, int R>
+__device__ __forceinline__ MixturePoly mixture_poly(const double *y, const ThermoTab &m) {
+  MixturePoly q{};
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    q.h0 = fma(y[s], m.h[R][s][0], q.h0);
+    q.c0 = fma(y[s], m.cp[R][s][0], q.c0);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      q.a[n] = fma(y[s], m.h[R][s][n + 1], q.a[n]);
+      q.c[n] = fma(y[s], m.cp[R][s][n + 1], q.c[n]);
+    }
+  }
+  return q;
+}
+
 // Newton inversion of T from the internal energy e (1T mixtures): stops at |1 - T1/T| <= 1e-5
 // or after 1000 iterations, starting from the previous temperature (src/FieldOperation.cu:67-85).
+// Inside the range of a NASA7 table an iteration is two Horner evaluations of the mixture's
+// polynomial, formed once (again if T crosses the middle); beyond it the species are summed.
 template <int NS>
 __device__ __forceinline__ double newton_temperature(double e, const double *y, double r_mix, double t,
                                                      const Mech &m) {
   double err = 1;
-  int iter = 0;
-  double h[NS], cp[NS];
+  int iter = 0, range = -1;
+  MixturePoly q{};
   while (err > 1e-5 && iter++ < 1000) {
-    species_h_cp<NS>(t, m, h, cp);
     double cpt = 0, ht = 0;
+    if (m.tab.use == 1 && t >= m.tab.t_low && t <= m.tab.t_high) {
+      const int want = t < m.tab.cut[0] ? 0 : 1;
+      if (want != range) {
+        range = want;
+        if (want == 0) q = mixture_poly<NS, 0>(y, m.tab);
+        else q = mixture_poly<NS, 1>(y, m.tab);
+      }
+      ht = fma(t, fma(t, fma(t, fma(t, fma(t, q.a[3], q.a[2]), q.a[1]), q.a[0]), q.c0), q.h0);
+      cpt = fma(t, fma(t, fma(t, fma(t, q.c[3], q.c[2]), q.c[1]), q.c[0]), q.c0);
+    } else {
+      double h[NS], cp[NS];
+      species_h_cp<NS>(t, m, h, cp);
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      cpt += cp[s] * y[s];
-      ht += h[s] * y[s];
+      for (int s = 0; s < NS; ++s) {
+        cpt += cp[s] * y[s];
+        ht += h[s] * y[s];
+      }
     }
     const double et = ht - r_mix * t;
     const double cvt = cpt - r_mix;
@@ -39,10 +73,10 @@ __device__ __forceinline__ double newton_temperature(double e, const double *y, 
 // SSP-RK3 stage update of one interior node (update_cv_and_bv_rk<mix>, src/RK.cuh:277-367).
 // TT: two-temperature model, rho*e_ve at cv comp 5 + NS (clipped at zero), e_ve at sv comp NS,
 // T_ve and T from the two-temperature inversion.
-// first: qn is not stored yet: it takes cv's value, which stands for it here (stage 0).
-template <int NS, bool TT = false>
+// FIRST: stage 0 with qn not stored yet: qn takes cv's value, which stands for it here.
+template <int NS, bool TT = false, bool FIRST = false>
 __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p, double dt, int rk, int i, int j,
-                                                   int k, bool first = false) {
+                                                   int k) {
   static_assert(!TT || NS > 0, "the two-temperature model needs species");
   constexpr int NV = 5 + NS + (TT ? 1 : 0);
   double a, b, c;
@@ -51,7 +85,7 @@ __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p
   const idx_t g0 = z.L0.at(i, j, k), sz0 = z.L0.sz;
   const double dtj = dt / z.jac[g];
   double q[NV];
-  if (first) {
+  if constexpr (FIRST) {
 #pragma unroll
     for (int l = 0; l < NV; ++l) {
       const double v = z.cv[g + l * sz];
@@ -103,7 +137,10 @@ __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p
       return;
     }
 #pragma unroll
-    for (int s = 0; s < NS; ++s) r_mix += y[s] * __ldg(p.mech.gas_const + s);
+    for (int s = 0; s < NS; ++s) r_mix += y[s] * p.mech.rg[s];
+    // cv is final here; storing it before the iteration frees its registers
+#pragma unroll
+    for (int l = 0; l < NV; ++l) z.cv[g + l * sz] = q[l];
     const double e = q[4] / rho - 0.5 * V2;
     const double t = newton_temperature<NS>(e, y, r_mix, z.bv[g + 5 * sz], p.mech);
     const double pr = rho * t * r_mix;
@@ -111,8 +148,10 @@ __device__ __forceinline__ void stage_update_point(const Zone &z, const Param &p
     z.bv[g + 4 * sz] = pr;
     if (!(t > 0) || !(pr > 0)) flag_status(p, 2u);
   }
+  if constexpr (NS == 0) {
 #pragma unroll
-  for (int l = 0; l < NV; ++l) z.cv[g + l * sz] = q[l];
+    for (int l = 0; l < NV; ++l) z.cv[g + l * sz] = q[l];
+  }
 }
 
 // Physical properties of one node (update_physical_properties<mix>,
@@ -137,7 +176,7 @@ __device__ __forceinline__ void properties_point(const Zone &z, const Param &p, 
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       y[s] = z.sv[g + s * sz];
-      imw = fma(y[s], __ldg(p.mech.imw + s), imw);
+      imw = fma(y[s], p.mech.iw[s], imw);
       cpt = fma(y[s], cp[s], cpt);
     }
     const double mw = 1 / fmax(imw, 1e-12);

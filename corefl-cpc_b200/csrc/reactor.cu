@@ -660,7 +660,7 @@ int launch_reactor_advance(const Param &p, cb2_reactor *r, int n, int max_attemp
   const unsigned blocks = (unsigned)((n + kReactorWarps - 1) / kReactorWarps);
   ProfScope prof(krylov ? "reactor_advance_krylov" : "reactor_advance", s);
   const unsigned th = 32 * kReactorWarps;
-  const ChemTabs *tab = !krylov && p.mech.tab.use ? p.mech.chem_tabs : nullptr;
+  const ChemTabs *tab = !krylov && p.mech.tab.use == 1 ? p.mech.chem_tabs : nullptr;
   if (tab && tab->ns == 9) {
     k_reactor_rok4e<9><<<blocks, th, 0, s>>>(r, n, p.mech, tab->t9, static_cast<const ChemReac<9> *>(tab->rows),
                                              max_attempts, rtol, atol);

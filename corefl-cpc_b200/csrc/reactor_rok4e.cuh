@@ -161,7 +161,7 @@ __device__ __noinline__ double rok_temperature(double t0, double y, double irho,
   double h0, c0, a1, a2, a3, a4, c1, c2, c3, c4;
   int range = -1;
   for (int iter = 0; err > 1e-8 && iter < 100; ++iter) {
-    const int want = t < mech.tab.t_mid ? 0 : 1;
+    const int want = t < mech.tab.cut[0] ? 0 : 1;
     if (want != range) {
       range = want;
       __syncwarp();

@@ -87,23 +87,39 @@ __device__ __forceinline__ void nasa9_gibbs_rt(double t, const Mech &m, double *
 // species' fit: the coefficients, scaled by the gas constant and the integration factors at upload,
 // are constant-bank operands of the Horner steps (one instruction each), where reading them from
 // memory costs as many loads as the arithmetic and the generic form divides by 3 per species.
+template <int NS, int R>
+__device__ __forceinline__ void tab7_range(double t, const ThermoTab &m, double *h, double *cp) {
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double *a = m.h[R][s], *c = m.cp[R][s];
+    if (h) h[s] = fma(t, fma(t, fma(t, fma(t, fma(t, a[4], a[3]), a[2]), a[1]), c[0]), a[0]);
+    if (cp) cp[s] = fma(t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), c[0]);
+  }
+}
+template <int NS, int R>
+__device__ __forceinline__ void tab9_range(double t, double it, double lnt, const ThermoTab &m, double *h, double *cp) {
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double *a = m.h9[R][s], *c = m.cp9[R][s];
+    if (h)
+      h[s] = fma(t, fma(t, fma(t, fma(t, fma(t, a[3], a[2]), a[1]), a[0]), c[2]),
+                 fma(c[1], lnt, fma(-c[0], it, a[4])));
+    if (cp) cp[s] = fma(it, fma(c[0], it, c[1]), fma(t, fma(t, fma(t, fma(t, c[6], c[5]), c[4]), c[3]), c[2]));
+  }
+}
 template <int NS>
 __device__ __forceinline__ void tab_h_cp(double t, const ThermoTab &m, double *h, double *cp) {
-  if (t < m.t_mid) {
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const double *a = m.h[0][s], *c = m.cp[0][s];
-      if (h) h[s] = fma(t, fma(t, fma(t, fma(t, fma(t, a[4], a[3]), a[2]), a[1]), c[0]), a[0]);
-      if (cp) cp[s] = fma(t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), c[0]);
-    }
-  } else {
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const double *a = m.h[1][s], *c = m.cp[1][s];
-      if (h) h[s] = fma(t, fma(t, fma(t, fma(t, fma(t, a[4], a[3]), a[2]), a[1]), c[0]), a[0]);
-      if (cp) cp[s] = fma(t, fma(t, fma(t, fma(t, c[4], c[3]), c[2]), c[1]), c[0]);
+  if constexpr (NS <= kTab9Spec) {
+    if (m.use == 2) {
+      const double it = 1.0 / t, lnt = h ? log(t) : 0.0;
+      if (t <= m.cut[0]) tab9_range<NS, 0>(t, it, lnt, m, h, cp);
+      else if (t <= m.cut[1]) tab9_range<NS, 1>(t, it, lnt, m, h, cp);
+      else tab9_range<NS, 2>(t, it, lnt, m, h, cp);
+      return;
     }
   }
+  if (t < m.cut[0]) tab7_range<NS, 0>(t, m, h, cp);
+  else tab7_range<NS, 1>(t, m, h, cp);
 }
 
 // h_k [J/kg] and cp_k [J/(kg K)] of every species at temperature t
@@ -246,7 +262,7 @@ __device__ __forceinline__ void characteristic_thermo(double t, const double *y,
   double e_tr = 0, r = 0, cpm = 0, cvm = 0;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    const double rs = __ldg(m.gas_const + s);
+    const double rs = m.rg[s];
     e_tr += y[s] * (h[s] - rs * te);
     r += y[s] * rs;
     cpm += y[s] * cp[s];
@@ -261,10 +277,20 @@ __device__ __forceinline__ void characteristic_thermo(double t, const double *y,
     const double inv_gm1 = 1.0 / fmax(gm1, 1e-12);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const double a = (gamma * __ldg(m.gas_const + s) * te - gm1 * h[s]) / c2;
+      const double a = (gamma * m.rg[s] * te - gm1 * h[s]) / c2;
       alpha[s] = a;
       ecoef[s] = -a * c2 * inv_gm1;
     }
+  }
+}
+
+template <int NS, int R>
+__device__ __forceinline__ void tab7_range_f32(float t, const ThermoTab &m, float *h, float *cp) {
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const float *a = m.hf[R][s], *c = m.cpf[R][s];
+    h[s] = fmaf(t, fmaf(t, fmaf(t, fmaf(t, fmaf(t, a[4], a[3]), a[2]), a[1]), c[0]), a[0]);
+    cp[s] = fmaf(t, fmaf(t, fmaf(t, fmaf(t, c[4], c[3]), c[2]), c[1]), c[0]);
   }
 }
 
@@ -273,6 +299,11 @@ __device__ __forceinline__ void characteristic_thermo(double t, const double *y,
 // structure, coefficients rounded to FP32.
 template <int NS>
 __device__ __forceinline__ void species_h_cp_f32(float t, const Mech &m, float *h, float *cp) {
+  if (m.tab.use == 1 && t >= float(m.tab.t_low) && t <= float(m.tab.t_high)) {
+    if (t < float(m.tab.cut[0])) tab7_range_f32<NS, 0>(t, m.tab, h, cp);
+    else tab7_range_f32<NS, 1>(t, m.tab, h, cp);
+    return;
+  }
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     const float tl = float(__ldg(m.t_low + s)), th = float(__ldg(m.t_high + s));
@@ -285,7 +316,7 @@ __device__ __forceinline__ void species_h_cp_f32(float t, const Mech &m, float *
     float hs = tt * (c0 + tt * (0.5f * c1 + tt * (c2 * (1.0f / 3) + tt * (0.25f * c3 + tt * (0.2f * c4))))) + c5;
     const float cps = c0 + tt * (c1 + tt * (c2 + tt * (c3 + tt * c4)));
     if (out) hs += cps * (t - tt);
-    const float r = float(__ldg(m.gas_const + s));
+    const float r = float(m.rg[s]);
     h[s] = hs * r;
     cp[s] = cps * r;
   }
@@ -300,7 +331,7 @@ __device__ __forceinline__ void characteristic_thermo_f32(float t, const float *
   float e_tr = 0, r = 0, cpm = 0, cvm = 0;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    const float rs = float(__ldg(m.gas_const + s));
+    const float rs = float(m.rg[s]);
     e_tr += y[s] * (h[s] - rs * te);
     r += y[s] * rs;
     cpm += y[s] * cp[s];
@@ -315,7 +346,7 @@ __device__ __forceinline__ void characteristic_thermo_f32(float t, const float *
     const float inv_gm1 = 1.0f / fmaxf(gm1, 1e-12f);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const float a = (gamma * float(__ldg(m.gas_const + s)) * te - gm1 * h[s]) / c2;
+      const float a = (gamma * float(m.rg[s]) * te - gm1 * h[s]) / c2;
       alpha[s] = a;
       ecoef[s] = -a * c2 * inv_gm1;
     }

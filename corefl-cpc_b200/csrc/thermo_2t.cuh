@@ -20,7 +20,7 @@ __device__ __forceinline__ double vib_energy(int i, double t, const Mech &m) {
   double e = 0.0;
   if (th > 0) {
     const double x = th / temp;
-    if (x < 200) e += __ldg(m.gas_const + i) * th / expm1(x);
+    if (x < 200) e += m.rg[i] * th / expm1(x);
   }
   return e;
 }
@@ -34,7 +34,7 @@ __device__ __forceinline__ double vib_cv(int i, double t, const Mech &m) {
     if (x < 200) {
       const double ex = exp(x);
       const double d = ex - 1.0;
-      c += __ldg(m.gas_const + i) * x * x * ex / (d * d);
+      c += m.rg[i] * x * x * ex / (d * d);
     }
   }
   return c;
@@ -48,8 +48,8 @@ __device__ __forceinline__ double vib_cv(int i, double t, const Mech &m) {
 // the result -- unchanged.  At the cold freestream of a hypersonic case this skips most of the
 // 46 exponentials of AIR5.
 __device__ __forceinline__ double ve_energy(int i, double t, const Mech &m, double *cv) {
-  const double temp = fmax(t, 1.0);
-  const double r = __ldg(m.gas_const + i);
+  const double temp = fmax(t, 1.0), it = 1.0 / temp;
+  const double r = m.rg[i];
   double e = vib_energy(i, temp, m);
   double c = cv ? vib_cv(i, temp, m) : 0.0;
   const int nl = __ldg(m.n_level + i);
@@ -61,7 +61,7 @@ __device__ __forceinline__ double ve_energy(int i, double t, const Mech &m, doub
       const double th = __ldg(m.elec_theta + i * m.max_level + l);
       if (l == 1) th1 = th;
       else if (l > 1 && th - th1 > cut_t) break;
-      const double bz = __ldg(m.elec_g + i * m.max_level + l) * exp(-th / temp);
+      const double bz = __ldg(m.elec_g + i * m.max_level + l) * exp(-th * it);
       zs += bz;
       b += bz * th;
       cc += bz * th * th;
@@ -70,7 +70,7 @@ __device__ __forceinline__ double ve_energy(int i, double t, const Mech &m, doub
       e += r * b / zs;
       if (cv) {
         const double mean = b / zs;
-        c += r * (cc / zs - mean * mean) / (temp * temp);
+        c += r * (cc / zs - mean * mean) * (it * it);
       }
     }
   }
@@ -111,7 +111,7 @@ __device__ __forceinline__ double mixture_tr_energy(double t, const double *y, c
   double e = 0.0, cpm = 0.0, rm = 0.0;
 #pragma unroll
   for (int i = 0; i < NS; ++i) {
-    const double r = __ldg(m.gas_const + i);
+    const double r = m.rg[i];
     cpm += y[i] * cp[i];
     rm += y[i] * r;
     e += y[i] * (h[i] - r * t);
@@ -133,7 +133,7 @@ __device__ __forceinline__ void tr_heat_capacities(double t, const double *y, co
 #pragma unroll
   for (int i = 0; i < NS; ++i) {
     cpm += y[i] * cp[i];
-    rm += y[i] * __ldg(m.gas_const + i);
+    rm += y[i] * m.rg[i];
   }
   double cv_eq;
   mixture_ve_energy<NS>(t, y, m, &cv_eq);
@@ -163,34 +163,27 @@ __device__ __forceinline__ double invert_tve_from_eve(double eve_target, const d
   return tve;
 }
 
-// Millikan-White time of the pair (vibrator iv, partner ip) at (t, p) (src/Thermo.cu:800-821).
-__device__ __forceinline__ double pair_mw_time(int iv, int ip, double t, double pr, const Mech &m) {
+// Millikan-White time of the pair (vibrator iv, partner ip) (src/Thermo.cu:800-821); t13 = t^(-1/3).
+// The pair's constants are resolved at mechanism upload (the given ones, or the defaults from the
+// reduced mass and the vibrational temperature).
+__device__ __forceinline__ double pair_mw_time(int iv, int ip, double t, double t13, double pr, const Mech &m) {
   if (pr <= 1e-16 || t <= 1.0) return 1e30;
-  const double mv = 1.0 / fmax(__ldg(m.imw + iv), 1e-20);
-  const double mp = 1.0 / fmax(__ldg(m.imw + ip), 1e-20);
-  const double mu = mv * mp / fmax(mv + mp, 1e-20);
-  double a = __ldg(m.lt_a + iv * m.n_spec + ip);
-  double b = __ldg(m.lt_b + iv * m.n_spec + ip);
-  if (a <= 0.0 || b <= 0.0) {
-    a = 1.16e-3 * sqrt(fmax(mu, 1e-20)) * pow(fmax(__ldg(m.theta_v + iv), 0.0), 4.0 / 3.0);
-    b = 0.015 * pow(fmax(mu, 1e-20), 0.25);
-  }
-  const double ex = a * (pow(t, -1.0 / 3.0) - b) - 18.421;
+  const double ex = __ldg(m.lt_a + iv * m.n_spec + ip) * (t13 - __ldg(m.lt_b + iv * m.n_spec + ip)) - 18.421;
   return fmax(exp(ex) * kPatm / pr, 1e-30);
 }
 
 // Relaxation time of vibrator iv: mole-weighted Millikan-White plus Park's high-temperature
 // correction (src/Thermo.cu:823-853).
 template <int NS>
-__device__ __forceinline__ double species_vt_time(int iv, double density, double t, double pr, const double *y,
-                                                  const Mech &m) {
+__device__ __forceinline__ double species_vt_time(int iv, double density, double t, double t13, double pr,
+                                                  const double *y, const Mech &m) {
   double conc = 0.0, denom = 0.0;
 #pragma unroll
   for (int j = 0; j < NS; ++j) {
     const double yj = fmax(y[j], 0.0);
     if (yj <= 0.0) continue;
-    const double ml = yj / (1.0 / fmax(__ldg(m.imw + j), 1e-20));
-    const double tau = pair_mw_time(iv, j, t, pr, m);
+    const double ml = yj / (1.0 / fmax(m.iw[j], 1e-20));
+    const double tau = pair_mw_time(iv, j, t, t13, pr, m);
     conc += ml;
     denom += ml / tau;
   }
@@ -216,9 +209,10 @@ __device__ __forceinline__ double vt_relaxation_source(double density, double t,
   }
   double rm = 0.0;
 #pragma unroll
-  for (int i = 0; i < NS; ++i) rm += fmax(y[i], 0.0) * __ldg(m.gas_const + i);
+  for (int i = 0; i < NS; ++i) rm += fmax(y[i], 0.0) * m.rg[i];
   const double pr = density * rm * fmax(t, 1.0);
   double eq_mix = 0.0, e_mix = 0.0, src = 0.0;
+  const double t13 = rcbrt(t);
   for (int i = 0; i < NS; ++i) {
     if (__ldg(m.theta_v + i) <= 0.0) continue;
     const double yi = fmax(y[i], 0.0);
@@ -229,7 +223,7 @@ __device__ __forceinline__ double vt_relaxation_source(double density, double t,
     eq_mix += yi * e_eq;
     e_mix += yi * e_i;
     if (fabs(d) <= 1e-16) continue;
-    const double tau = species_vt_time<NS>(i, density, t, pr, y, m);
+    const double tau = species_vt_time<NS>(i, density, t, t13, pr, y, m);
     if (tau < 1e29) src += density * yi * d / tau;
   }
   eve_eq = eq_mix;
@@ -249,7 +243,7 @@ __device__ __forceinline__ void temperature_2t(const Zone &z, const Param &p, id
 #pragma unroll
   for (int l = 0; l < NS; ++l) {
     y[l] = z.sv[g + l * sz];
-    gc += y[l] * __ldg(p.mech.gas_const + l);
+    gc += y[l] * p.mech.rg[l];
   }
   const double u = z.bv[g + sz], v = z.bv[g + 2 * sz], w = z.bv[g + 3 * sz];
   const double e = total_energy / density - 0.5 * (u * u + v * v + w * w);
@@ -320,7 +314,7 @@ __device__ __forceinline__ double total_energy_2t(const Zone &z, const Param &p,
 #pragma unroll
   for (int l = 0; l < NS; ++l) {
     y[l] = z.sv[g + l * sz];
-    E += (h[l] - __ldg(p.mech.gas_const + l) * t) * y[l];
+    E += (h[l] - p.mech.rg[l] * t) * y[l];
   }
   E -= mixture_ve_energy<NS>(t, y, p.mech, nullptr);
   E += z.sv[g + NS * sz];
@@ -372,7 +366,7 @@ __device__ __forceinline__ void characteristic_thermo_2t(double t, const double 
   for (int s = 0; s < NS; ++s) {
     double cv_ve;
     const double e_ve = ve_energy(s, te, m, &cv_ve);
-    const double rs = __ldg(m.gas_const + s);
+    const double rs = m.rg[s];
     htr[s] = h[s] - e_ve;
     const double cp_tr = cp[s] - cv_ve;
     e_tr += y[s] * (htr[s] - rs * te);
@@ -389,7 +383,7 @@ __device__ __forceinline__ void characteristic_thermo_2t(double t, const double 
   const double inv_gm1 = 1.0 / fmax(gm1, 1e-12);
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    const double a = (gamma * __ldg(m.gas_const + s) * te - gm1 * htr[s]) / c2;
+    const double a = (gamma * m.rg[s] * te - gm1 * htr[s]) / c2;
     alpha[s] = a;
     ecoef[s] = -a * c2 * inv_gm1;
   }

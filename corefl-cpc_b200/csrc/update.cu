@@ -10,14 +10,14 @@ namespace cb2 {
 
 constexpr int kPtThreads = 128;
 
-template <int NS, bool TT>
-__global__ void __launch_bounds__(kPtThreads) k_stage_update(const __grid_constant__ Zone z, const __grid_constant__ Param p,
-                                                             double dt, int rk, int first) {
+template <int NS, bool TT, bool FIRST>
+__global__ void __launch_bounds__(kPtThreads, NS > 0 ? 5 : 8) k_stage_update(const __grid_constant__ Zone z, const __grid_constant__ Param p,
+                                                             double dt, int rk) {
   chain_begin();
   const int i = blockIdx.x * kPtThreads + threadIdx.x;
   const int j = blockIdx.y, k = blockIdx.z;
   if (i >= z.mx) return;
-  stage_update_point<NS, TT>(z, p, step_dt(p, dt), rk, i, j, k, first != 0);
+  stage_update_point<NS, TT, FIRST>(z, p, step_dt(p, dt), rk, i, j, k);
 }
 
 // VT relaxation of every interior node over dt_scale x the step's dt (apply_vt_relaxation_rk,
@@ -131,12 +131,11 @@ static int launch_update_ns(const Zone &z, const Param &p, double dt, int rk, bo
   const bool tt = p.i_eve >= 0;
   {
     ProfScope prof("stage_update", s);
+    auto go = [&](auto kern) { return launch_chain(kern, grid, kPtThreads, 0, s, z, p, dt, rk); };
     if constexpr (NS > 0) {
-      CB2_TRY(launch_chain(tt ? k_stage_update<NS, true> : k_stage_update<NS, false>, grid, kPtThreads, 0, s, z, p, dt,
-                           rk, (int)first));
-    } else {
-      CB2_TRY(launch_chain(k_stage_update<NS, false>, grid, kPtThreads, 0, s, z, p, dt, rk, (int)first));
+      if (tt) CB2_TRY(go(first ? k_stage_update<NS, true, true> : k_stage_update<NS, true, false>));
     }
+    if (!tt) CB2_TRY(go(first ? k_stage_update<NS, false, true> : k_stage_update<NS, false, false>));
   }
   if constexpr (NS > 0) {
     // the stage's VT relaxation follows its update and precedes limit_flow (src/RK.cuh:198-207)

@@ -15,6 +15,7 @@
 #include "thermo_2t.cuh"
 #include "launch.h"
 #include "stencil8.cuh"
+#include "rcp.cuh"
 
 namespace cb2 {
 
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(kVisThreads) k_visc8_node_flux_mix(Zone z, Par
     cx += dif[s] * fx[s];
     cy += dif[s] * fy[s];
     cz += dif[s] * fz[s];
-    const double iw = __ldg(m.imw + s);
+    const double iw = m.iw[s];
     swx += fx[s] * iw;
     swy += fy[s] * iw;
     swz += fz[s] * iw;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kVisThreads) k_visc8_node_flux_mix(Zone z, Par
     const double gpz = (zeta_x * p_x + zeta_y * p_y + zeta_z * p_z) / pg;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const double co = (mwt * __ldg(m.imw + s) - 1) * yk[s];
+      const double co = (mwt * m.iw[s] - 1) * yk[s];
       fx[s] += co * gpx;
       fy[s] += co * gpy;
       fz[s] += co * gpz;
@@ -351,208 +352,240 @@ __global__ void __launch_bounds__(kVisRow, 16) k_visc8_divergence_f32(Zone z, Pa
 }
 
 // ---- 2nd-order face fluxes ----------------------------------------------------------------
-// Face between node (i,j,k) and its +1 neighbour along DIR.  The compact difference is taken
-// along DIR and the two transverse derivatives are averaged over the two nodes (4-point).
-template <int NS, int DIR, bool TT = false>
-__device__ __forceinline__ void visc2_face(const Zone &z, const Param &p, int i, int j, int k, double *fv) {
-  const Layout &L = z.L;
-  const idx_t sz = L.sz;
-  const idx_t st[3] = {1, L.disp2, L.disp1};
-  const idx_t g = L.at(i, j, k), gn = g + st[DIR];
-  const double *M = z.metric;
-  double mtr[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) mtr[c] = 0.5 * (M[g + c * sz] + M[gn + c * sz]);
-  // derivatives of a field along xi, eta, zeta at the face
-  auto grad = [&](const double *f, double &dxi, double &deta, double &dzeta) {
-    double d[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      if (a == DIR) d[a] = f[gn] - f[g];
-      else d[a] = 0.25 * (f[g + st[a]] - f[g - st[a]] + f[gn + st[a]] - f[gn - st[a]]);
-    }
-    dxi = d[0]; deta = d[1]; dzeta = d[2];
-  };
-  double u_xi, u_eta, u_zeta, v_xi, v_eta, v_zeta, w_xi, w_eta, w_zeta, t_xi, t_eta, t_zeta;
-  grad(z.bv + sz, u_xi, u_eta, u_zeta);
-  grad(z.bv + 2 * sz, v_xi, v_eta, v_zeta);
-  grad(z.bv + 3 * sz, w_xi, w_eta, w_zeta);
-  grad(z.bv + 5 * sz, t_xi, t_eta, t_zeta);
-  const double xi_x = mtr[0], xi_y = mtr[1], xi_z = mtr[2], eta_x = mtr[3], eta_y = mtr[4], eta_z = mtr[5];
-  const double zeta_x = mtr[6], zeta_y = mtr[7], zeta_z = mtr[8];
-  const double u_x = u_xi * xi_x + u_eta * eta_x + u_zeta * zeta_x;
-  const double u_y = u_xi * xi_y + u_eta * eta_y + u_zeta * zeta_y;
-  const double u_z = u_xi * xi_z + u_eta * eta_z + u_zeta * zeta_z;
-  const double v_x = v_xi * xi_x + v_eta * eta_x + v_zeta * zeta_x;
-  const double v_y = v_xi * xi_y + v_eta * eta_y + v_zeta * zeta_y;
-  const double v_z = v_xi * xi_z + v_eta * eta_z + v_zeta * zeta_z;
-  const double w_x = w_xi * xi_x + w_eta * eta_x + w_zeta * zeta_x;
-  const double w_y = w_xi * xi_y + w_eta * eta_y + w_zeta * zeta_y;
-  const double w_z = w_xi * xi_z + w_eta * eta_z + w_zeta * zeta_z;
-  const double mu = 0.5 * (z.mul[g] + z.mul[gn]);
-  const double txx = mu * (4 * u_x - 2 * v_y - 2 * w_z) / 3.0;
-  const double tyy = mu * (4 * v_y - 2 * u_x - 2 * w_z) / 3.0;
-  const double tzz = mu * (4 * w_z - 2 * u_x - 2 * v_y) / 3.0;
-  const double txy = mu * (u_y + v_x), txz = mu * (u_z + w_x), tyz = mu * (v_z + w_y);
-  const double *Md = M + (idx_t)(3 * DIR) * sz;
-  const double jl = z.jac[g], jr = z.jac[gn];
-  const double kxj = 0.5 * (Md[g] * jl + Md[gn] * jr);
-  const double kyj = 0.5 * (Md[g + sz] * jl + Md[gn + sz] * jr);
-  const double kzj = 0.5 * (Md[g + 2 * sz] * jl + Md[gn + 2 * sz] * jr);
-  fv[0] = kxj * txx + kyj * txy + kzj * txz;
-  fv[1] = kxj * txy + kyj * tyy + kzj * tyz;
-  fv[2] = kxj * txz + kyj * tyz + kzj * tzz;
-  const double um = 0.5 * (z.bv[g + sz] + z.bv[gn + sz]);
-  const double vm = 0.5 * (z.bv[g + 2 * sz] + z.bv[gn + 2 * sz]);
-  const double wm = 0.5 * (z.bv[g + 3 * sz] + z.bv[gn + 3 * sz]);
-  const double t_x = t_xi * xi_x + t_eta * eta_x + t_zeta * zeta_x;
-  const double t_y = t_xi * xi_y + t_eta * eta_y + t_zeta * zeta_y;
-  const double t_z = t_xi * xi_z + t_eta * eta_z + t_zeta * zeta_z;
-  double kap;
-  if constexpr (NS == 0) {
-    const double cp = kGammaAir * kRAir / (kGammaAir - 1);
-    kap = mu / p.Pr * cp;
-  } else {
-    kap = 0.5 * (z.kappa[g] + z.kappa[gn]);
-  }
-  fv[3] = um * fv[0] + vm * fv[1] + wm * fv[2] + kap * (kxj * t_x + kyj * t_y + kzj * t_z);
-  if constexpr (NS > 0) {
-    const Mech &m = p.mech;
-    double dif[NS], yk[NS], force[NS];
-    double sum_gy_w = 0, sum_rdy = 0, corr = 0, mwt = 0;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const double *ys = z.sv + s * sz;
-      yk[s] = 0.5 * (ys[g] + ys[gn]);
-      dif[s] = 0.5 * (z.rhoD[g + s * sz] + z.rhoD[gn + s * sz]);
-      double y_xi, y_eta, y_zeta;
-      grad(ys, y_xi, y_eta, y_zeta);
-      const double y_x = y_xi * xi_x + y_eta * eta_x + y_zeta * zeta_x;
-      const double y_y = y_xi * xi_y + y_eta * eta_y + y_zeta * zeta_y;
-      const double y_z = y_xi * xi_z + y_eta * eta_z + y_zeta * zeta_z;
-      const double gdy = kxj * y_x + kyj * y_y + kzj * y_z;
-      force[s] = gdy;
-      corr += dif[s] * gdy;
-      sum_gy_w += gdy * __ldg(m.imw + s);
-      mwt += yk[s] * __ldg(m.imw + s);
-      sum_rdy += dif[s] * yk[s];
-    }
-    mwt = 1.0 / mwt;
-    corr -= mwt * sum_rdy * sum_gy_w;
-    if (p.gradP) {
-      double p_xi, p_eta, p_zeta;
-      grad(z.bv + 4 * sz, p_xi, p_eta, p_zeta);
-      const double p_x = p_xi * xi_x + p_eta * eta_x + p_zeta * zeta_x;
-      const double p_y = p_xi * xi_y + p_eta * eta_y + p_zeta * zeta_y;
-      const double p_z = p_xi * xi_z + p_eta * eta_z + p_zeta * zeta_z;
-      const double gp = (kxj * p_x + kyj * p_y + kzj * p_z) / (0.5 * (z.bv[gn + 4 * sz] + z.bv[g + 4 * sz]));
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        force[s] += (mwt * __ldg(m.imw + s) - 1) * yk[s] * gp;
-        corr += (mwt * __ldg(m.imw + s) - 1) * yk[s] * gp * dif[s];
-      }
-    }
-    double h[NS];
-    const double tm = 0.5 * (z.bv[g + 5 * sz] + z.bv[gn + 5 * sz]);
-    species_h<NS>(tm, m, h);
-    const double tve_m = TT ? 0.5 * (z.tve[g] + z.tve[gn]) : tm;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const double jd = dif[s] * (force[s] - mwt * yk[s] * sum_gy_w) - yk[s] * corr;
-      fv[4 + s] = jd;
-      // two-temperature: the diffusing enthalpy carries e_ve at T_ve
-      // (compute_nonequilibrium_diffusion_enthalpy, src/Thermo.cuh:43-47)
-      const double hd = TT ? h[s] - ve_energy(s, tm, m, nullptr) + ve_energy(s, tve_m, m, nullptr) : h[s];
-      fv[3] += hd * jd;
-    }
-    if constexpr (TT) {
-      // e_ve conduction kappa_ve grad T_ve in the energy flux, and the e_ve flux
-      // (src/ViscousScheme.cu:1024-1039)
-      double v_xi, v_eta, v_zeta;
-      grad(z.tve, v_xi, v_eta, v_zeta);
-      const double v_x = v_xi * xi_x + v_eta * eta_x + v_zeta * zeta_x;
-      const double v_y = v_xi * xi_y + v_eta * eta_y + v_zeta * zeta_y;
-      const double v_z = v_xi * xi_z + v_eta * eta_z + v_zeta * zeta_z;
-      const double kve = 0.5 * (z.kappa_ve[g] + z.kappa_ve[gn]);
-      const double cond_ve = kve * (kxj * v_x + kyj * v_y + kzj * v_z);
-      fv[3] += cond_ve;
-      double ef = cond_ve;
-#pragma unroll
-      for (int s = 0; s < NS; ++s) ef += ve_energy(s, tve_m, m, nullptr) * fv[4 + s];
-      fv[4 + NS] = ef;
-    }
-  }
+// Face between node n and its +1 neighbour along DIR: the compact difference along DIR, and the two
+// transverse derivatives averaged over the two nodes (a 4-point difference).
+//
+// A CTA owns S nodes along DIR for C positions of a transverse index; a thread loads its node once --
+// a field's value and its two transverse central differences, 5 loads, into shared memory -- and
+// forms the face to its right from its own and its neighbour's entries.  Each face loading both of
+// its nodes took 200 loads a thread where this takes 95, and the kernel is bound by the latency of
+// those loads.  The species' gradients are needed along the face normal only, as three numbers
+// G_a = (J grad xi) . grad a times the derivatives along xi, eta, zeta.  Shared memory holds the flow
+// fields and metrics first, then the species, then the fluxes whose difference goes to dq; it is kept
+// to 55 KB a CTA and two CTAs per SM because the loads of a node's neighbours hit in what it leaves
+// of the L1 (three CTAs of 74 KB: 16.9 ms per step on the 192^3 H2/air box; three of 55 KB, 64-byte
+// rows: 12.4; two of 55 KB, 128-byte rows: 8.5; one thread per face, 27 KB: 15.2).
+constexpr int kV2Threads = 256;
+template <int DIR>
+struct V2Tile {
+  static constexpr int C = DIR == 0 ? 8 : 16, S = kV2Threads / C;  // transverse positions, nodes along DIR
+};
+
+template <int NS, bool TT>
+__host__ __device__ constexpr int visc2_slots() {
+  // metrics 9, J, (u, v, w, T, p) x 3, mu, kappa; two temperatures: T_ve x 3, kappa_ve
+  const int flow = 9 + 1 + 5 * 3 + 2 + (TT ? 4 : 0), spec = 3 * NS;
+  return flow > spec ? flow : spec;
 }
 
-constexpr int kV2TI = 16, kV2TS = 16;  // tile of 16 transverse x 16 faces along the direction
-
-// Face fluxes of a tile and their difference: a CTA owns kV2TS faces along DIR (the first
-// one is the left face of the first node) for kV2TI positions of the transverse index.  The
-// thread index runs fastest along i in every direction (along the faces for x, along the
-// transverse index for y/z), so a warp's loads are contiguous.
 template <int NS, int DIR, bool TT = false>
 __device__ __forceinline__ void visc2_tile(const Zone &z, const Param &p) {
   constexpr int NF = 4 + NS + (TT ? 1 : 0);
-  constexpr int kPrev = DIR == 0 ? 1 : kV2TI;  // thread of the previous face along DIR
-  __shared__ double sfv[NF][kV2TI * kV2TS];
+  constexpr int kV2C = V2Tile<DIR>::C, kV2S = V2Tile<DIR>::S;
+  constexpr int kNb = DIR == 0 ? 1 : kV2C;           // thread of the next node along DIR
+  constexpr int A1 = DIR == 0 ? 1 : 0, A2 = DIR == 2 ? 1 : 2;  // the transverse directions
+  constexpr int kM = 0, kJ = 9, kU = 10, kT = 19, kP = 22, kMu = 25, kKap = 26, kTv = 27, kKve = 30;
+  extern __shared__ double v2_smem[];
+  double(*S)[kV2Threads] = reinterpret_cast<double(*)[kV2Threads]>(v2_smem);
   const int tid = threadIdx.x;
-  const int tt = DIR == 0 ? tid / kV2TS : tid % kV2TI, ts = DIR == 0 ? tid % kV2TS : tid / kV2TI;
-  int i, j, k, n;
-  const int s0 = blockIdx.y * (kV2TS - 1);
-  n = s0 - 1 + ts;  // face n + 1/2 along DIR
-  if (DIR == 0) { i = n; j = blockIdx.x * kV2TI + tt; k = blockIdx.z; }
-  else if (DIR == 1) { i = blockIdx.x * kV2TI + tt; j = n; k = blockIdx.z; }
-  else { i = blockIdx.x * kV2TI + tt; j = blockIdx.z; k = n; }
-  const int ext[3] = {z.mx, z.my, z.mz};
-  const int tr = DIR == 0 ? j : i;
-  const int trmax = DIR == 0 ? z.my : z.mx;
-  const bool valid = tr < trmax && n <= ext[DIR] - 1;
-  if (valid) {
-    double fv[NF];
-    visc2_face<NS, DIR, TT>(z, p, i, j, k, fv);
+  const int tt = DIR == 0 ? tid / kV2S : tid % kV2C, ts = DIR == 0 ? tid % kV2S : tid / kV2C;
+  const int n = (int)blockIdx.y * (kV2S - 2) - 1 + ts;  // node along DIR
+  const int tr = blockIdx.x * kV2C + tt;
+  int i, j, k;
+  if (DIR == 0) { i = n; j = tr; k = blockIdx.z; }
+  else if (DIR == 1) { i = tr; j = n; k = blockIdx.z; }
+  else { i = tr; j = blockIdx.z; k = n; }
+  const int ms = DIR == 0 ? z.mx : (DIR == 1 ? z.my : z.mz);
+  const bool node = tr < (DIR == 0 ? z.my : z.mx) && n <= ms;
+  const bool face = node && n <= ms - 1 && ts < kV2S - 1;
+  const Layout &L = z.L;
+  const idx_t sz = L.sz, g = L.at(i, j, k);
+  const idx_t st[3] = {1, L.disp2, L.disp1};
+  auto put = [&](int slot, const double *f) {
+    const double *q = f + g;
+    S[slot][tid] = q[0];
+    S[slot + 1][tid] = q[st[A1]] - q[-st[A1]];
+    S[slot + 2][tid] = q[st[A2]] - q[-st[A2]];
+  };
+  if (node) {
 #pragma unroll
-    for (int c = 0; c < NF; ++c) sfv[c][tid] = fv[c];
+    for (int c = 0; c < 9; ++c) S[kM + c][tid] = z.metric[g + c * sz];
+    S[kJ][tid] = z.jac[g];
+    put(kU, z.bv + sz);
+    put(kU + 3, z.bv + 2 * sz);
+    put(kU + 6, z.bv + 3 * sz);
+    put(kT, z.bv + 5 * sz);
+    if (NS > 0 && p.gradP) put(kP, z.bv + 4 * sz);
+    S[kMu][tid] = z.mul[g];
+    if constexpr (NS > 0) S[kKap][tid] = z.kappa[g];
+    if constexpr (TT) {
+      put(kTv, z.tve);
+      S[kKve][tid] = z.kappa_ve[g];
+    }
   }
   __syncthreads();
-  if (valid && ts >= 1 && n >= 0) {
-    const idx_t g0 = z.L0.at(i, j, k), sz0 = z.L0.sz;
+  const int o = tid + kNb;
+  auto mean = [&](int slot) { return 0.5 * (S[slot][tid] + S[slot][o]); };
+  // derivatives along xi, eta, zeta at the face
+  auto deriv = [&](int slot, double *d) {
+    d[DIR] = S[slot][o] - S[slot][tid];
+    d[A1] = 0.25 * (S[slot + 1][tid] + S[slot + 1][o]);
+    d[A2] = 0.25 * (S[slot + 2][tid] + S[slot + 2][o]);
+  };
+  double fv[4], G[3], tm = 0, tve_m = 0, gp = 0, cond_ve = 0;
+  if (face) {
+    double mtr[9];
 #pragma unroll
-    for (int c = 0; c < NF; ++c) z.dq[g0 + (c + 1) * sz0] += sfv[c][tid] - sfv[c][tid - kPrev];
+    for (int c = 0; c < 9; ++c) mtr[c] = mean(kM + c);
+    const double jl = S[kJ][tid], jr = S[kJ][o];
+    double kj[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) kj[c] = 0.5 * (S[kM + 3 * DIR + c][tid] * jl + S[kM + 3 * DIR + c][o] * jr);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) G[a] = kj[0] * mtr[3 * a] + kj[1] * mtr[3 * a + 1] + kj[2] * mtr[3 * a + 2];
+    double gr[3][3];  // gr[c][x]: d u_c / d x
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      double d[3];
+      deriv(kU + 3 * c, d);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) gr[c][x] = d[0] * mtr[x] + d[1] * mtr[3 + x] + d[2] * mtr[6 + x];
+    }
+    const double mu = mean(kMu);
+    const double txx = mu * (4 * gr[0][0] - 2 * gr[1][1] - 2 * gr[2][2]) * (1.0 / 3.0);
+    const double tyy = mu * (4 * gr[1][1] - 2 * gr[0][0] - 2 * gr[2][2]) * (1.0 / 3.0);
+    const double tzz = mu * (4 * gr[2][2] - 2 * gr[0][0] - 2 * gr[1][1]) * (1.0 / 3.0);
+    const double txy = mu * (gr[0][1] + gr[1][0]), txz = mu * (gr[0][2] + gr[2][0]), tyz = mu * (gr[1][2] + gr[2][1]);
+    fv[0] = kj[0] * txx + kj[1] * txy + kj[2] * txz;
+    fv[1] = kj[0] * txy + kj[1] * tyy + kj[2] * tyz;
+    fv[2] = kj[0] * txz + kj[1] * tyz + kj[2] * tzz;
+    double kap;
+    if constexpr (NS == 0) kap = mu / p.Pr * (kGammaAir * kRAir / (kGammaAir - 1));
+    else kap = mean(kKap);
+    double d[3];
+    deriv(kT, d);
+    fv[3] = mean(kU) * fv[0] + mean(kU + 3) * fv[1] + mean(kU + 6) * fv[2] + kap * (G[0] * d[0] + G[1] * d[1] + G[2] * d[2]);
+    if constexpr (NS > 0) {
+      tm = mean(kT);
+      if (p.gradP) {
+        deriv(kP, d);
+        gp = (G[0] * d[0] + G[1] * d[1] + G[2] * d[2]) / mean(kP);
+      }
+    }
+    if constexpr (TT) {
+      // e_ve conduction kappa_ve grad T_ve in the energy flux and the e_ve flux
+      // (src/ViscousScheme.cu:1024-1039)
+      tve_m = mean(kTv);
+      deriv(kTv, d);
+      cond_ve = mean(kKve) * (G[0] * d[0] + G[1] * d[1] + G[2] * d[2]);
+    }
+  }
+  __syncthreads();
+  double js[NS > 0 ? NS : 1], ef = 0;
+  if constexpr (NS > 0) {
+    if (node) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) put(3 * s, z.sv + s * sz);
+    }
+    __syncthreads();
+    if (face) {
+      const Mech &m = p.mech;
+      auto grad = [&](int s) {
+        double d[3];
+        deriv(3 * s, d);
+        return G[0] * d[0] + G[1] * d[1] + G[2] * d[2];
+      };
+      const idx_t gn = g + st[DIR];
+      auto rho_d = [&](int s) { return 0.5 * (z.rhoD[g + s * sz] + z.rhoD[gn + s * sz]); };
+      double sum_gy_w = 0, sum_rdy = 0, corr = 0, mwt = 0;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const double yk = mean(3 * s), dif = rho_d(s), gdy = grad(s), w = m.iw[s];
+        js[s] = gdy;
+        corr += dif * gdy;
+        sum_gy_w += gdy * w;
+        mwt += yk * w;
+        sum_rdy += dif * yk;
+      }
+      mwt = recip(mwt);
+      corr -= mwt * sum_rdy * sum_gy_w;
+      if (p.gradP) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          const double f = (mwt * m.iw[s] - 1) * mean(3 * s) * gp;
+          js[s] += f;
+          corr += f * rho_d(s);
+        }
+      }
+      double h[NS];
+      species_h<NS>(tm, m, h);
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const double yk = mean(3 * s);
+        js[s] = rho_d(s) * (js[s] - mwt * yk * sum_gy_w) - yk * corr;
+        if constexpr (TT) {
+          // the diffusing enthalpy carries e_ve at T_ve (compute_nonequilibrium_diffusion_enthalpy,
+          // src/Thermo.cuh:43-47)
+          const double ev = ve_energy(s, tve_m, m, nullptr);
+          fv[3] += (h[s] - ve_energy(s, tm, m, nullptr) + ev) * js[s];
+          ef += ev * js[s];
+        } else {
+          fv[3] += h[s] * js[s];
+        }
+      }
+      if constexpr (TT) {
+        fv[3] += cond_ve;
+        ef += cond_ve;
+      }
+    }
+    __syncthreads();
+  }
+  if (face) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) S[c][tid] = fv[c];
+    if constexpr (NS > 0) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) S[4 + s][tid] = js[s];
+    }
+    if constexpr (TT) S[4 + NS][tid] = ef;
+  }
+  const bool upd = face && ts >= 1 && n >= 0;
+  const idx_t g0 = z.L0.at(i, j, k), sz0 = z.L0.sz;
+  double old[NF];
+  if (upd) {
+#pragma unroll
+    for (int c = 0; c < NF; ++c) old[c] = z.dq[g0 + (c + 1) * sz0];
+  }
+  __syncthreads();
+  if (upd) {
+#pragma unroll
+    for (int c = 0; c < NF; ++c) z.dq[g0 + (c + 1) * sz0] = old[c] + (S[c][tid] - S[c][tid - kNb]);
   }
 }
 
-template <int NS, int DIR>
-__global__ void __launch_bounds__(kV2TI *kV2TS) k_visc2(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
+template <int NS, int DIR, bool TT>
+__global__ void __launch_bounds__(kV2Threads, 2)
+k_visc2(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
   chain_begin();
-  visc2_tile<NS, DIR, false>(z, p);
-}
-
-// Two temperatures: held to 128 registers (two CTAs per SM; 170-180 unbounded).
-template <int NS, int DIR>
-__global__ void __launch_bounds__(kV2TI *kV2TS, 2) k_visc2_2t(Zone z, Param p) {
-  visc2_tile<NS, DIR, true>(z, p);
+  visc2_tile<NS, DIR, TT>(z, p);
 }
 
 template <int NS, bool TT = false>
 static int launch_visc2_ns(const Zone &z, const Param &p, cudaStream_t s, int &nl) {
   const int ndir = z.mz > 1 ? 3 : 2;
+  const size_t smem = sizeof(double) * visc2_slots<NS, TT>() * kV2Threads;
   for (int d = 0; d < ndir; ++d) {
     const int ext[3] = {z.mx, z.my, z.mz};
     const int tr = d == 0 ? z.my : z.mx;
     const int other = d == 2 ? z.my : z.mz;
-    dim3 grid((tr + kV2TI - 1) / kV2TI, (ext[d] + kV2TS - 2) / (kV2TS - 1), other);
+    const int C = d == 0 ? V2Tile<0>::C : V2Tile<1>::C, S = kV2Threads / C;
+    dim3 grid((tr + C - 1) / C, (ext[d] + S - 3) / (S - 2), other);
     static const char *names[3] = {"visc2_x", "visc2_y", "visc2_z"};
     ProfScope prof(names[d], s);
-    if constexpr (TT) {
-      if (d == 0) k_visc2_2t<NS, 0><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
-      else if (d == 1) k_visc2_2t<NS, 1><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
-      else k_visc2_2t<NS, 2><<<grid, kV2TI * kV2TS, 0, s>>>(z, p);
-    } else {
-      CB2_TRY(launch_chain(d == 0 ? k_visc2<NS, 0> : (d == 1 ? k_visc2<NS, 1> : k_visc2<NS, 2>), grid, kV2TI * kV2TS, 0,
-                           s, z, p));
-    }
+    auto kern = d == 0 ? k_visc2<NS, 0, TT> : (d == 1 ? k_visc2<NS, 1, TT> : k_visc2<NS, 2, TT>);
+    CB2_TRY(prepare_smem(kern, smem));
+    CB2_TRY(launch_chain(kern, grid, kV2Threads, smem, s, z, p));
     ++nl;
-    CB2_TRY(check_launch());
   }
   return CB2_OK;
 }
