@@ -61,7 +61,7 @@ __device__ __forceinline__ void char_flux(const double *__restrict__ sQ, const d
 #pragma unroll
     for (int s = 0; s < NSC; ++s) svm[s] = rlc * Qv(5 + s, 0) + rrc * Qv(5 + s, 1);
 #pragma unroll
-    for (int s = 0; s < NS; ++s) rmix += svm[s] * __ldg(mech.gas_const + s);
+    for (int s = 0; s < NS; ++s) rmix += svm[s] * mech.rg[s];
     const double t_roe = (rlc * Fv(4, 0) + rrc * Fv(4, 1)) / fmax(rmix, 1e-12);
     double gamma;
     if constexpr (TT) characteristic_thermo_2t<NS>(t_roe, svm, mech, gamma, cm, alpha, ecoef);

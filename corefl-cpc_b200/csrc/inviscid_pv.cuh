@@ -127,7 +127,7 @@ __device__ __forceinline__ void state_energy(T *pv, const Mech &m) {
 #pragma unroll
     for (int s = 0; s < NSP; ++s) {
       y[s] = double(pv[5 + s]);
-      r += y[s] * __ldg(m.gas_const + s);
+      r += y[s] * m.rg[s];
     }
     const double t = double(pv[4]) / fmax(double(pv[0]) * r, 1e-12);
     double gam, c, etr;
@@ -144,7 +144,7 @@ __device__ __forceinline__ void state_energy(T *pv, const Mech &m) {
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       y[s] = float(pv[5 + s]);
-      r += y[s] * float(__ldg(m.gas_const + s));
+      r += y[s] * float(m.rg[s]);
     }
     const float t = float(pv[4]) / fmaxf(float(pv[0]) * r, 1e-12f);
     float gam, c, etr;
@@ -156,7 +156,7 @@ __device__ __forceinline__ void state_energy(T *pv, const Mech &m) {
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       y[s] = double(pv[5 + s]);
-      r += y[s] * __ldg(m.gas_const + s);
+      r += y[s] * m.rg[s];
     }
     const double t = double(pv[4]) / fmax(double(pv[0]) * r, 1e-12);
     double gam, c, etr;
@@ -270,7 +270,7 @@ __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *ml, cons
 #pragma unroll
     for (int s = 0; s < NSP; ++s) {
       svm[s] = double(rlc * pl[5 + s] + rrc * pr[5 + s]);
-      r += svm[s] * __ldg(mech.gas_const + s);
+      r += svm[s] * mech.rg[s];
     }
     const double t = double(rlc * mul_rn(pl[4], idl) + rrc * mul_rn(pr[4], idr)) / fmax(r, 1e-12);
     double gam, c64;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *ml, cons
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       svm[s] = float(rlc * pl[5 + s] + rrc * pr[5 + s]);
-      r += svm[s] * float(__ldg(mech.gas_const + s));
+      r += svm[s] * float(mech.rg[s]);
     }
     const float t = float(rlc * mul_rn(pl[4], idl) + rrc * mul_rn(pr[4], idr)) / fmaxf(r, 1e-12f);
     float gam, c32;
@@ -293,7 +293,7 @@ __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *ml, cons
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       svm[s] = double(rlc * pl[5 + s] + rrc * pr[5 + s]);
-      r += svm[s] * __ldg(mech.gas_const + s);
+      r += svm[s] * mech.rg[s];
     }
     const double t = double(rlc * mul_rn(pl[4], idl) + rrc * mul_rn(pr[4], idr)) / fmax(r, 1e-12);
     double gam, c64;
@@ -397,7 +397,7 @@ __device__ __forceinline__ void roe_flux(const T *pl, const T *pr, const T *ml, 
     for (int s = 0; s < NS; ++s) {
       svm[s] = (dl * pl[5 + s] + dr * pr[5 + s]) * idn;
       sv64[s] = double(svm[s]);
-      r += sv64[s] * __ldg(p.mech.gas_const + s);
+      r += sv64[s] * p.mech.rg[s];
     }
     const double t = double((dl * (pl[4] / pl[0]) + dr * (pr[4] / pr[0])) * idn) / fmax(r, 1e-12);
     double g64, c64, a64[NS], e64[NS];
@@ -659,12 +659,19 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
 #pragma unroll
     for (int v = 0; v < NV; ++v) sF[v * kSweepThreads + tid] = fc[v];
   }
+  const idx_t gd = z.L0.at(i, j, k);
+  const idx_t sz0 = z.L0.sz;
+  // the residual to add to, read under the barrier
+  const bool assign = !VF && DIR == 0 && p.assign_x;
+  double old[VF ? 1 : NV];
+  if (!VF && upd && !assign) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) old[v] = z.dq[gd + v * sz0];
+  }
   __syncthreads();
 
   if (upd) {
     const int tprev = tid - st;
-    const idx_t gd = z.L0.at(i, j, k);
-    const idx_t sz0 = z.L0.sz;
     if constexpr (VF) {
       // physical-boundary closures of the stencil along this direction
       bool bl, br;
@@ -692,13 +699,13 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
         if (first) z.dq[gd + v * sz0] = vis - inv;
         else z.dq[gd + v * sz0] = (z.dq[gd + v * sz0] + vis) - inv;
       }
-    } else if (DIR == 0 && p.assign_x) {
+    } else if (assign) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) z.dq[gd + v * sz0] = -double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v)
-        z.dq[gd + v * sz0] -= double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
+        z.dq[gd + v * sz0] = old[v] - double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
     }
   }
   __syncthreads();
@@ -782,7 +789,12 @@ static int launch_pv_yz_ni(const Zone &z, const Param &p, cudaStream_t s) {
     if (ni == 4) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 4, VF>(z, p, s);
     if (ni == 16) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 16, VF>(z, p, s);
   }
-  return launch_pv_yz<T, NS, DIR, REC, SOLVER, kNI, VF, TT>(z, p, s);
+  // mixtures: 16 columns (128-byte rows) although 2 of 16 nodes are overlap instead of 2 of 32; their
+  // 18 arrays per node make the loads count (192^3 H2/air: y, z 6.5 -> 6.3 ms per step each; with the
+  // gas constants as kernel parameters 3.85: as global loads they missed an L1 that the tiles' shared
+  // memory leaves 20 KB)
+  if constexpr (NS > 0) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 16, VF, TT>(z, p, s);
+  else return launch_pv_yz<T, NS, DIR, REC, SOLVER, kNI, VF, TT>(z, p, s);
 }
 
 template <typename T, int NS, int REC, int SOLVER, bool VF, bool TT = false>
