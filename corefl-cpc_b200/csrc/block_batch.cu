@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_head(const BlockCase *c
 template <int DIR, int REC, int SOLVER, int NI>
 __global__ void __launch_bounds__(kSweepThreads, 4) k_batch_sweep(const BlockCase *cases, BlockState *state, const int *owner,
                                                                const int *first, const __grid_constant__ Param p0) {
+  constexpr int TB = kSweepThreads;  // small blocks: 32 nodes along y, z at the default width
   extern __shared__ __align__(16) unsigned char bb_smem[];
   chain_begin();
   const BatchItem it = batch_item(owner, first);
@@ -118,13 +119,13 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_batch_sweep(const BlockCas
   const Param p = block_param(p0, z, &st);
   if constexpr (DIR == 0) {
     const idx_t run = (idx_t)z.L.my * z.L.disp2;
-    const int ntx = (int)((run + (kSweepThreads - 2) - 1) / (kSweepThreads - 2));
-    pv_tile<double, 0, 0, REC, SOLVER>(z, p, run, it.t % ntx, 0, it.t / ntx, bb_smem);
+    const int ntx = (int)((run + (TB - 2) - 1) / (TB - 2));
+    pv_tile<double, 0, 0, REC, SOLVER, kNI, false, false, TB>(z, p, run, it.t % ntx, 0, it.t / ntx, bb_smem);
   } else {
-    constexpr int NSW = kSweepThreads / NI;
+    constexpr int NSW = TB / NI;
     const int nit = (z.mx + NI - 1) / NI, ms = DIR == 1 ? z.my : z.mz, nst = (ms + NSW - 3) / (NSW - 2);
     const int bx = it.t % nit, r = it.t / nit;
-    pv_tile<double, 0, DIR, REC, SOLVER, NI>(z, p, 0, bx, r % nst, r / nst, bb_smem);
+    pv_tile<double, 0, DIR, REC, SOLVER, NI, false, false, TB>(z, p, 0, bx, r % nst, r / nst, bb_smem);
   }
 }
 
@@ -202,7 +203,7 @@ template <int DIR, int REC, int SOLVER, int NI>
 int sweep(const Batch &t, const Param &p) {
   const int ph = DIR == 0 ? kTilesX : (DIR == 1 ? kTilesY : kTilesZ);
   if (!t.count(ph)) return CB2_OK;
-  const size_t smem = pv_tile_smem<double, 0, REC, SOLVER>(DIR, NI);
+  const size_t smem = pv_tile_smem<double, 0, REC, SOLVER, false, kSweepThreads>(DIR, NI);
   auto kern = k_batch_sweep<DIR, REC, SOLVER, NI>;
   CB2_TRY(prepare_smem(kern, smem));
   ++t.nl;

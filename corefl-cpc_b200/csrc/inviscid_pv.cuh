@@ -494,19 +494,29 @@ __device__ __forceinline__ void lax_friedrichs_air(const T *pl, const T *pr, con
 template <int REC>
 __host__ __device__ constexpr int pv_half_width() { return REC == 1 ? 0 : (REC <= 3 ? 1 : REC / 2); }
 
+// Threads (nodes) of a tile.  FP64 air with AUSM+: 512, so that a y/z tile has 128-byte rows (16 columns) and
+// still 30 of its 32 nodes along the sweep are its own (257^3: 3.64 -> 3.30 ms per step and direction;
+// with 256 threads 16 columns leave 14 of 16).  AUSM+ fits the 64 registers a thread that two such
+// CTAs per SM allow; the other solvers and the mixtures do not, and the FP32 tiles are faster at 256
+// (161x129x97, y: 129 against 159 us).
+template <typename T, int NS, int SOLVER>
+__host__ __device__ constexpr int pv_threads() {
+  return sizeof(T) == 8 && NS == 0 && SOLVER == CB2_INV_AUSMP ? 512 : kSweepThreads;
+}
+
 // Shared-memory bytes of one sweep tile.
 // VF: the tile also holds the node flux comps 1-4 of the 8th-order viscous terms along the sweep.
-template <typename T, int NS, int REC, int SOLVER, bool VF = false>
+template <typename T, int NS, int REC, int SOLVER, bool VF = false, int TB = pv_threads<T, NS, SOLVER>()>
 __host__ __device__ constexpr size_t pv_tile_smem(int dir, int ni = kNI) {
   return sizeof(T) * ((size_t)(5 + NS + 4 + (SOLVER == CB2_INV_ROE ? 1 : 0) + (VF ? 4 : 0)) *
-                          (dir == 0 ? (kSweepThreads + 2 * pv_half_width<REC>())
-                                    : ni * (kSweepThreads / ni + 2 * pv_half_width<REC>())) +
-                      (size_t)(2 * (5 + NS) + 2) * kSweepThreads);
+                          (dir == 0 ? (TB + 2 * pv_half_width<REC>())
+                                    : ni * (TB / ni + 2 * pv_half_width<REC>())) +
+                      (size_t)(2 * (5 + NS) + 2) * TB);
 }
 
 // One tile of the sweep: tile (bx, by, bz) of the grid that node_sweep_grid describes, run by a
-// CTA of kSweepThreads threads; sN holds the node data [NSLOT][NN], sR the right states
-// [NV+2][kSweepThreads], sF the interface fluxes [NV][kSweepThreads].  The tile ends with the
+// CTA of TB = pv_threads threads; sN holds the node data [NSLOT][NN], sR the right states
+// [NV+2][TB], sF the interface fluxes [NV][TB].  The tile ends with the
 // whole CTA in step, so a CTA may run several tiles back to back.
 // VF (air, WENO7): the 8th-order viscous divergence along this direction is taken here too
 // (compute_viscous_flux_derivative<8>, src/ViscousScheme.cu:790-834, one direction of it): the
@@ -514,15 +524,16 @@ __host__ __device__ constexpr size_t pv_tile_smem(int dir, int ni = kNI) {
 // periodic exchange), and every updated node adds J d8(F) before subtracting its inviscid flux
 // difference.  The WENO7 tile's halo of 3 nodes plus the neighbour node covers the +-4 stencil
 // of every updated node.
-template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false, bool TT = false>
+template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false, bool TT = false,
+          int TB = pv_threads<T, NS, SOLVER>()>
 __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_t run, int bx, int by, int bz,
                                              T *sN, T *sR, T *sF) {
   static_assert(!VF || (REC == 7 && NS == 0 && sizeof(T) == 4),
                 "the fused viscous divergence is built for the mixed form's WENO7 air tile");
   constexpr int NV = 5 + NS;
   constexpr int RH = pv_half_width<REC>();
-  constexpr int NSW = kSweepThreads / NI;  // y/z tile: nodes along the sweep
-  constexpr int NN = DIR == 0 ? (kSweepThreads + 2 * RH) : NI * (NSW + 2 * RH);
+  constexpr int NSW = TB / NI;  // y/z tile: nodes along the sweep
+  constexpr int NN = DIR == 0 ? (TB + 2 * RH) : NI * (NSW + 2 * RH);
   const int tid = threadIdx.x;
   const int g = z.ngg;
   const Layout &L = z.L;
@@ -584,11 +595,11 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
     // holds far fewer than 2^31 nodes, and 32-bit division is several times cheaper
     k = bz;
     const int d2 = (int)L.disp2;
-    const int q0 = bx * (kSweepThreads - 2) - 1;
+    const int q0 = bx * (TB - 2) - 1;
     const idx_t base = (idx_t)k * L.disp1 + L.dispt - g;
     const int qlo = q0 - RH;
     const int qmin = -L.gj * d2, qmax = (L.my + L.gj) * d2;
-    for (int s = tid; s < NN; s += kSweepThreads) {
+    for (int s = tid; s < NN; s += TB) {
       const int q = qlo + s;
       if (q >= qmin && q < qmax) {
         const int jj = q >= 0 ? q / d2 : -((-q + d2 - 1) / d2);
@@ -626,7 +637,7 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
     st = NI;
   }
   const bool rec = inside && n >= -1 && n <= ms;
-  const bool face = rec && n <= ms - 1 && tpos < (DIR == 0 ? kSweepThreads : NSW) - 1;
+  const bool face = rec && n <= ms - 1 && tpos < (DIR == 0 ? TB : NSW) - 1;
   const bool upd = face && n >= 0 && tpos >= 1;
   copy_async_wait();
   __syncthreads();
@@ -638,7 +649,7 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
     state_energy<NS, T, TT>(pl, p.mech);
     state_energy<NS, T, TT>(pr, p.mech);
 #pragma unroll
-    for (int v = 0; v < NV + 2; ++v) sR[v * kSweepThreads + tid] = pr[v];
+    for (int v = 0; v < NV + 2; ++v) sR[v * TB + tid] = pr[v];
   }
   __syncthreads();
 
@@ -646,7 +657,7 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
     const int tn = tid + st;  // the thread of node n+1 (st is 1 or NI, as the thread layout)
     T pr[NV + 2];
 #pragma unroll
-    for (int v = 0; v < NV + 2; ++v) pr[v] = sR[v * kSweepThreads + tn];
+    for (int v = 0; v < NV + 2; ++v) pr[v] = sR[v * TB + tn];
     const T ml[3] = {sN[NV * NN + c], sN[(NV + 1) * NN + c], sN[(NV + 2) * NN + c]};
     const T mr[3] = {sN[NV * NN + c + st], sN[(NV + 1) * NN + c + st], sN[(NV + 2) * NN + c + st]};
     const T jl = sN[(NV + 3) * NN + c], jr = sN[(NV + 3) * NN + c + st];
@@ -657,7 +668,7 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
       roe_flux<NS>(pl, pr, ml, mr, jl, jr, sN[(NV + 4) * NN + c], sN[(NV + 4) * NN + c + st], p, fc);
     else lax_friedrichs_air(pl, pr, ml, mr, jl, jr, fc);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) sF[v * kSweepThreads + tid] = fc[v];
+    for (int v = 0; v < NV; ++v) sF[v * TB + tid] = fc[v];
   }
   const idx_t gd = z.L0.at(i, j, k);
   const idx_t sz0 = z.L0.sz;
@@ -694,39 +705,41 @@ __device__ __forceinline__ void pv_tile_body(const Zone &z, const Param &p, idx_
       for (int v = 1; v < 5; ++v) {
         const T *Fv = sN + (NSB + v - 1) * NN + c;
         const T dv = d8<T>([&](int m) { return Fv[m * st]; }, n, ms, bl, br);
-        const double inv = double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
+        const double inv = double(sF[v * TB + tid] - sF[v * TB + tprev]);
         const double vis = double(dv * jac);
         if (first) z.dq[gd + v * sz0] = vis - inv;
         else z.dq[gd + v * sz0] = (z.dq[gd + v * sz0] + vis) - inv;
       }
     } else if (assign) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) z.dq[gd + v * sz0] = -double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
+      for (int v = 0; v < NV; ++v) z.dq[gd + v * sz0] = -double(sF[v * TB + tid] - sF[v * TB + tprev]);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v)
-        z.dq[gd + v * sz0] = old[v] - double(sF[v * kSweepThreads + tid] - sF[v * kSweepThreads + tprev]);
+        z.dq[gd + v * sz0] = old[v] - double(sF[v * TB + tid] - sF[v * TB + tprev]);
     }
   }
   __syncthreads();
 }
 
 // One whole tile with pv_tile_smem bytes at pv_smem.
-template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false, bool TT = false>
+template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false, bool TT = false,
+          int TB = pv_threads<T, NS, SOLVER>()>
 __device__ __forceinline__ void pv_tile(const Zone &z, const Param &p, idx_t run, int bx, int by, int bz,
                                         unsigned char *pv_smem) {
   constexpr int NV = 5 + NS;
   constexpr int RH = pv_half_width<REC>();
-  constexpr int NN = DIR == 0 ? (kSweepThreads + 2 * RH) : NI * (kSweepThreads / NI + 2 * RH);
+  constexpr int NN = DIR == 0 ? (TB + 2 * RH) : NI * (TB / NI + 2 * RH);
   constexpr int NSLOT = NV + 4 + (SOLVER == CB2_INV_ROE ? 1 : 0) + (VF ? 4 : 0);
   T *sN = reinterpret_cast<T *>(pv_smem);
   T *sR = sN + NSLOT * NN;
-  T *sF = sR + (NV + 2) * kSweepThreads;
-  pv_tile_body<T, NS, DIR, REC, SOLVER, NI, VF, TT>(z, p, run, bx, by, bz, sN, sR, sF);
+  T *sF = sR + (NV + 2) * TB;
+  pv_tile_body<T, NS, DIR, REC, SOLVER, NI, VF, TT, TB>(z, p, run, bx, by, bz, sN, sR, sF);
 }
 
 template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false, bool TT = false>
-__global__ void __launch_bounds__(kSweepThreads) k_inviscid_pv(const __grid_constant__ Zone z, const __grid_constant__ Param p, idx_t run) {
+__global__ void __launch_bounds__((pv_threads<T, NS, SOLVER>()))
+k_inviscid_pv(const __grid_constant__ Zone z, const __grid_constant__ Param p, idx_t run) {
   chain_begin();
   extern __shared__ __align__(16) unsigned char pv_smem[];
   pv_tile<T, NS, DIR, REC, SOLVER, NI, VF, TT>(z, p, run, blockIdx.x, blockIdx.y, blockIdx.z, pv_smem);
@@ -735,7 +748,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_inviscid_pv(const __grid_cons
 // The mixture sweeps, held to 128 registers (two CTAs per SM): they would otherwise take up to 170
 // and run one CTA per SM (192^3 H2/air box, WENO5 + HLLC, FP64: 21.6 -> 18.1 ms per step).
 template <typename T, int NS, int DIR, int REC, int SOLVER, int NI = kNI, bool VF = false>
-__global__ void __launch_bounds__(kSweepThreads, 2) k_inviscid_pv_mb2(const __grid_constant__ Zone z, const __grid_constant__ Param p, idx_t run) {
+__global__ void __launch_bounds__(kSweepThreads, 2)
+k_inviscid_pv_mb2(const __grid_constant__ Zone z, const __grid_constant__ Param p, idx_t run) {
   chain_begin();
   extern __shared__ __align__(16) unsigned char pv_smem[];
   pv_tile<T, NS, DIR, REC, SOLVER, NI, VF>(z, p, run, blockIdx.x, blockIdx.y, blockIdx.z, pv_smem);
@@ -773,11 +787,11 @@ __global__ void k_entropy_fix_delta(Zone z, Param p) {
 template <typename T, int NS, int DIR, int REC, int SOLVER, int NI, bool VF = false, bool TT = false>
 static int launch_pv_yz(const Zone &z, const Param &p, cudaStream_t s) {
   SweepGeom geo;
-  const dim3 grid = node_sweep_grid(DIR, z.L, geo, NI);
+  const dim3 grid = node_sweep_grid(DIR, z.L, geo, NI, pv_threads<T, NS, SOLVER>());
   const size_t smem = pv_tile_smem<T, NS, REC, SOLVER, VF>(DIR, NI);
   auto kern = pv_kernel<T, NS, DIR, REC, SOLVER, NI, VF, TT>();
   CB2_TRY(prepare_smem(kern, smem));
-  return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, (idx_t)0);
+  return launch_chain(kern, grid, pv_threads<T, NS, SOLVER>(), smem, s, z, p, (idx_t)0);
 }
 
 // y/z sweep with the block's tile width: the autotuned widths exist for the WENO5/7 air sweeps
@@ -785,7 +799,8 @@ static int launch_pv_yz(const Zone &z, const Param &p, cudaStream_t s) {
 template <typename T, int NS, int DIR, int REC, int SOLVER, bool VF = false, bool TT = false>
 static int launch_pv_yz_ni(const Zone &z, const Param &p, cudaStream_t s) {
   if constexpr ((REC == 5 || REC == 7) && NS == 0) {
-    const int ni = z.tile_ni[DIR];
+    // the tuned width, or the one that fits the block best
+    const int ni = z.tile_ni[DIR] || sizeof(T) == 4 ? z.tile_ni[DIR] : fewest_slots_ni(z.L, DIR, pv_threads<T, NS, SOLVER>());
     if (ni == 4) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 4, VF>(z, p, s);
     if (ni == 16) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 16, VF>(z, p, s);
   }
@@ -801,11 +816,11 @@ template <typename T, int NS, int REC, int SOLVER, bool VF, bool TT = false>
 static int launch_pv_dir(int d, const Zone &z, const Param &p, cudaStream_t s) {
   if (d == 0) {
     SweepGeom geo;
-    const dim3 grid = node_sweep_grid(0, z.L, geo);
+    const dim3 grid = node_sweep_grid(0, z.L, geo, kNI, pv_threads<T, NS, SOLVER>());
     const size_t smem = pv_tile_smem<T, NS, REC, SOLVER, VF>(0);
     auto kern = pv_kernel<T, NS, 0, REC, SOLVER, kNI, VF, TT>();
     CB2_TRY(prepare_smem(kern, smem));
-    return launch_chain(kern, grid, kSweepThreads, smem, s, z, p, geo.run);
+    return launch_chain(kern, grid, pv_threads<T, NS, SOLVER>(), smem, s, z, p, geo.run);
   }
   if (d == 1) return launch_pv_yz_ni<T, NS, 1, REC, SOLVER, VF, TT>(z, p, s);
   return launch_pv_yz_ni<T, NS, 2, REC, SOLVER, VF, TT>(z, p, s);

@@ -18,11 +18,11 @@ constexpr int kPropTabCtas = 4;  // CTAs per SM of the FP64 transport kernels: 1
 template <int NS, bool F32T = false>
 __global__ void __launch_bounds__(kPropThreads, 6) k_properties(const __grid_constant__ Zone z, const __grid_constant__ Param p) {
   chain_begin();
-  const int g_ = z.ngg;
-  const int i = blockIdx.x * kPropThreads + threadIdx.x - g_;
-  const int j = blockIdx.y - g_, k = blockIdx.z - g_;
-  if (i >= z.mx + g_) return;
-  properties_point<NS, F32T>(z, p, i, j, k);
+  const int g_ = z.ngg, px = z.mx + 2 * g_;
+  const int q = blockIdx.x * kPropThreads + threadIdx.x;
+  if (q >= px * (z.my + 2 * g_)) return;
+  const int j = q / px, i = q - j * px;
+  properties_point<NS, F32T>(z, p, i - g_, j - g_, (int)blockIdx.y - g_);
 }
 
 // FP64 transport on the repacked mechanism (transport_tab.cuh).  A tile runs along the padded k
@@ -122,7 +122,7 @@ int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_laun
   const int g = z.ngg;
   const bool planar = z.mz == 1 && p.dim == 2;
   const bool mixed = p.precision == CB2_PREC_MIXED;  // transport in FP32
-  dim3 grid((z.mx + 2 * g + kPropThreads - 1) / kPropThreads, z.my + 2 * g, planar ? 1 : z.mz + 2 * g);
+  const dim3 grid((z.mx + 2 * g + kPropThreads - 1) / kPropThreads, z.my + 2 * g);  // 2-D blocks
   ++n_launch;
   ProfScope prof("properties", s);
   const TransTabs *tab = mixed ? nullptr : p.mech.trans_tabs;
@@ -130,15 +130,19 @@ int launch_properties(const Zone &z, const Param &p, cudaStream_t s, int &n_laun
   if (tab && p.n_spec == 5) return launch_properties_tab<5>(z, p, tab->t5, planar, s);
   // nothing changes for air of constant viscosity without a Mach array
   if (p.n_spec == 0 && p.mu_constant > 0 && !z.mach) { --n_launch; return CB2_OK; }
-  auto go = [&](auto kern) { return launch_chain(kern, grid, kPropThreads, 0, s, z, p); };
+  const int plane = (z.mx + 2 * g) * (z.my + 2 * g);
+  const dim3 pgrid((unsigned)((plane + kPropThreads - 1) / kPropThreads), (unsigned)(z.mz + 2 * g));
+  auto go = [&](auto flat, auto all) {
+    return planar ? launch_chain(flat, grid, kPropThreads, 0, s, z, p) : launch_chain(all, pgrid, kPropThreads, 0, s, z, p);
+  };
   switch (p.n_spec) {
-    case 0: return go(planar ? k_properties_planar<0> : k_properties<0>);
+    case 0: return go(k_properties_planar<0>, k_properties<0>);
     case 5:
-      if (mixed) return go(planar ? k_properties_planar<5, true> : k_properties<5, true>);
-      return go(planar ? k_properties_planar<5> : k_properties<5>);
+      if (mixed) return go(k_properties_planar<5, true>, k_properties<5, true>);
+      return go(k_properties_planar<5>, k_properties<5>);
     case 9:
-      if (mixed) return go(planar ? k_properties_planar<9, true> : k_properties<9, true>);
-      return go(planar ? k_properties_planar<9> : k_properties<9>);
+      if (mixed) return go(k_properties_planar<9, true>, k_properties<9, true>);
+      return go(k_properties_planar<9>, k_properties<9>);
     default: return CB2_ERR_UNSUPPORTED;
   }
 }

@@ -48,14 +48,30 @@ __host__ __device__ __forceinline__ int node_sweep_nodes(int dir, int r) {
 // it per block and direction among kTileNI.
 constexpr int kTileNI[3] = {4, 8, 16};
 
-inline dim3 node_sweep_grid(int dir, const Layout &L, SweepGeom &g, int ni = kNI) {
+// The y/z tile width that spends the fewest node slots on a block (whole tiles of ni columns by
+// threads / ni nodes, two of them overlap), the wider rows on a tie.
+inline int fewest_slots_ni(const Layout &L, int dir, int threads) {
+  const long long ms = dir == 1 ? L.my : L.mz;
+  int best = kTileNI[0];
+  long long least = -1;
+  for (int ni : kTileNI) {
+    const long long ns = threads / ni, slots = (L.mx + ni - 1) / ni * ni * ((ms + ns - 3) / (ns - 2)) * ns;
+    if (least < 0 || slots <= least) {
+      least = slots;
+      best = ni;
+    }
+  }
+  return best;
+}
+
+inline dim3 node_sweep_grid(int dir, const Layout &L, SweepGeom &g, int ni = kNI, int threads = kSweepThreads) {
   g.dir = dir;
   if (dir == 0) {
     g.run = (idx_t)L.my * L.disp2;
-    const idx_t per = kSweepThreads - 2;
+    const idx_t per = threads - 2;
     return dim3((unsigned)((g.run + per - 1) / per), 1, (unsigned)L.mz);
   }
-  const int ns = kSweepThreads / ni;
+  const int ns = threads / ni;
   g.n_itile = (L.mx + ni - 1) / ni;
   const int ms = dir == 1 ? L.my : L.mz;
   g.n_stile = (ms + ns - 3) / (ns - 2);
