@@ -141,6 +141,12 @@ __global__ void k_bc_outflow(const __grid_constant__ Zone z, const __grid_consta
   }
   {
     const idx_t gg = z.L.at(i + gl * d[0], j + gl * d[1], k + gl * d[2]);
+    if (NS == 0 || p.i_eve < 0) {
+      NodeState<NS> a;
+      a.load(z, gb);
+      a.store(z, p, gg);
+      return;
+    }
     for (int l = 0; l < 6; ++l) z.bv[gg + l * sz] = z.bv[gb + l * sz];
     for (int l = 0; l < p.n_scalar; ++l) z.sv[gg + l * sz] = z.sv[gb + l * sz];
     // two-temperature: the ghost T_ve (the starting guess of its inversion from e_ve) is the
@@ -689,7 +695,8 @@ __global__ void k_bc_periodic_pair(const __grid_constant__ Zone z, const __grid_
 }
 
 // The same pairing for the 8th-order viscous node fluxes (components 1..n_var-1 of the three
-// flux arrays; component 0 carries no viscous flux and is never read).
+// flux arrays; component 0 carries no viscous flux and is never read), four components read before
+// any is written.
 template <typename F>
 __global__ void k_periodic_flux_pair(const __grid_constant__ Zone z, const __grid_constant__ Param p,
                                      const __grid_constant__ FaceBC f) {
@@ -703,20 +710,42 @@ __global__ void k_periodic_flux_pair(const __grid_constant__ Zone z, const __gri
   flux_arrays<F>(z, arr);
   if (it.p == 0) {
     const idx_t ga = along(z.L, f.face, it.i, it.j, it.k, 0), gb = along(z.L, f.face, it.i, it.j, it.k, m - 1);
-    for (int l = 1; l < p.n_var; ++l)
-      for (int a = 0; a < 3; ++a) {
-        const F ave = F(0.5) * (arr[a][ga + l * sz] + arr[a][gb + l * sz]);
-        arr[a][ga + l * sz] = ave;
-        arr[a][gb + l * sz] = ave;
-      }
+    for (int l0 = 1; l0 < p.n_var; l0 += 4) {
+      F v[3][4];
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int l = min(l0 + c, p.n_var - 1);
+          v[a][c] = F(0.5) * (arr[a][ga + l * sz] + arr[a][gb + l * sz]);
+        }
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int l = l0 + c;
+          if (l >= p.n_var) break;
+          arr[a][ga + l * sz] = v[a][c];
+          arr[a][gb + l * sz] = v[a][c];
+        }
+    }
     return;
   }
   const bool left = it.p <= g;
   const int dst = left ? -it.p : m - 1 + (it.p - g);
   const int src = left ? m - 1 - it.p : it.p - g;
   const idx_t gg = along(z.L, f.face, it.i, it.j, it.k, dst), gs = along(z.L, f.face, it.i, it.j, it.k, src);
-  for (int l = 1; l < p.n_var; ++l)
-    for (int a = 0; a < 3; ++a) arr[a][gg + l * sz] = arr[a][gs + l * sz];
+  // the divergence differentiates each array along its own direction only (fFlux along xi, gFlux
+  // along eta, hFlux along zeta), so only that array's ghosts along this direction are read
+  F *own = arr[f.face];
+  for (int l0 = 1; l0 < p.n_var; l0 += 4) {
+    F v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = own[gs + min(l0 + c, p.n_var - 1) * sz];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (l0 + c < p.n_var) own[gg + (l0 + c) * sz] = v[c];
+  }
 }
 
 // If periodic face f and the next periodic face in list order are the two faces of one

@@ -10,14 +10,25 @@ namespace cb2 {
 // 2-D blocks: copy the k = 0 plane into every k ghost plane (eliminate_k_gradient,
 // src/FieldOperation.cu:96-121).
 __device__ __forceinline__ void eliminate_k_gradient_point(const Zone &z, const Param &p, int i, int j) {
+  constexpr int B = 6;  // variables read before any is written
   const int g_ = z.ngg;
-  const idx_t sz = z.L.sz;
+  const idx_t sz = z.L.sz, pl = z.L.disp1;
   const idx_t g0 = z.L.at(i, j, 0);
-  for (int kk = 1; kk <= g_; ++kk) {
-    const idx_t gp = z.L.at(i, j, kk), gm = z.L.at(i, j, -kk);
-    for (int l = 0; l < 6; ++l) { z.bv[gp + l * sz] = z.bv[g0 + l * sz]; z.bv[gm + l * sz] = z.bv[g0 + l * sz]; }
-    for (int l = 0; l < p.n_scalar; ++l) { z.sv[gp + l * sz] = z.sv[g0 + l * sz]; z.sv[gm + l * sz] = z.sv[g0 + l * sz]; }
-    for (int l = 0; l < p.n_var; ++l) { z.cv[gp + l * sz] = z.cv[g0 + l * sz]; z.cv[gm + l * sz] = z.cv[g0 + l * sz]; }
+  const int n = 6 + p.n_scalar + p.n_var;
+  for (int l0 = 0; l0 < n; l0 += B) {
+    double *at[B], v[B];
+#pragma unroll
+    for (int a = 0; a < B; ++a) {
+      const int l = min(l0 + a, n - 1);
+      at[a] = (l < 6 ? z.bv + l * sz : l < 6 + p.n_scalar ? z.sv + (l - 6) * sz : z.cv + (l - 6 - p.n_scalar) * sz) + g0;
+      v[a] = *at[a];
+    }
+    for (int kk = 1; kk <= g_; ++kk)
+#pragma unroll
+      for (int a = 0; a < B; ++a) {
+        at[a][kk * pl] = v[a];
+        at[a][-kk * pl] = v[a];
+      }
   }
 }
 
@@ -65,8 +76,21 @@ __device__ __forceinline__ void bc_periodic_pair_item(const Zone &z, const Param
   if (!pair_item(f, g, t, it)) return;
   const int m = f.face == 0 ? z.mx : (f.face == 1 ? z.my : z.mz);
   const idx_t sz = z.L.sz;
+  const bool tt = NS > 0 && p.i_eve >= 0;
   if (it.p == 0) {
     const idx_t ga = along(z.L, f.face, it.i, it.j, it.k, 0), gb = along(z.L, f.face, it.i, it.j, it.k, m - 1);
+    if (!tt) {
+      NodeState<NS> a, b;
+      a.load(z, ga);
+      b.load(z, gb);
+#pragma unroll
+      for (int l = 0; l < 6; ++l) a.bv[l] = 0.5 * (a.bv[l] + b.bv[l]);
+#pragma unroll
+      for (int l = 0; l < NS; ++l) a.y[l] = 0.5 * (a.y[l] + b.y[l]);
+      a.store(z, p, ga);
+      a.store(z, p, gb);
+      return;
+    }
     for (int l = 0; l < 6; ++l) {
       const double ave = 0.5 * (z.bv[ga + l * sz] + z.bv[gb + l * sz]);
       z.bv[ga + l * sz] = ave;
@@ -85,6 +109,12 @@ __device__ __forceinline__ void bc_periodic_pair_item(const Zone &z, const Param
   const int dst = left ? -it.p : m - 1 + (it.p - g);
   const int src = left ? m - 1 - it.p : it.p - g;
   const idx_t gg = along(z.L, f.face, it.i, it.j, it.k, dst), gs = along(z.L, f.face, it.i, it.j, it.k, src);
+  if (!tt) {
+    NodeState<NS> a;
+    a.load(z, gs);
+    a.store(z, p, gg);
+    return;
+  }
   for (int l = 0; l < 6; ++l) z.bv[gg + l * sz] = z.bv[gs + l * sz];
   for (int l = 0; l < p.n_scalar; ++l) z.sv[gg + l * sz] = z.sv[gs + l * sz];
   cv_point<NS>(z, p, gg);

@@ -277,12 +277,12 @@ __device__ __forceinline__ double local_dt_point(const Zone &z, const Param &p, 
   return dt;
 }
 
-// Conservative variables of one node from its primitives (compute_cv_from_bv_1_point,
-// src/FieldOperation.cuh:163).
+// Conservative variables at g from primitive values (compute_cv_from_bv_1_point,
+// src/FieldOperation.cuh:163), one temperature.
 template <int NS>
-__device__ __forceinline__ void cv_point(const Zone &z, const Param &p, idx_t g) {
+__device__ __forceinline__ void cv_store(const Zone &z, const Param &p, idx_t g, const double *bv, const double *y) {
   const idx_t sz = z.L.sz;
-  const double rho = z.bv[g], u = z.bv[g + sz], v = z.bv[g + 2 * sz], w = z.bv[g + 3 * sz];
+  const double rho = bv[0], u = bv[1], v = bv[2], w = bv[3];
   z.cv[g] = rho;
   z.cv[g + sz] = rho * u;
   z.cv[g + 2 * sz] = rho * v;
@@ -290,26 +290,66 @@ __device__ __forceinline__ void cv_point(const Zone &z, const Param &p, idx_t g)
   double E = 0.5 * (u * u + v * v + w * w);
   if constexpr (NS == 0) {
     E *= rho;
-    E += z.bv[g + 4 * sz] / (kGammaAir - 1);
-  } else if (p.i_eve >= 0) {
-    // two-temperature (src/FieldOperation.cuh:154-158, 97-109)
-    sync_two_temperature<NS>(z, p, g);
-#pragma unroll
-    for (int s = 0; s <= NS; ++s) z.cv[g + (5 + s) * sz] = rho * z.sv[g + s * sz];
-    E = total_energy_2t<NS>(z, p, g);
+    E += bv[4] / (kGammaAir - 1);
   } else {
     double h[NS];
-    species_h<NS>(z.bv[g + 5 * sz], p.mech, h);
+    species_h<NS>(bv[5], p.mech, h);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const double y = z.sv[g + s * sz];
-      z.cv[g + (5 + s) * sz] = rho * y;
-      E += h[s] * y;
+      z.cv[g + (5 + s) * sz] = rho * y[s];
+      E += h[s] * y[s];
     }
     E *= rho;
-    E -= z.bv[g + 4 * sz];
+    E -= bv[4];
   }
   z.cv[g + 4 * sz] = E;
+}
+
+// The primitives of a node in registers (one temperature).  The face fills read a whole node before
+// they write one: a fill that copies variable by variable waits for memory at each, because the
+// compiler cannot move a load over the store before it.
+template <int NS>
+struct NodeState {
+  double bv[6], y[NS > 0 ? NS : 1];
+  __device__ __forceinline__ void load(const Zone &z, idx_t g) {
+    const idx_t sz = z.L.sz;
+#pragma unroll
+    for (int l = 0; l < 6; ++l) bv[l] = z.bv[g + l * sz];
+#pragma unroll
+    for (int l = 0; l < NS; ++l) y[l] = z.sv[g + l * sz];
+  }
+  __device__ __forceinline__ void store(const Zone &z, const Param &p, idx_t g) const {
+    const idx_t sz = z.L.sz;
+#pragma unroll
+    for (int l = 0; l < 6; ++l) z.bv[g + l * sz] = bv[l];
+#pragma unroll
+    for (int l = 0; l < NS; ++l) z.sv[g + l * sz] = y[l];
+    cv_store<NS>(z, p, g, bv, y);
+  }
+};
+
+// Conservative variables of one node from its stored primitives.
+template <int NS>
+__device__ __forceinline__ void cv_point(const Zone &z, const Param &p, idx_t g) {
+  const idx_t sz = z.L.sz;
+  if (NS > 0 && p.i_eve >= 0) {
+    if constexpr (NS > 0) {
+      const double rho = z.bv[g], u = z.bv[g + sz], v = z.bv[g + 2 * sz], w = z.bv[g + 3 * sz];
+      z.cv[g] = rho;
+      z.cv[g + sz] = rho * u;
+      z.cv[g + 2 * sz] = rho * v;
+      z.cv[g + 3 * sz] = rho * w;
+      // two-temperature (src/FieldOperation.cuh:154-158, 97-109)
+      sync_two_temperature<NS>(z, p, g);
+#pragma unroll
+      for (int s = 0; s <= NS; ++s) z.cv[g + (5 + s) * sz] = rho * z.sv[g + s * sz];
+      z.cv[g + 4 * sz] = total_energy_2t<NS>(z, p, g);
+    }
+    return;
+  }
+  NodeState<NS> q;
+  q.load(z, g);
+  cv_store<NS>(z, p, g, q.bv, q.y);
 }
 
 }  // namespace cb2
