@@ -864,7 +864,7 @@ def square_cylinder_variants(args, local_rank, one_case_value=None):
 def batched_blocks(args, local_rank):
     """Batched form: --batch-blocks closed periodic sine-wave blocks (WENO7 + AUSM+, inviscid,
     FP64) of seeded uneven sizes n^3 nodes, n ~ U{12..40}, advanced --batch-steps CFL steps
-    (a) in one persistent launch (cb2_block_batch_advance, tile width and cluster size tuned first) and (b) one
+    (a) together (cb2_block_batch_advance, tile width tuned first) and (b) one
     block after another through cb2_rk3_step, each from the same initial states.  Wall clock
     around each form (the batch call synchronises; the loop ends with a synchronise)."""
     import numpy as np
@@ -884,7 +884,7 @@ def batched_blocks(args, local_rank):
     out = {"workload": f"{args.batch_blocks} periodic sine-wave blocks of n^3 nodes, n ~ U{{12..40}} (seeded), "
                        f"WENO7 + AUSM+, inviscid, CFL 0.5 steps, FP64", "blocks": args.batch_blocks,
            "nodes": nodes, "steps": S}
-    # (a) one persistent launch
+    # (a) all blocks together
     devs = [DeviceBlock(hb, device=f"cuda:{local_rank}") for _, hb, _ in blocks]
     ctx = cb200.Context(p0)
     cs = (abi.BlockCase * len(blocks))()

@@ -143,12 +143,12 @@ class Context:
         return list(out)
 
     def block_batch_advance(self, cases, max_steps, stream=None):
-        """Advance a ctypes array of abi.BlockCase in one persistent launch (cb2_block_batch_advance)."""
+        """Advance a ctypes array of abi.BlockCase together (cb2_block_batch_advance)."""
         check(self.lib.cb2_block_batch_advance(self.h, C.cast(cases, C.c_void_p), len(cases), max_steps, stream),
               "cb2_block_batch_advance")
 
     def block_batch_autotune(self, cases, stream=None):
-        """(tile width, cluster size) picked by timing the batch's residual phase."""
+        """(tile width picked by timing the batch's residual phase, cluster size last set)."""
         out = (C.c_int * 2)()
         check(self.lib.cb2_block_batch_autotune(self.h, C.cast(cases, C.c_void_p), len(cases), out, stream),
               "cb2_block_batch_autotune")
