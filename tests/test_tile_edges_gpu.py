@@ -1,5 +1,5 @@
-"""Residuals at block sizes around the edges of the sweep tiles, against the oracle: 510 and 254 nodes
-of a run along x; 14, 30 or 62 own nodes by 16 or 8 columns along y and z; 30 (x) and 14 (y, z) own
+"""Residuals at block sizes around the edges of the sweep tiles, against the oracle: runs of a k plane
+along x around 510 and 254 nodes; 14, 30 or 62 own nodes by 16 or 8 columns along y and z; 30 (x) and 14 (y, z) own
 nodes of the 2nd-order viscous tiles.  One residual at 1e-12 of each variable's largest value, the bar
 of the parity tests."""
 import os
@@ -29,7 +29,7 @@ def gpu_rhs(p, hb, faces):
     return out
 
 
-@pytest.mark.parametrize("dims", [(16, 30, 6), (17, 31, 6), (8, 62, 6), (9, 63, 6), (6, 6, 33), (503, 6, 6), (247, 7, 6), (15, 14, 15)])
+@pytest.mark.parametrize("dims", [(16, 30, 6), (17, 31, 6), (8, 62, 6), (9, 63, 6), (6, 6, 33), (57, 8, 6), (43, 10, 6), (15, 14, 15)])
 @pytest.mark.parametrize("scheme,rec", [(abi.INV_AUSMP, abi.REC_WENO7), (abi.INV_HLLC, abi.REC_WENO5), (abi.INV_WENO7_CH, abi.REC_MUSCL)],
                          ids=["ausm_weno7", "hllc_weno5", "weno7_ch"])
 def test_air_sweeps(dims, scheme, rec):
