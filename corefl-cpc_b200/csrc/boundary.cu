@@ -18,6 +18,7 @@
 #include "point.cuh"
 #include "launch.h"
 #include "boundary.cuh"
+#include "outflow_apart.h"
 
 namespace cb2 {
 
@@ -770,18 +771,12 @@ static int periodic_pair(const Zone &z, const FaceBC *faces, int n, int f, int *
   return a.direction < 0 ? f : q;
 }
 
-// Whether two outflow faces neither write a common ghost node nor read what the other writes: faces of
-// the block's own extent (not extended into the tangential ghosts), on different sides or with
-// tangential ranges apart.
 static bool outflow_apart(const Zone &z, const FaceBC &a, const FaceBC &b) {
   const int ext[3] = {z.mx, z.my, z.mz};
-  for (const FaceBC *f : {&a, &b})
-    for (int d = 0; d < 3; ++d)
-      if (std::min(f->start[d], f->end[d]) < 0 || std::max(f->start[d], f->end[d]) > ext[d] - 1) return false;
-  if (a.face != b.face || a.direction != b.direction) return true;
-  for (int d = 0; d < 3; ++d)
-    if (d != a.face && (a.end[d] < b.start[d] || b.end[d] < a.start[d])) return true;
-  return false;
+  auto range = [](const FaceBC &f) {
+    return OutflowRange{f.face, f.direction, {f.start[0], f.start[1], f.start[2]}, {f.end[0], f.end[1], f.end[2]}, f.p > 0};
+  };
+  return outflow_apart(ext, z.ngg, range(a), range(b));
 }
 
 // Small CTAs: a face has few nodes, and spreading them over more SMs shortens the launch.
@@ -812,8 +807,8 @@ static int launch_bc_ns(const Zone &z, const Param &p, const FaceBC *faces, int 
         }
       }
       if (t == CB2_BC_OUTFLOW) {
-        // an outflow face reads the block's nodes and writes ghosts beyond it, so faces whose ghosts
-        // do not overlap fill in one launch
+        // faces that neither write nor read what another writes (outflow_apart.h) fill in one launch,
+        // the others one after the other in list order
         FaceSet set;
         int ns = 0;
         long long most = 0;
