@@ -167,8 +167,10 @@ __device__ __forceinline__ void state_energy(T *pv, const Mech &m) {
 }
 
 // FP64: |grad xi|, its reciprocal and the sound speeds from reciprocal square roots,
-// sqrt(gamma p / rho) = gamma p / sqrt(gamma p rho), and products with reciprocals in place of the
+// sqrt(gamma p / rho) = |gamma p| / sqrt(gamma p rho), and products with reciprocals in place of the
 // divisions.  FP32 keeps the hardware's own square roots and quotients, which cost one instruction.
+// Where gamma p rho leaves the normal range the factors are scaled into it, and p = 0 has the sound
+// speed 0: the flux between it and a side of positive pressure is finite.
 template <typename T>
 __device__ __forceinline__ void norm_pair(T k2, T &k, T &ik) {
   if constexpr (sizeof(T) == 8) {
@@ -182,8 +184,14 @@ __device__ __forceinline__ void norm_pair(T k2, T &k, T &ik) {
 template <typename T>
 __device__ __forceinline__ T sound_speed(T gamma, T p, T rho) {
   if constexpr (sizeof(T) == 8) {
-    const T gp = gamma * p;
-    return mul_rn(gp, recip_sqrt(gp * rho));
+    T gp = gamma * p, x = gp * rho;
+    if (!(x >= T(2.2250738585072014e-308) && x <= T(1.7976931348623157e+308))) {
+      const T s = fabs(x) < 1 ? T(0x1p600) : T(0x1p-600);
+      gp *= s;
+      x = gp * (rho * s);
+      if (gp == 0 && fabs(rho) > 0) return 0;
+    }
+    return mul_rn(fabs(gp), recip_sqrt(x));
   } else {
     return sqrt(gamma * p / rho);
   }
