@@ -51,8 +51,9 @@ __global__ void k_batch_owner(const int *first, int n, int total, int *owner) {
   owner[t] = lo;
 }
 
-// Closes the step just taken (if any) and opens the next one.
-__global__ void k_batch_step(BlockState *state, int n, int close, int *n_active) {
+// Closes the step just taken (if any) and opens the next one; all: for every block, whether or not it
+// has reached its end time (a residual to be timed).
+__global__ void k_batch_step(BlockState *state, int n, int close, int all, int *n_active) {
   chain_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
@@ -67,7 +68,7 @@ __global__ void k_batch_step(BlockState *state, int n, int close, int *n_active)
       ++s.steps;
     }
   }
-  s.active = !(s.status & CB2_BLOCK_FAILED) && s.time < s.t_end;
+  s.active = all || (!(s.status & CB2_BLOCK_FAILED) && s.time < s.t_end);
   s.bad = 0;
   s.dt_bits = (unsigned long long)__double_as_longlong(s.dt_fixed > 0 ? s.dt_fixed : 1e+6);
   if (s.active) atomicAdd(n_active, 1);
@@ -228,7 +229,7 @@ int run(const Batch &t, const Param &p0, int max_steps, int mode) {
   const int T = kBatchThreads, nb = (t.n + T - 1) / T;
   auto open = [&](int close) {
     CB2_TRY(check_cuda(cudaMemsetAsync(b.n_active, 0, sizeof(int), t.s)));
-    CB2_TRY(launch_chain(k_batch_step, nb, T, 0, t.s, b.state, t.n, close, b.n_active));
+    CB2_TRY(launch_chain(k_batch_step, nb, T, 0, t.s, b.state, t.n, close, mode == 1 ? 1 : 0, b.n_active));
     ++t.nl;
     return check_launch();
   };

@@ -109,6 +109,24 @@ def test_batch_result_independent_of_company_and_tiles(oracle_lib):
         assert np.array_equal(d.to_host(["cv"])["cv"], hb.a["cv"])
 
 
+def test_autotune_times_the_residual_of_every_block(oracle_lib):
+    """Blocks at or past their end time too: each candidate width leaves every block's residual in dq."""
+    blocks = _blocks(oracle_lib, abi.INV_AUSMP, abi.REC_WENO7)
+    ctx = cb200.Context(blocks[0][0])
+    cases, devs = _cases_for(blocks, 1e-3)
+    for c, (t, t_end) in zip(cases, ((0.0, 0.0), (0.0, 1.0), (2.0, 1.0), (0.5, 0.5))):
+        c.time, c.t_end = t, t_end
+    ctx.block_batch_autotune(cases)
+    for (p, hb, faces), d in zip(blocks, devs):
+        one = DeviceBlock(hb)
+        path = cb200.Context(p)
+        path.bind(0, one.view(), faces)
+        path.rhs(0)
+        _sync()
+        assert np.array_equal(d.to_host(["dq"])["dq"], one.to_host(["dq"])["dq"]), (hb.mx, hb.my, hb.mz)
+        path.close()
+
+
 def test_batch_stops_each_block_at_its_end_time(oracle_lib):
     blocks = _blocks(oracle_lib, abi.INV_HLLC, abi.REC_WENO5)[:3]
     ctx = cb200.Context(blocks[0][0])
