@@ -60,3 +60,22 @@ def curvilinear_air_case(mx=20, my=18, mz=16, ngg=4, scheme=abi.INV_WENO5_CH, re
     if sensor is not None:
         param.shock_sensor, param.sensor_threshold, param.sensor_eps = sensor
     return param, b, faces
+
+
+def sub_mechanism(mech, names):
+    """The mechanism of the named species of `mech` and the reactions among them."""
+    from cb200 import mech as mechmod
+    keep = [mech.index(n) for n in names]
+    gone = [s for s in range(mech.ns) if s not in keep]
+    nr, d = mech.nr, dict(mech.d)
+    both = np.asarray(d["stoi_f"]).reshape(nr, -1) + np.asarray(d["stoi_b"]).reshape(nr, -1)
+    reac = [r for r in range(nr) if not both[r, gone].any()]
+    for name in abi.MECH_DOUBLE + ("species",):
+        a = np.asarray(d[name])
+        a = a.reshape(mech.ns, mech.ns)[np.ix_(keep, keep)] if a.size == mech.ns ** 2 else a.reshape(mech.ns, -1)[keep]
+        d[name] = a.reshape(-1).tolist()
+    for name in abi.MECH_INT + abi.MECH_REAC:
+        a = np.asarray(d[name]).reshape(nr, -1)[reac]
+        d[name] = (a[:, keep] if a.shape[1] == mech.ns else a).reshape(-1).tolist()
+    d["n_spec"], d["n_reac"] = len(keep), len(reac)
+    return mechmod.MechStruct(d)

@@ -1,7 +1,7 @@
-"""Batched closed blocks (cb2_block_batch_advance): uneven 2-D and 3-D periodic air blocks in one
-persistent launch must give, block by block, the same bits as cb2_rk3_step on that block, with
-fixed and CFL steps, whatever other blocks share the batch and whatever tile width and cluster
-size the autotuner picks."""
+"""Batched closed blocks (cb2_block_batch_advance): uneven 2-D and 3-D periodic air blocks, every phase of
+a step in one launch over all of them, must give, block by block, the same bits as cb2_rk3_step on that
+block, with fixed and CFL steps, whatever other blocks share the batch (failing ones among them) and
+whatever tile width is set or tuned."""
 import numpy as np
 import pytest
 
@@ -97,13 +97,15 @@ def test_batch_result_independent_of_company_and_tiles(oracle_lib):
     alone, _ = _batch(ctx, blocks[1:2], 3, dt)
     ref = alone[0].to_host(["cv"])["cv"]
     for w in (4, 8, 16):
-        for cs in (1, 2, 4, 8):
-            ctx.block_batch_set_schedule(w, cs)
-            together, cases = _batch(ctx, blocks, 3, dt)
-            assert np.array_equal(together[1].to_host(["cv"])["cv"], ref), (w, cs)
+        ctx.block_batch_set_schedule(w, 8)
+        for company in ((1,), (0, 1, 2, 3), (2, 1), (3, 1, 0, 1)):
+            together, cases = _batch(ctx, [blocks[c] for c in company], 3, dt)
+            for c, d in zip(company, together):
+                if c == 1:
+                    assert np.array_equal(d.to_host(["cv"])["cv"], ref), (w, company)
     tune_cases, keep = _cases_for(blocks, dt)
     ni, cs = ctx.block_batch_autotune(tune_cases)
-    assert ni in (4, 8, 16) and cs in (1, 2, 4, 8)
+    assert ni in (4, 8, 16) and cs == 8  # the cluster size is the one last set
     # tuning touched only the residual scratch dq
     for (_, hb, _), d in zip(blocks, keep):
         assert np.array_equal(d.to_host(["cv"])["cv"], hb.a["cv"])
@@ -139,6 +141,38 @@ def test_batch_stops_each_block_at_its_end_time(oracle_lib):
     ctx.block_batch_advance(cases, 100)
     assert [c.steps for c in cases] == [3, 5, 8]
     assert all(c.status == abi.BLOCK_DONE for c in cases)
+
+
+@pytest.mark.parametrize("kind", ["cfl", "update"])
+def test_batch_reports_failed_blocks(oracle_lib, kind):
+    """A block whose CFL step is not a number stops before it; one whose update leaves the physical range
+    runs on and is reported; the others do not notice."""
+    blocks = _blocks(oracle_lib, abi.INV_AUSMP, abi.REC_WENO7)
+    bad, steps = 1, 3
+    dts = [0.0 if kind == "cfl" else 0.2 * oracle_lib.cfl_dt(p, hb) for p, hb, _ in blocks]
+    if kind == "cfl":
+        hb = blocks[bad][1]
+        hb.a["bv"][5, hb.ngg + 2, hb.ngg + 3, hb.ngg + 4] = np.nan
+    else:
+        dts[bad] *= 1e4
+    cases, devs = _cases_for(blocks, 0.0)
+    for c, dt in zip(cases, dts):
+        c.dt = dt
+    ctx = cb200.Context(blocks[0][0])
+    ctx.block_batch_advance(cases, steps)
+    _sync()
+    assert cases[bad].status == abi.BLOCK_FAILED
+    if kind == "cfl":
+        assert cases[bad].steps == 0 and cases[bad].time == 0.0 and cases[bad].last_dt == 0.0
+        assert np.array_equal(devs[bad].to_host(["cv"])["cv"], blocks[bad][1].a["cv"])
+    else:
+        assert cases[bad].steps == steps
+    for i, ((p, hb, faces), d, c) in enumerate(zip(blocks, devs, cases)):
+        if i == bad:
+            continue
+        ref, t = _reference(p, hb, faces, steps, dts[i])
+        assert (c.steps, c.status, c.time) == (steps, 0, t)
+        assert np.array_equal(d.to_host(["cv"])["cv"], ref["cv"]), i
 
 
 def test_batch_rejects_unsupported_settings(oracle_lib):

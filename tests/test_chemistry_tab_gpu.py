@@ -1,13 +1,16 @@
 """The block chemistry kernel on a repacked mechanism against the oracle: sizes around the edges of
 its tiles of 128 nodes of a k plane, temperatures in both ranges of the NASA7 fits, at their middle
-and beyond their ends, absent species, and the mechanisms that do not fit a table (more than 24
-reactions, more than eight reactants), which run the generic kernel."""
+and beyond their ends, absent species, five species, a species with a middle temperature of its own,
+third bodies that are absent, the longest mechanism and the longest side of a reaction that fit a table,
+and the mechanisms that do not (more than 24 reactions, more than eight reactants), which run the
+generic kernel."""
 import copy
 import os
 
 import numpy as np
 import pytest
 
+import helpers
 import oracle_py
 from cb200 import abi, cases, mech as mechmod
 from cb200.field import HostBlock, array_specs
@@ -20,15 +23,27 @@ def mechanism(kind):
     h2 = mechmod.load_json(GOLD)
     d = copy.deepcopy(h2.d)
     ns, nr = h2.ns, h2.nr
-    if kind == "long":  # the first eight reactions again: 27
+    if kind in ("long", "full"):  # the first reactions again: 27, 24
+        more = 8 if kind == "long" else 5
         for name in abi.MECH_INT + abi.MECH_REAC:
             a = np.asarray(d[name]).reshape(nr, -1)
-            d[name] = np.concatenate([a, a[:8]]).reshape(-1).tolist()
-        d["n_reac"] = nr + 8
-    elif kind == "steep":  # H + O2 -> O + OH with ten H on the left
+            d[name] = np.concatenate([a, a[:more]]).reshape(-1).tolist()
+        d["n_reac"] = nr + more
+    elif kind in ("steep", "eight"):  # H + O2 -> O + OH with ten H on the left; with seven
         a = np.asarray(d["stoi_f"]).reshape(nr, ns)
-        a[0, list(h2.species).index("H")] = 10
+        a[0, list(h2.species).index("H")] = 10 if kind == "steep" else 7
         d["stoi_f"] = a.reshape(-1).tolist()
+    elif kind == "five":
+        return helpers.sub_mechanism(h2, ("H", "O2", "O", "OH", "HO2"))
+    elif kind == "five_h2":
+        return helpers.sub_mechanism(h2, ("O", "H2", "OH", "O2", "H"))
+    elif kind == "middles":  # a middle temperature of its own
+        d["t_mid"][3] = 1100.0
+    elif kind == "no_body":  # the only third body of every such reaction is a species that is not there
+        a = np.zeros((nr, ns))
+        a[:, 1] = 1.0
+        d["third_body_coeff"] = a.reshape(-1).tolist()
+        d["reac_type"] = [5 if t > 5 else t for t in d["reac_type"]]  # Troe's form has no value there
     elif kind == "irreversible":  # no backward rate for some
         d["reac_type"][1] = d["reac_type"][16] = 0
     elif kind == "explicit":  # every backward rate from its own Arrhenius constants
@@ -60,7 +75,9 @@ def block(mech, dims, seed):
 @pytest.mark.parametrize("dims,kind", [((1, 1, 1), "h2"), ((127, 1, 1), "h2"), ((43, 3, 2), "h2"), ((64, 2, 3), "h2"),
                                        ((17, 23, 5), "h2"), ((17, 5, 2), "irreversible"), ((17, 5, 2), "explicit"),
                                        ((17, 5, 2), "long"),
-                                       ((17, 5, 2), "steep")])
+                                       ((17, 5, 2), "steep"), ((17, 5, 2), "full"), ((17, 5, 2), "eight"),
+                                       ((17, 5, 2), "five"), ((43, 3, 2), "five_h2"), ((17, 5, 2), "middles"),
+                                       ((17, 5, 2), "no_body")])
 def test_chemistry_against_oracle(dims, kind):
     import torch
     import cb200
