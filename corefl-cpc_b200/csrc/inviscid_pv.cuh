@@ -185,7 +185,7 @@ template <typename T>
 __device__ __forceinline__ T sound_speed(T gamma, T p, T rho) {
   if constexpr (sizeof(T) == 8) {
     T gp = gamma * p, x = gp * rho;
-    if (!(x >= T(2.2250738585072014e-308) && x <= T(1.7976931348623157e+308))) {
+    if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) {  // not a positive normal number
       const T s = fabs(x) < 1 ? T(0x1p600) : T(0x1p-600);
       gp *= s;
       x = gp * (rho * s);
