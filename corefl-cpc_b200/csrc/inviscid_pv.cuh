@@ -808,14 +808,15 @@ template <typename T, int NS, int DIR, int REC, int SOLVER, bool VF = false, boo
 static int launch_pv_yz_ni(const Zone &z, const Param &p, cudaStream_t s) {
   if constexpr ((REC == 5 || REC == 7) && NS == 0) {
     // the tuned width, or the one that fits the block best
-    const int ni = z.tile_ni[DIR] || sizeof(T) == 4 ? z.tile_ni[DIR] : fewest_slots_ni(z.L, DIR, pv_threads<T, NS, SOLVER>());
+    const int ni = z.tile_ni[DIR] || sizeof(T) == 4 ? z.tile_ni[DIR] : cheapest_ni(z.L, DIR, pv_threads<T, NS, SOLVER>());
     if (ni == 4) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 4, VF>(z, p, s);
     if (ni == 16) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 16, VF>(z, p, s);
   }
   // mixtures: 16 columns (128-byte rows) although 2 of 16 nodes are overlap instead of 2 of 32; their
-  // 18 arrays per node make the loads count (192^3 H2/air: y, z 6.5 -> 6.3 ms per step each; with the
-  // gas constants as kernel parameters 3.85: as global loads they missed an L1 that the tiles' shared
-  // memory leaves 20 KB)
+  // 18 arrays per node make the loads count.  64^3 H2/air residuals (three sweeps) at 8 and at 16
+  // columns, us: AUSM+ 136 / 117 (MUSCL) and 206 / 183 (WENO7), HLLC 184 / 163 (WENO5), Roe 342 / 315
+  // (WENO7), in the mixed form 143 / 131 (HLLC, WENO5); two temperatures, bound by their thermodynamics,
+  // the same either way; the smallest blocks lose a little (24^3 with viscous and chemistry 78.7 / 80.9).
   if constexpr (NS > 0) return launch_pv_yz<T, NS, DIR, REC, SOLVER, 16, VF, TT>(z, p, s);
   else return launch_pv_yz<T, NS, DIR, REC, SOLVER, kNI, VF, TT>(z, p, s);
 }

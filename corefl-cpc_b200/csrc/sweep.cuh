@@ -48,16 +48,21 @@ __host__ __device__ __forceinline__ int node_sweep_nodes(int dir, int r) {
 // it per block and direction among kTileNI.
 constexpr int kTileNI[3] = {4, 8, 16};
 
-// The y/z tile width that spends the fewest node slots on a block (whole tiles of ni columns by
-// threads / ni nodes, two of them overlap), the wider rows on a tie.
-inline int fewest_slots_ni(const Layout &L, int dir, int threads) {
+// The y/z tile width that spends the least on a block: node slots (whole tiles of ni columns by
+// threads / ni nodes, two of them overlap), a slot of 4 columns counted 1.3 times, the wider rows on a
+// tie.  Rows of 4 columns are 32 bytes, a quarter of a cache line.  FP64 AUSM+ and
+// WENO7, y, us at 4 / 8 / 16 columns: 126^3 160 / 164 / 142 (the fewest slots: 4), 124x120x124
+// 146 / 129 / 124 (4), 257x257x65 400 / 312 / 288 (16), 20x126x126 29 / 35 / 39 (4), 5x200x200
+// 29 / 28 / 45 (8).
+inline int cheapest_ni(const Layout &L, int dir, int threads) {
   const long long ms = dir == 1 ? L.my : L.mz;
   int best = kTileNI[0];
   long long least = -1;
   for (int ni : kTileNI) {
     const long long ns = threads / ni, slots = (L.mx + ni - 1) / ni * ni * ((ms + ns - 3) / (ns - 2)) * ns;
-    if (least < 0 || slots <= least) {
-      least = slots;
+    const long long cost = slots * (ni == 4 ? 13 : 10);
+    if (least < 0 || cost <= least) {
+      least = cost;
       best = ni;
     }
   }
