@@ -54,11 +54,12 @@ KERNEL_BYTES_PER_NODE_MIXED = dict(KERNEL_BYTES_PER_NODE, **{
 # sm__sass_thread_inst_executed_op_d{fma,mul,add}_pred_on on the 129^3 sine wave, per node of one
 # launch; these kernels are bound by the FP64 pipe, not by HBM.  The FP64 peak is the B200's
 # nominal (no measured FP64 figure is available).
-KERNEL_FP64_FLOPS_PER_NODE = {"pv_flux_x": 1500, "pv_flux_y": 1500, "pv_flux_z": 1500}
+KERNEL_FP64_FLOPS_PER_NODE = {"pv_flux_x": 1089, "pv_flux_y": 1145, "pv_flux_z": 1147}
 FP64_NOMINAL_TFLOPS = 37.0
-FLOPS_PER_CELL_UPDATE = 15000  # 3 stages x (3 sweeps x 1,500 + node fluxes 406 + divergence 144)
+# 3 stages x (sweeps 1,089 + 1,145 + 1,147, node fluxes 355, divergence 144, update 80)
+FLOPS_PER_CELL_UPDATE = 11880
 # per padded node (kernels that sweep the ghost layers too)
-KERNEL_BYTES_PER_PADDED_NODE = {"bv_to_f32": 6 * (8 + 4), "store_qn": 5 * 16, "properties": 8 * (4 + 2)}
+KERNEL_BYTES_PER_PADDED_NODE = {"bv_to_f32": 6 * (8 + 4), "properties": 8 * (4 + 2)}
 
 
 def kernel_rooflines(prof, nodes, padded, bytes_map, peak):
@@ -115,7 +116,7 @@ def parse():
                     help="time one ROK4E attempt of the batched H2/air reactors at several batch sizes")
     ap.add_argument("--schedule", default=None,
                     help="use these tile widths instead of timing them: 'NI' for the y/z sweeps and the "
-                         "batch, or 'NI,CS' to also fix the batch's cluster size (e.g. from an earlier run)")
+                         "batch (e.g. from an earlier run); a second number, 'NI,CS', has no effect on the launches")
     ap.add_argument("--accuracy-steps", type=int, default=100,
                     help="RK3 steps of the mixed-vs-FP64 accuracy run (the workload's 100 steps)")
     return ap.parse_args()

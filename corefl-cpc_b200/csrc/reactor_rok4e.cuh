@@ -205,7 +205,7 @@ struct RokLU {
     step = N;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
-      // the largest |a| by its leading bits (16 of the mantissa); ties go to the lowest lane
+      // the largest |a| by its leading bits (15 of the mantissa); ties go to the lowest lane
       const unsigned key = used ? 0u : (((unsigned)__double2hiint(fabs(a[n])) & ~31u) | (31u - lane)) | 1u << 31;
       const unsigned best = __reduce_max_sync(kFullWarp, key);
       const int p = 31 - (int)(best & 31u);

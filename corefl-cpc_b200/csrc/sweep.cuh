@@ -44,8 +44,8 @@ __host__ __device__ __forceinline__ int node_sweep_nodes(int dir, int r) {
   return dir == 0 ? (kSweepThreads + 2 * r) : kNI * (kNS + 2 * r);
 }
 
-// ni: i-columns of a y/z tile (kSweepThreads / ni nodes along the sweep); the autotuner picks
-// it per block and direction among kTileNI.
+// ni: i-columns of a y/z tile (threads / ni nodes along the sweep); the autotuner picks it per
+// block and direction among kTileNI.
 constexpr int kTileNI[3] = {4, 8, 16};
 
 // The y/z tile width that spends the least on a block: node slots (whole tiles of ni columns by

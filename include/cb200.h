@@ -99,7 +99,9 @@ typedef struct cb2_zone_view {
   double *acoustic_speed; /* ghost ngg, mixtures                             */
   double *gamma;    /* ghost ngg, mixtures                                  */
   double *mach;     /* ghost ngg, optional                                  */
-  double *fFlux, *gFlux, *hFlux; /* n_var comps, ghost ngg (8th-order viscous node fluxes) */
+  double *fFlux, *gFlux, *hFlux; /* n_var comps, ghost ngg (8th-order viscous node fluxes along xi, eta,
+                     * zeta; scratch: of the ghosts beyond periodic faces only those along the array's
+                     * own direction, which its derivative reads, are filled) */
   double *vis_flux; /* n_var-1 comps, ghost 1 (2nd-order viscous face fluxes)  */
   double *shock_sensor;         /* ghost ngg, hybrid schemes only           */
   double *dt_local;             /* ghost 0                                  */
