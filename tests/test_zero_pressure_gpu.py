@@ -1,8 +1,9 @@
 """AUSM+ and HLLC fluxes next to nodes whose sound speed leaves the range of the fast reciprocal square
 root, against the oracle: a pressure of exactly zero (no sound speed; the flux between it and a side of
-positive pressure is finite), pressures whose product with the density is subnormal or underflows, and
-for AUSM+ a node of negative density and pressure, whose quotient is positive.  The odd nodes are
-isolated, so that first-order and MUSCL (minmod) states take their values exactly."""
+positive pressure is finite), pressures whose product with the density is subnormal (a sound speed of
+at most 1e-153, nothing beside the other side's whatever its digits), and for AUSM+ a node of negative
+density and pressure, whose quotient is positive.  The odd nodes are isolated, so that first-order and
+MUSCL (minmod) states take their values exactly."""
 import os
 
 import numpy as np
