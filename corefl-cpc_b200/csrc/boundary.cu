@@ -37,7 +37,8 @@ __device__ __forceinline__ bool face_point(const FaceBC &f, int &i, int &j, int 
 
 // One thread per (face node, layer): consecutive threads take consecutive nodes of one layer.
 // The layers of a face node are independent of one another in the outflow, inflow, symmetry and
-// wall fills (each reads only interior nodes or the face's own constants), so every layer's cv
+// wall fills (each reads only interior nodes or the face's own constants; not so on thin blocks, see
+// thin_block), so every layer's cv
 // rebuild -- the costly part with two temperatures -- runs in its own thread.
 __device__ __forceinline__ bool face_layer_point(const FaceBC &f, int n_layer, int &i, int &j, int &k, int &l) {
   const long long n = (long long)(f.end[0] - f.start[0] + 1) * (f.end[1] - f.start[1] + 1) * (f.end[2] - f.start[2] + 1);
@@ -282,10 +283,11 @@ __device__ __forceinline__ void project_to_interior(const Zone &z, int &i, int &
 // supersonic outflow keeps the interior state; the scalars come from the farfield on inflow and
 // from the interior on outflow.  Subsonic ghosts are reflected about the face state, supersonic
 // ones equal it.  One thread per (face node, layer): every layer reads interior nodes only.
-template <int NS>
+// LINE: one thread per face node takes the layers in order (see thin_block).
+template <int NS, bool LINE>
 __global__ void k_bc_farfield(Zone z, Param p, FaceBC f) {
   int i, j, k, gl;
-  if (!face_layer_point(f, z.ngg + 1, i, j, k, gl)) return;
+  if (!face_layer_point(f, LINE ? 1 : z.ngg + 1, i, j, k, gl)) return;
   int d[3] = {0, 0, 0};
   d[f.face] = f.direction;
   const idx_t sz = z.L.sz;
@@ -348,32 +350,34 @@ __global__ void k_bc_farfield(Zone z, Param p, FaceBC f) {
       t_b = p_b / fmax(rho_b * r_mix(), 1e-12);
     }
   }
-  double st[6] = {rho_b, u_b, v_b, w_b, p_b, t_b};
-  double tve_s = tve_b;
-  idx_t gw = gf;
-  if (gl > 0) {
-    int ai = i - gl * d[0], aj = j - gl * d[1], ak = k - gl * d[2];
-    project_to_interior(z, ai, aj, ak);
-    const idx_t gi = z.L.at(ai, aj, ak);
-    gw = z.L.at(i + gl * d[0], j + gl * d[1], k + gl * d[2]);
-    if (mn_in > -1.0 && mn_in < 1.0) {
-      double rho_g = 2 * rho_b - z.bv[gi], p_g = 2 * p_b - z.bv[gi + 4 * sz];
-      rho_g = fmax(rho_g, 0.1 * fmax(rho_b, 1e-12));
-      p_g = fmax(p_g, 0.1 * fmax(p_b, 1.0));
-      st[0] = rho_g;
-      st[1] = 2 * u_b - z.bv[gi + sz];
-      st[2] = 2 * v_b - z.bv[gi + 2 * sz];
-      st[3] = 2 * w_b - z.bv[gi + 3 * sz];
-      st[4] = p_g;
-      st[5] = p_g / fmax(rho_g * r_mix(), 1e-12);
+  const int last = LINE ? z.ngg : gl;
+  for (; gl <= last; ++gl) {
+    double st[6] = {rho_b, u_b, v_b, w_b, p_b, t_b};
+    idx_t gw = gf;
+    if (gl > 0) {
+      int ai = i - gl * d[0], aj = j - gl * d[1], ak = k - gl * d[2];
+      project_to_interior(z, ai, aj, ak);
+      const idx_t gi = z.L.at(ai, aj, ak);
+      gw = z.L.at(i + gl * d[0], j + gl * d[1], k + gl * d[2]);
+      if (mn_in > -1.0 && mn_in < 1.0) {
+        double rho_g = 2 * rho_b - z.bv[gi], p_g = 2 * p_b - z.bv[gi + 4 * sz];
+        rho_g = fmax(rho_g, 0.1 * fmax(rho_b, 1e-12));
+        p_g = fmax(p_g, 0.1 * fmax(p_b, 1.0));
+        st[0] = rho_g;
+        st[1] = 2 * u_b - z.bv[gi + sz];
+        st[2] = 2 * v_b - z.bv[gi + 2 * sz];
+        st[3] = 2 * w_b - z.bv[gi + 3 * sz];
+        st[4] = p_g;
+        st[5] = p_g / fmax(rho_g * r_mix(), 1e-12);
+      }
     }
-  }
-  // set_boundary_state (src/BoundCond.cu:55-76)
+    // set_boundary_state (src/BoundCond.cu:55-76)
 #pragma unroll
-  for (int l = 0; l < 6; ++l) z.bv[gw + l * sz] = st[l];
-  for (int l = 0; l < p.n_scalar; ++l) z.sv[gw + l * sz] = sv_b[l];
-  if (tt) z.tve[gw] = fmax(tve_s, 1.0);
-  cv_point<NS>(z, p, gw);
+    for (int l = 0; l < 6; ++l) z.bv[gw + l * sz] = st[l];
+    for (int l = 0; l < p.n_scalar; ++l) z.sv[gw + l * sz] = sv_b[l];
+    if (tt) z.tve[gw] = fmax(tve_b, 1.0);
+    cv_point<NS>(z, p, gw);
+  }
 }
 
 // No-slip, non-catalytic wall, isothermal (wall_T > 0) or adiabatic (apply_wall,
@@ -384,10 +388,10 @@ __global__ void k_bc_farfield(Zone z, Param p, FaceBC f) {
 // given wall_Tve (else T_wall) on an isothermal wall and the interior's on an adiabatic one; the
 // ghost T_ve mirrors it like T (floored at 0.1 max(T_ve,wall, 1)); e_ve of the wall node and of
 // every ghost is the mixture's at that T_ve.
-template <int NS>
+template <int NS, bool LINE>
 __global__ void k_bc_wall(Zone z, Param p, FaceBC f) {
   int i, j, k, gl;
-  if (!face_layer_point(f, z.ngg + 1, i, j, k, gl)) return;
+  if (!face_layer_point(f, LINE ? 1 : z.ngg + 1, i, j, k, gl)) return;
   int d[3] = {0, 0, 0};
   d[f.face] = f.direction;
   const idx_t sz = z.L.sz;
@@ -423,78 +427,81 @@ __global__ void k_bc_wall(Zone z, Param p, FaceBC f) {
     wv = -blow * ny;
     ww = -blow * nz;
   }
-  double R = kRAir;
-  if (gl == 0) {
-    const double pw = z.bv[g1 + 4 * sz];
-    if constexpr (NS > 0) {
-      R = 0;
-      for (int s = 0; s < NS; ++s) {
-        z.sv[gb + s * sz] = cat ? f.sv[s] : z.sv[g1 + s * sz];
-        R += z.sv[gb + s * sz] * __ldg(p.mech.gas_const + s);
+  const int last = LINE ? z.ngg : gl;
+  for (; gl <= last; ++gl) {
+    double R = kRAir;
+    if (gl == 0) {
+      const double pw = z.bv[g1 + 4 * sz];
+      if constexpr (NS > 0) {
+        R = 0;
+        for (int s = 0; s < NS; ++s) {
+          z.sv[gb + s * sz] = cat ? f.sv[s] : z.sv[g1 + s * sz];
+          R += z.sv[gb + s * sz] * __ldg(p.mech.gas_const + s);
+        }
       }
-    }
-    z.bv[gb] = pw / (t_wall * R);
-    z.bv[gb + sz] = wu;
-    z.bv[gb + 2 * sz] = wv;
-    z.bv[gb + 3 * sz] = ww;
-    z.bv[gb + 4 * sz] = pw;
-    z.bv[gb + 5 * sz] = t_wall;
-    if constexpr (NS > 0) {
-      if (tt) {
-        double y[NS];
+      z.bv[gb] = pw / (t_wall * R);
+      z.bv[gb + sz] = wu;
+      z.bv[gb + 2 * sz] = wv;
+      z.bv[gb + 3 * sz] = ww;
+      z.bv[gb + 4 * sz] = pw;
+      z.bv[gb + 5 * sz] = t_wall;
+      if constexpr (NS > 0) {
+        if (tt) {
+          double y[NS];
 #pragma unroll
-        for (int s = 0; s < NS; ++s) y[s] = z.sv[gb + s * sz];
-        z.tve[gb] = tve_wall;
-        z.sv[gb + p.i_eve * sz] = mixture_ve_energy<NS>(tve_wall, y, p.mech, nullptr);
+          for (int s = 0; s < NS; ++s) y[s] = z.sv[gb + s * sz];
+          z.tve[gb] = tve_wall;
+          z.sv[gb + p.i_eve * sz] = mixture_ve_energy<NS>(tve_wall, y, p.mech, nullptr);
+        }
       }
-    }
-    cv_point<NS>(z, p, gb);
-  } else {
-    int ai = i - gl * d[0], aj = j - gl * d[1], ak = k - gl * d[2];
-    project_to_interior(z, ai, aj, ak);
-    const idx_t gi = z.L.at(ai, aj, ak);
-    const idx_t gg = z.L.at(i + gl * d[0], j + gl * d[1], k + gl * d[2]);
-    const double p_i = z.bv[gi + 4 * sz], t_i = z.bv[gi + 5 * sz];
-    double t_g = t_i;
-    if (iso) {
-      t_g = 2 * t_wall - t_i;
-      if (t_g <= 0.1 * t_wall) t_g = tt ? 0.1 * t_wall : t_wall;
-    }
-    double tve_g = t_g;
-    if (tt) {
-      const double tve_i = z.tve[gi] > 0.0 ? z.tve[gi] : t_i;
-      tve_g = tve_i;
+      cv_point<NS>(z, p, gb);
+    } else {
+      int ai = i - gl * d[0], aj = j - gl * d[1], ak = k - gl * d[2];
+      project_to_interior(z, ai, aj, ak);
+      const idx_t gi = z.L.at(ai, aj, ak);
+      const idx_t gg = z.L.at(i + gl * d[0], j + gl * d[1], k + gl * d[2]);
+      const double p_i = z.bv[gi + 4 * sz], t_i = z.bv[gi + 5 * sz];
+      double t_g = t_i;
       if (iso) {
-        tve_g = 2 * tve_wall - tve_i;
-        const double floor_ve = 0.1 * fmax(tve_wall, 1.0);
-        if (tve_g <= floor_ve) tve_g = floor_ve;
+        t_g = 2 * t_wall - t_i;
+        if (t_g <= 0.1 * t_wall) t_g = tt ? 0.1 * t_wall : t_wall;
       }
-    }
-    if constexpr (NS > 0) {
-      R = 0;
-      for (int s = 0; s < NS; ++s) {
-        // catalytic: R of the face node, which holds the wall's mass fractions
-        const double y = cat ? f.sv[s] : z.sv[gi + s * sz];
-        z.sv[gg + s * sz] = y;
-        R += y * __ldg(p.mech.gas_const + s);
-      }
-    }
-    z.bv[gg] = p_i / (t_g * R);
-    z.bv[gg + sz] = 2 * wu - z.bv[gi + sz];
-    z.bv[gg + 2 * sz] = 2 * wv - z.bv[gi + 2 * sz];
-    z.bv[gg + 3 * sz] = 2 * ww - z.bv[gi + 3 * sz];
-    z.bv[gg + 4 * sz] = p_i;
-    z.bv[gg + 5 * sz] = t_g;
-    if constexpr (NS > 0) {
+      double tve_g = t_g;
       if (tt) {
-        double y[NS];
-#pragma unroll
-        for (int s = 0; s < NS; ++s) y[s] = z.sv[gg + s * sz];
-        z.tve[gg] = tve_g;
-        z.sv[gg + p.i_eve * sz] = mixture_ve_energy<NS>(tve_g, y, p.mech, nullptr);
+        const double tve_i = z.tve[gi] > 0.0 ? z.tve[gi] : t_i;
+        tve_g = tve_i;
+        if (iso) {
+          tve_g = 2 * tve_wall - tve_i;
+          const double floor_ve = 0.1 * fmax(tve_wall, 1.0);
+          if (tve_g <= floor_ve) tve_g = floor_ve;
+        }
       }
+      if constexpr (NS > 0) {
+        R = 0;
+        for (int s = 0; s < NS; ++s) {
+          // catalytic: R of the face node, which holds the wall's mass fractions
+          const double y = cat ? f.sv[s] : z.sv[gi + s * sz];
+          z.sv[gg + s * sz] = y;
+          R += y * __ldg(p.mech.gas_const + s);
+        }
+      }
+      z.bv[gg] = p_i / (t_g * R);
+      z.bv[gg + sz] = 2 * wu - z.bv[gi + sz];
+      z.bv[gg + 2 * sz] = 2 * wv - z.bv[gi + 2 * sz];
+      z.bv[gg + 3 * sz] = 2 * ww - z.bv[gi + 3 * sz];
+      z.bv[gg + 4 * sz] = p_i;
+      z.bv[gg + 5 * sz] = t_g;
+      if constexpr (NS > 0) {
+        if (tt) {
+          double y[NS];
+#pragma unroll
+          for (int s = 0; s < NS; ++s) y[s] = z.sv[gg + s * sz];
+          z.tve[gg] = tve_g;
+          z.sv[gg + p.i_eve * sz] = mixture_ve_energy<NS>(tve_g, y, p.mech, nullptr);
+        }
+      }
+      cv_point<NS>(z, p, gg);
     }
-    cv_point<NS>(z, p, gg);
   }
 }
 
@@ -779,6 +786,14 @@ static bool outflow_apart(const Zone &z, const FaceBC &a, const FaceBC &b) {
   return outflow_apart(ext, z.ngg, range(a), range(b));
 }
 
+// On a block of at most two nodes across a wall or a farfield face, the node inside lies on the opposite
+// boundary and is moved off it, onto the face itself (project_to_interior): the layers read the node
+// that the first of them writes, so one thread takes them in order.
+static bool thin_block(const Zone &z, const FaceBC &f) {
+  const int ext[3] = {z.mx, z.my, z.mz};
+  return (f.type == CB2_BC_WALL || f.type == CB2_BC_FARFIELD) && ext[f.face] <= 2;
+}
+
 // Small CTAs: a face has few nodes, and spreading them over more SMs shortens the launch.
 constexpr int kFaceThreads = 64;
 
@@ -831,15 +846,22 @@ static int launch_bc_ns(const Zone &z, const Param &p, const FaceBC *faces, int 
       const long long np = face_points(faces[f]);
       if (np == 0) continue;
       // threads per face node: one per layer including the face node (farfield, inflow, symmetry,
-      // wall), one per line (periodic)
-      const int layers = t == CB2_BC_PERIODIC ? 1 : z.ngg + 1;
+      // wall), one per line (periodic; walls and farfields of thin blocks)
+      const bool line = thin_block(z, faces[f]);
+      const int layers = t == CB2_BC_PERIODIC || line ? 1 : z.ngg + 1;
       const unsigned blocks = (unsigned)((np * layers + kFaceThreads - 1) / kFaceThreads);
       ProfScope prof("boundary_face", s);
       switch (t) {
-        case CB2_BC_FARFIELD: k_bc_farfield<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
+        case CB2_BC_FARFIELD:
+          if (line) k_bc_farfield<NS, true><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]);
+          else k_bc_farfield<NS, false><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]);
+          break;
         case CB2_BC_INFLOW: k_bc_inflow<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
         case CB2_BC_SYMMETRY: k_bc_symmetry<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
-        case CB2_BC_WALL: k_bc_wall<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
+        case CB2_BC_WALL:
+          if (line) k_bc_wall<NS, true><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]);
+          else k_bc_wall<NS, false><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]);
+          break;
         case CB2_BC_PERIODIC: k_bc_periodic<NS><<<blocks, kFaceThreads, 0, s>>>(z, p, faces[f]); break;
       }
       ++nl;
